@@ -808,6 +808,13 @@ def distributed_exact_dense_dynamic(mat, chunks: int | None = None, group=None, 
 
 
 CHECKPOINT_FORMAT = "perm_b200_checkpoint_v1"
+# from order 25 a shard's terms are those of the column-cube layout, so sums of
+# an earlier library's shards cannot be completed by this one's
+CHECKPOINT_FORMAT_CUBE = "perm_b200_checkpoint_v2"
+
+
+def _checkpoint_format(n: int) -> str:
+    return CHECKPOINT_FORMAT_CUBE if n >= 25 else CHECKPOINT_FORMAT
 
 
 def _fingerprint(a: np.ndarray) -> str:
@@ -829,7 +836,7 @@ def _read_checkpoint(path, fingerprint: str, n: int, chunks: int, variant: int) 
         return {}
     except (OSError, ValueError) as e:
         raise PermError(PERM_EIO, f"checkpoint {path} is unreadable ({e}); remove it to start over") from e
-    want = {"format": CHECKPOINT_FORMAT, "matrix_sha256": fingerprint, "n": n, "chunks": chunks,
+    want = {"format": _checkpoint_format(n), "matrix_sha256": fingerprint, "n": n, "chunks": chunks,
             "variant": variant}
     for k, v in want.items():
         if state.get(k) != v:
@@ -851,7 +858,7 @@ def _write_checkpoint(path, fingerprint: str, n: int, chunks: int, variant: int,
                       done: dict[int, tuple[float, float]]) -> None:
     import json
 
-    state = {"format": CHECKPOINT_FORMAT, "matrix_sha256": fingerprint, "n": n, "chunks": chunks,
+    state = {"format": _checkpoint_format(n), "matrix_sha256": fingerprint, "n": n, "chunks": chunks,
              "variant": variant,
              "done": {str(c): [h.hex(), l.hex()] for c, (h, l) in sorted(done.items())}}
     tmp = f"{path}.tmp"

@@ -29,7 +29,7 @@ NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompil
 HOST_CXX = os.environ.get("PERM_HOST_CXX", "/usr/bin/g++")
 
 LIB_SOURCES = [
-    "engine.cu", "ryser_skipper.cu", "mc.cu", "mc_sparse.cu", "batch.cu", "serve.cu", "noalloc.cu", "multi_device.cpp",
+    "engine.cu", "cube_plan.cpp", "ryser_skipper.cu", "mc.cu", "mc_sparse.cu", "batch.cu", "serve.cu", "noalloc.cu", "multi_device.cpp",
     "ryser_dense_inst_0.cu", "ryser_dense_inst_1.cu", "ryser_dense_inst_2.cu",
     "ryser_dense_inst_3.cu", "ryser_dense_inst_4.cu", "ryser_dense_2l_inst_0.cu", "ryser_dense_2l_inst_1.cu", "ryser_dense_int_g3.cu", "ryser_dense_int_g4.cu",
     "ryser_dense_int_g5.cu", "ryser_dense_int_g6.cu", "ryser_dense_int_sparse_g4.cu", "ryser_dense_int_sparse_g5.cu",
@@ -44,6 +44,7 @@ LIB_SOURCES = [
     "ryser_sparse_sdd_r28.cu", "ryser_sdd_3l_r16.cu", "ryser_sdd_3l_r20.cu", "ryser_sdd_3l_r24.cu",
     "ryser_sdd_3l_r28.cu", "ryser_dense_3l_r20.cu", "ryser_dense_3l_r24.cu", "ryser_dense_3l_r28.cu",
     "ryser_dense_3l_r32.cu", "ryser_dense_3l_r36.cu",
+    *[f"ryser_cube_{kind}_n{size}.cu" for kind in ("f64", "sdd") for size in (20, 24, 28, 32, 36, 40)],
 ]
 CLI_SOURCES = ["perman_cli.cpp"]
 

@@ -1,0 +1,31 @@
+// cube_plan.h -- host-side layout of the column-cube walks (ryser_cube.cuh):
+// which four columns are summed at once, which compiled shape holds the row
+// classes they make, and which row sits in which slot.  Host only.
+#pragma once
+#include <vector>
+
+#include "cube_shapes.h"
+
+namespace perm {
+
+struct CubeLayout {
+  int shape = -1;             // index into kCubeShapes, -1: none fits or none is cheap enough
+  double cost = 0;            // cube_shape_cost of the shape
+  std::vector<double> mat;    // row-major n x n: the fast columns first, rows in slot order
+                              // (the matrix or its transpose; same permanent)
+  std::vector<int> slot_row;  // row of `mat` in each slot, -1: a row of the constant 1
+};
+
+// The cheapest compiled shape, of at most max_cost, that holds the rows of some four columns of the n x n row-major
+// matrix or of its transpose; false when there is none (orders outside
+// 9..40 among them).
+bool cube_layout(const std::vector<double>& a, int n, double max_cost, CubeLayout* layout);
+
+// FP64 operations per 16 terms of a shape's FP64 walk, and the same weighted
+// by the rate its size reaches: measured 0.80..0.85 of the FP64 pipe up to 130
+// row values, 0.73 at 198, 0.65 at 257, 0.62 at 364, as operations at a rate
+// of 0.82.
+double cube_shape_ops(int shape);
+double cube_shape_cost(int shape);
+
+}  // namespace perm

@@ -29,10 +29,12 @@
 
 #include "../../include/perman_b200.h"
 #include "batch.h"
+#include "cube_plan.h"
 #include "matrix_io.h"
 #include "mc.h"
 #include "mc_sparse.h"
 #include "perman_common.cuh"
+#include "ryser_cube.h"
 #include "ryser_dense.cuh"
 #include "ryser_dense_dd.cuh"
 #include "ryser_dense_split.cuh"
@@ -128,10 +130,37 @@ const void* sdd_3l_kernel_r20(int n, int r1);
 const void* sdd_3l_kernel_r24(int n, int r1);
 const void* sdd_3l_kernel_r28(int n, int r1);
 
+const void* cube_f64_n20(int i);
+const void* cube_f64_n24(int i);
+const void* cube_f64_n28(int i);
+const void* cube_f64_n32(int i);
+const void* cube_f64_n36(int i);
+const void* cube_f64_n40(int i);
+const void* cube_sdd_n20(int i);
+const void* cube_sdd_n24(int i);
+const void* cube_sdd_n28(int i);
+const void* cube_sdd_n32(int i);
+const void* cube_sdd_n36(int i);
+const void* cube_sdd_n40(int i);
 const void* dense_tc_kernel_g3(int n);
 const void* dense_tc_kernel_g4(int n);
 const void* dense_tc_kernel_g5(int n);
 const void* dense_tc_kernel_g6(int n);
+
+static int cube_size(int shape) {
+  int i = 0;
+  while (shape >= kCubeFirst[i + 1]) i++;
+  return i;
+}
+static const void* cube_kernel(int shape, bool pair) {
+  using Pick = const void* (*)(int);
+  static const Pick f64[kCubeSizeCount] = {cube_f64_n20, cube_f64_n24, cube_f64_n28,
+                                           cube_f64_n32, cube_f64_n36, cube_f64_n40};
+  static const Pick sdd[kCubeSizeCount] = {cube_sdd_n20, cube_sdd_n24, cube_sdd_n28,
+                                           cube_sdd_n32, cube_sdd_n36, cube_sdd_n40};
+  const int i = cube_size(shape);
+  return (pair ? sdd : f64)[i](shape - kCubeFirst[i]);
+}
 
 static const void* dense_tc_kernel(int n, int g) {
   switch (g) {
@@ -443,6 +472,11 @@ using namespace perm;
 struct DenseOperand;
 struct perm_matrix;
 
+// Smallest order of the column-cube walks: the shards of shard_bounds are
+// whole cubes of 16 terms from here on, and below it the search for four
+// columns (some 30 us on the host) costs what the walk gains.
+constexpr int kCubeMinN = 25;
+
 struct perm_ctx {
   int device = 0;
   int num_sms = 0;
@@ -475,6 +509,7 @@ struct perm_ctx {
   // + ngo - 1] int32-X in the two-level row layout, [34 + 3 family + ngo - 1]
   // certified int32-X in the two-level layout
   int dense_occ[122][PERM_MAX_EXACT_N + 1] = {};
+  int cube_occ[2][kCubeShapeCount] = {};         // column-cube walks: [0] FP64, [1] split-dd
   int batch_m[kBatchMaxOrder + 1] = {};          // autotuned lane-range exponents (0: default)
   int dense_pref[PERM_MAX_EXACT_N + 1] = {};     // autotuned kernel for integer inputs (0: built-in choice)
   double rel_target = 1e-10;                     // rerun in double-double above this estimate (<=0: never)
@@ -490,6 +525,10 @@ struct perm_ctx {
 };
 
 static const int kMaxBlocks = 8192;
+// Column-cube walks recompute b after this many cubes: its updates' roundings
+// add up over no more steps than in the row layouts (2^11 terms a segment),
+// and the n (n - 5) additions are below 2% of the segment.
+constexpr uint64_t kCubeSegment = 256;
 
 static int fail(perm_ctx* ctx, int code, const char* fmt, ...) {
   char buf[512];
@@ -699,6 +738,8 @@ struct DenseOperand {
   int ng1 = 0, ng2 = 0;  // int32-X walk: groups of the three-level layout's first and second level (0: not)
   int inner = 0;  // split-dd and FP64 X: rows 0..inner-1 hold the support of columns 0..2 (0: one level)
   int inner1 = 0;  // split-dd three-level layout: rows 0..inner1-1 hold column 0's support (0: not)
+  int shape = -1;  // column-cube walk (ryser_cube.cuh): its shape, -1: one of the row layouts above
+  std::vector<double> sums;  // ... and the fast columns' sums, then (split-dd) those of their remainders
   std::vector<unsigned char> image;
 };
 
@@ -1161,11 +1202,13 @@ constexpr LevelLimits kFp64Levels = {28, 48, 2, 5, 7, 5, 9};
 // one-level walk costs 16n operations, the two-level 7 (2R + 1) + 2n, the
 // three-level 8 R1 + 6 R2 + 2n + 13; the three-level layout is taken when
 // cheapest.
-static void fp64_choose(const std::vector<double>& a, int n, int* inner, int* inner1, std::vector<double>* perm) {
+static void fp64_choose(const std::vector<double>& a, int n, int* inner, int* inner1, std::vector<double>* perm,
+                        long* cost8 = nullptr) {
   int c3[3] = {0, 1, 2};
   *inner = fp64_two_level_rows(a, n, c3);
   *inner1 = 0;
   const long cost = *inner ? 7L * (2 * *inner + 1) + 2L * n : 16L * n;
+  if (cost8) *cost8 = cost;
   int ng1 = 0, ng2 = 0;
   std::vector<double> three;
   if (three_level_permutation(a, n, 4, &ng1, &ng2, &three, kFp64Levels) &&
@@ -1173,6 +1216,7 @@ static void fp64_choose(const std::vector<double>& a, int n, int* inner, int* in
     *inner = 4 * (ng1 + ng2);
     *inner1 = 4 * ng1;
     *perm = std::move(three);
+    if (cost8) *cost8 = 32L * ng1 + 24L * (ng1 + ng2) + 2L * n + 13;
     return;
   }
   if (*inner) *perm = sparse_permutation(a.data(), n, c3);
@@ -1295,8 +1339,72 @@ static bool intc_three_level_layout(const std::vector<double>& a, int n, long be
   return best != best_cost;
 }
 
+// Column-major FP64 image, even column stride.
+static void build_fp64_image(const std::vector<double>& a, int n, DenseOperand* op) {
+  const int np = (n + 1) & ~1;
+  op->image.assign(sizeof(double) * (size_t)n * np, 0);
+  double* img = reinterpret_cast<double*>(op->image.data());
+  for (int k = 0; k < n; k++)
+    for (int j = 0; j < n; j++) img[(size_t)k * np + j] = a[(size_t)j * n + k];
+}
+
+// Turns the column-major image of a cube layout's matrix (`parts` column sets
+// of stride np) into the column-cube walk's operand: columns 4..n-1 in slot
+// order, and the sums of columns 0..3 for each row value.  Slots without a
+// row hold the constant 1 (2 in the last column, which is halved).
+static void build_cube_operand(const CubeLayout& l, int parts, DenseOperand* op) {
+  const int n = op->n, np = (n + 1) & ~1;
+  const CubeShape& shape = kCubeShapes[l.shape];
+  const int N = cube_rows(shape), nc = n - 4;
+  const std::vector<unsigned char> columns = std::move(op->image);
+  const double* col = reinterpret_cast<const double*>(columns.data());
+  op->shape = l.shape;
+  op->image.assign(sizeof(double) * parts * nc * N, 0);
+  op->sums.assign((size_t)parts * kCubeMaxSums, 0.0);
+  double* img = reinterpret_cast<double*>(op->image.data());
+  for (int part = 0; part < parts; part++) {
+    const double* from = col + (size_t)part * n * np;
+    double* to = img + (size_t)part * nc * N;
+    for (int slot = 0; slot < N; slot++) {
+      const int j = l.slot_row[slot];
+      if (j < 0) {
+        if (part == 0) to[(size_t)(nc - 1) * N + slot] = 2.0;
+        continue;
+      }
+      for (int k = 0; k < nc; k++) to[(size_t)k * N + slot] = from[(size_t)(k + 4) * np + j];
+    }
+    for (int i = 1; i < 16; i++) {
+      const int cls = cube_class(i), half = (1 << cube_bits(cls)) / 2;
+      for (int r = 0; r < shape.rows[cls]; r++) {
+        const int j = l.slot_row[cube_slot(shape, i) + r];
+        if (j < 0) continue;
+        for (int s = 0; s < half; s++) {
+          double t = 0.0;  // the last column of the set has sign plus
+          for (int k = 0, b = 0; k < 4; k++) {
+            if (!((cls >> k) & 1)) continue;
+            const double c = 0.5 * from[(size_t)k * np + j];
+            t += (s + half) >> b++ & 1 ? c : -c;
+          }
+          op->sums[(size_t)part * kCubeMaxSums + cube_sum(shape, i) + r * half + s] = t;
+        }
+      }
+    }
+  }
+}
+
 static int build_sdd_operand(perm_ctx* ctx, const std::vector<double>& a, int n, DenseOperand* op) {
   if (n < 4 || n > 40) return fail(ctx, PERM_EUNSUPPORTED, "split-dd kernel covers orders 4..40 (got %d)", n);
+  CubeLayout l;
+  // any shape that fits: 6 operations per row value at 0.63 of the FP64 pipe
+  // cost less than the row layouts' 6 per row and term at 0.56..0.69 (n = 30,
+  // 364 values: 7.3 ms against 8.9 ms in the dense layout)
+  if (n >= kCubeMinN && cube_layout(a, n, 1e9, &l)) {
+    const int rc = build_split_operand(ctx, l.mat, n, op);
+    if (rc) return rc;
+    op->variant = PERM_KERNEL_DENSE_SDD;
+    build_cube_operand(l, 2, op);
+    return PERM_OK;
+  }
   int inner = 0, inner1 = 0;
   std::vector<double> perm;
   sdd_choose(a, n, &inner, &inner1, &perm);
@@ -1378,20 +1486,32 @@ static int build_operand(perm_ctx* ctx, const void* mat, int n, int dtype, int v
       y0[j] = (int)(2 * (long long)a[(size_t)j * n + n - 1] - rs);
     }
   } else {
-    const int np = (n + 1) & ~1;
     op->variant = variant == PERM_KERNEL_DENSE_DD ? PERM_KERNEL_DENSE_DD : PERM_KERNEL_DENSE;
     op->group = 0;
     op->inner = 0;
     op->inner1 = 0;
     if (op->variant == PERM_KERNEL_DENSE) {
+      // The column-cube walk unless a row layout needs fewer operations: their
+      // walks reach 0.93 (one level) and 0.87 of the FP64 pipe against 0.82.
+      // The smallest row layout (levels of 8 and 20 rows) needs 394 + 4n
+      // operations per 16 terms, so cheaper cubes skip the search for one.
+      CubeLayout l;
+      const bool cube = n >= kCubeMinN && cube_layout(a, n, 32.0 * n * 0.82 / 0.93, &l);
       std::vector<double> perm;
-      fp64_choose(a, n, &op->inner, &op->inner1, &perm);
+      if (!cube || l.cost > (394.0 + 4.0 * n) * 0.82 / 0.87) {
+        long cost8 = 0;  // operations per 8 terms
+        fp64_choose(a, n, &op->inner, &op->inner1, &perm, &cost8);
+        if (cube && l.cost / 0.82 > 2.0 * (double)cost8 / (op->inner ? 0.87 : 0.93)) l.shape = -1;
+      }
+      if (l.shape >= 0) {
+        op->inner = op->inner1 = 0;
+        build_fp64_image(l.mat, n, op);
+        build_cube_operand(l, 1, op);
+        return PERM_OK;
+      }
       if (op->inner) a.swap(perm);  // walk the permuted matrix (same permanent)
     }
-    op->image.assign(sizeof(double) * (size_t)n * np, 0);
-    double* img = reinterpret_cast<double*>(op->image.data());
-    for (int k = 0; k < n; k++)
-      for (int j = 0; j < n; j++) img[(size_t)k * np + j] = a[(size_t)j * n + k];
+    build_fp64_image(a, n, op);
   }
   return PERM_OK;
 }
@@ -1402,6 +1522,7 @@ struct perm_matrix {
 };
 
 static const void* operand_kernel(const DenseOperand& op) {
+  if (op.shape >= 0) return cube_kernel(op.shape, op.variant == PERM_KERNEL_DENSE_SDD);
   if (op.variant == PERM_KERNEL_DENSE_INT)
     return op.ng1 ? dense_int_3l_kernel(op.n, op.group, op.ng1, op.ng2)
            : op.ngo ? dense_int_sparse_kernel(op.n, op.group, op.ngo)
@@ -1418,8 +1539,12 @@ static const void* operand_kernel(const DenseOperand& op) {
          : op.inner ? dense_2l_kernel(op.n, op.inner)
                     : dense_kernel(op.n);
 }
-static int operand_threads(const DenseOperand& op) { return op.variant == PERM_KERNEL_DENSE_TC ? kTcThreads : 128; }
+static int operand_threads(const DenseOperand& op) {
+  return op.shape >= 0 ? kCubeThreads : op.variant == PERM_KERNEL_DENSE_TC ? kTcThreads : 128;
+}
 static size_t operand_smem(const DenseOperand& op) {
+  if (op.shape >= 0)
+    return cube_smem_bytes(op.variant == PERM_KERNEL_DENSE_SDD, op.n, cube_rows(kCubeShapes[op.shape]));
   if (op.variant == PERM_KERNEL_DENSE_INT || op.variant == PERM_KERNEL_DENSE_INT_DD) return dense_int_smem_bytes(op.n);
   if (op.variant == PERM_KERNEL_DENSE_SDD)
     return op.inner ? sparse_sdd_smem_bytes(op.n, op.inner, 128) : dense_sdd_smem_bytes(op.n);
@@ -1543,7 +1668,8 @@ static int dense_plan(perm_ctx* ctx, const DenseOperand& op, int shard, int nsha
   }
   for (int i = 0; i < 5; i++)
     if (op.inner1 && op.inner == kFp3lR2[i]) fp_slot = 102 + 4 * i + op.inner1 / 4 - 2;
-  int& occ_slot = ctx->dense_occ[op.variant == PERM_KERNEL_DENSE_INT
+  const bool pair = op.variant == PERM_KERNEL_DENSE_SDD;
+  int& occ_slot = op.shape >= 0 ? ctx->cube_occ[pair][op.shape] : ctx->dense_occ[op.variant == PERM_KERNEL_DENSE_INT
                                      ? (op.ng1 ? 50 + 6 * (op.group - 4) + 2 * (op.ng1 - 2) + op.ng2 - 1
                                         : op.ngo ? 25 + 3 * (op.group - 4) + op.ngo - 1
                                                  : op.group)
@@ -1588,6 +1714,25 @@ static int dense_plan(perm_ctx* ctx, const DenseOperand& op, int shard, int nsha
     return PERM_OK;
   }
   int grid = std::min(kMaxBlocks, ctx->num_sms * occ_slot);
+  if (op.shape >= 0) {
+    // ranges of whole cubes.  A thread owns ceil(blocks / threads) blocks of
+    // 2^m cubes at most; leaving a block costs about half a cube more, since
+    // the lanes then flip different columns.
+    const uint64_t cubes = (last - first) >> 4, threads = (uint64_t)grid * kCubeThreads;
+    double best = -1.0;
+    for (int m = 0; m <= 10 && m <= (nshards == 1 ? n - 5 : ms - 4); m++) {
+      const double each = std::ceil((double)(cubes >> m) / (double)threads);
+      const double cost = each * (std::ldexp(1.0, m) + 0.5);
+      if (best < 0.0 || cost < best) {
+        best = cost;
+        p->m = 4 + m;
+      }
+    }
+    p->block0 = first >> p->m;
+    p->nblocks = (last - first) >> p->m;
+    p->grid = (int)std::min<uint64_t>((uint64_t)grid, std::max<uint64_t>(1, (p->nblocks + kCubeThreads - 1) / kCubeThreads));
+    return PERM_OK;
+  }
   // Alignment m <= ms: each thread should own >= 64 aligned blocks when possible.
   const uint64_t len = last - first;
   const uint64_t threads = (uint64_t)grid * 128;
@@ -1605,7 +1750,29 @@ static int dense_plan(perm_ctx* ctx, const DenseOperand& op, int shard, int nsha
 static int dense_launch(perm_ctx* ctx, const DenseOperand& op, const void* d_image, const DensePlan& p) {
   const int n = op.n;
   CU(ctx, cudaEventRecord(ctx->ev0, ctx->stream));
-  if (op.variant == PERM_KERNEL_DENSE_TC) {
+  if (op.shape >= 0) {
+    CubeArgs args;
+    args.img = static_cast<const double*>(d_image);
+    args.n = n;
+    args.m = p.m - 4;
+    args.block0 = p.block0;
+    args.nblocks = p.nblocks;
+    args.seg = kCubeSegment;
+    args.partials = ctx->partials;
+    args.ticket = ctx->ticket;
+    args.out = ctx->d_out;
+    args.sums = ctx->d_est;
+    args.err = ctx->d_err;
+    args.inject = ctx->inject_timeouts > 0 && op.variant == PERM_KERNEL_DENSE ? 16u : 0u;
+    if (args.inject) ctx->inject_timeouts--;
+    memcpy(args.c, op.sums.data(), sizeof args.c);
+    if (op.variant == PERM_KERNEL_DENSE_SDD) {
+      memcpy(args.cl, op.sums.data() + kCubeMaxSums, sizeof args.cl);
+      CU(ctx, cudaMemsetAsync(ctx->d_est, 0, 2 * sizeof(double), ctx->stream));
+    }
+    void* kargs[] = {&args};
+    CU(ctx, cudaLaunchKernel(operand_kernel(op), dim3(p.grid), dim3(kCubeThreads), kargs, operand_smem(op), ctx->stream));
+  } else if (op.variant == PERM_KERNEL_DENSE_TC) {
     DenseTcArgs args;
     args.colI = static_cast<const int*>(d_image);
     args.np4 = (n + 3) & ~3;
@@ -1716,7 +1883,7 @@ static int dense_collect(perm_ctx* ctx, const DenseOperand& op, const DensePlan&
   } else if (sums) {
     // the int32-X walk's terms are prod y = 2^n prod x (|factor| 2^(1-n))
     ctx->walk_m1 = ctx->h_out[12] * (op.variant == PERM_KERNEL_DENSE_INT_DD ? std::ldexp(1.0, 1 - op.n) : 2.0);
-    const uint64_t threads = (uint64_t)p.grid * 128;
+    const uint64_t threads = (uint64_t)p.grid * operand_threads(op);
     ctx->walk_terms_per_thread = ((p.nblocks + threads - 1) / threads) << p.m;
   }
   float ms = 0;
@@ -1929,10 +2096,10 @@ static int refine_result(perm_ctx* ctx, const void* mat, int n, int dtype, const
   // the estimate samples an FP64 column image; an int32 or split operand is replaced by one
   DenseOperand f;
   const DenseOperand* fp = &op;
-  if (op.variant == PERM_KERNEL_DENSE_INT || op.variant == PERM_KERNEL_DENSE_TC ||
-      op.variant == PERM_KERNEL_DENSE_SPLIT || op.variant == PERM_KERNEL_DENSE_INT_DD ||
-      op.variant == PERM_KERNEL_DENSE_SDD) {
-    if ((rc = build_operand(ctx, mat, n, dtype, PERM_KERNEL_DENSE, &f))) return rc;
+  if (op.shape >= 0 || (op.variant != PERM_KERNEL_DENSE && op.variant != PERM_KERNEL_DENSE_DD)) {
+    std::vector<double> a((size_t)n * n);
+    for (size_t i = 0; i < a.size(); i++) a[i] = elem(mat, dtype, i);
+    build_fp64_image(a, n, &f);
     fp = &f;
   }
   if ((rc = stage_operand(ctx, *fp))) return rc;
@@ -2053,8 +2220,8 @@ static int policy_predicts_sdd(perm_ctx* ctx, const void* mat, int n, int dtype,
   }
   if (!split_rows_ok(a, n)) return PERM_OK;
   DenseOperand f;
-  int rc = build_operand(ctx, mat, n, dtype, PERM_KERNEL_DENSE, &f);
-  if (rc) return rc;
+  build_fp64_image(a, n, &f);
+  int rc;
   if ((rc = stage_operand(ctx, f))) return rc;
   const int np = (n + 1) & ~1;
   const uint64_t threads = (uint64_t)n * kSamplesPerClass;

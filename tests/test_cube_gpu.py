@@ -1,0 +1,79 @@
+"""The column-cube walks (four columns summed at once, rows in the classes of a
+compiled shape) of FP64 x and split-dd: orders at the edges of the shape sizes
+(no unused slot, up to three), sparse to dense shapes, shards, and the order
+limits; against the CPU double-double oracle, the double-double kernel and a
+product of smaller permanents, each within the walk's own error bound."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+U = 2.0 ** -53
+
+
+def _real(n, d, seed, signed=False):
+    """Density-d pattern with a hidden permutation, values (0, 1] or normal."""
+    rng = np.random.default_rng([n, seed])
+    mask = (rng.random((n, n)) < d) | (np.eye(n)[rng.permutation(n)] > 0)
+    return mask * (rng.standard_normal((n, n)) if signed else 1.0 - rng.random((n, n)))
+
+
+def _check(engine, A, want, want_err, kernels):
+    for variant in kernels:
+        r = engine.exact_dense(A, variant=variant)
+        assert r.kernel == variant
+        # the bound is of the (hi, lo) pair; value rounds it once more
+        tol = r.rel_error_estimate * abs(want) + want_err + U * abs(want)
+        assert abs(r.value - want) <= tol, (variant, r.value, want, tol)
+        parts = [engine.exact_dense_shard(A, s, 3, variant=variant) for s in range(3)]
+        assert abs(sum(p.hi for p in parts) + sum(p.lo for p in parts) - r.value) <= 2 * tol + 4 * U * abs(want), variant
+
+
+@pytest.mark.parametrize("n,d,signed", [(25, 0.12, False), (25, 0.5, True), (26, 0.95, False), (28, 0.35, False),
+                                        (29, 0.7, False)])
+def test_cube_vs_oracle_dd(engine, orc, pb, n, d, signed):
+    A = _real(n, d, 1, signed)
+    hi, lo = orc.perm_dd(A)
+    r = engine.exact_dense(A, variant=pb.PERM_KERNEL_DENSE_SDD)
+    # the oracle's own error: (4n + 32) u^2 sum|t|
+    _check(engine, A, hi + lo, (4 * n + 32) * U * U * r.abs_term_sum,
+           (pb.PERM_KERNEL_DENSE, pb.PERM_KERNEL_DENSE_SDD))
+
+
+@pytest.mark.parametrize("n,d", [(32, 0.5), (33, 0.25), (36, 0.2)])
+def test_cube_vs_double_double_kernel(engine, pb, n, d):
+    A = _real(n, d, 2)
+    r = engine.exact_dense(A, variant=pb.PERM_KERNEL_DENSE_DD)
+    _check(engine, A, r.hi + r.lo, (r.rel_error_estimate + U) * abs(r.value),
+           (pb.PERM_KERNEL_DENSE, pb.PERM_KERNEL_DENSE_SDD))
+
+
+@pytest.mark.parametrize("n,k", [(40, 21), (37, 20)])
+def test_cube_largest_orders_vs_product(engine, orc, pb, n, k):
+    """Two diagonal blocks, rows and columns shuffled: the permanent is the
+    product of the blocks'."""
+    rng = np.random.default_rng(n)
+    B, C = _real(k, 0.9, 3), _real(n - k, 0.9, 4)
+    A = np.zeros((n, n))
+    A[:k, :k], A[k:, k:] = B, C
+    A = A[rng.permutation(n)][:, rng.permutation(n)]
+    b, c = orc.perm_dd(B), orc.perm_dd(C)
+    want = (b[0] + b[1]) * (c[0] + c[1])
+    # each factor rounded once, and their product
+    r = engine.exact_dense(A, variant=pb.PERM_KERNEL_DENSE)
+    assert abs(r.value - want) <= (r.rel_error_estimate + 4 * U) * want
+
+
+def test_cube_transposed_and_permuted_inputs_agree(engine, pb):
+    """The layout may walk the transpose: a matrix with sparse rows and its
+    transpose (sparse columns) have one permanent."""
+    rng = np.random.default_rng(11)
+    n = 27
+    A = _real(n, 0.85, 5)
+    A[:4] *= rng.random((4, n)) < 0.3
+    A[np.arange(4), np.arange(4)] = 1.0
+    got = [engine.exact_dense(M, variant=pb.PERM_KERNEL_DENSE_SDD) for M in (A, A.T.copy(), A[::-1, ::-1].copy())]
+    for g in got[1:]:
+        assert abs(g.value - got[0].value) <= (g.rel_error_estimate + got[0].rel_error_estimate + 2 * U) * got[0].value
