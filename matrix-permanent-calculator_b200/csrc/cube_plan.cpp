@@ -4,6 +4,7 @@
 #include <algorithm>
 #include <cstdint>
 #include <cstring>
+#include <initializer_list>
 
 namespace perm {
 
@@ -119,7 +120,7 @@ double cube_shape_ops(int shape) {
   double ops = cube_rows(s);  // updates of b
   for (int i = 0; i < 16; i++) ops += k(i) * (i ? 2 * w(i) : 1);
   // class arrays: the first row of a chain only sets it; {02} and {13} are
-  // merged into 8 values, the second and third chain into top
+  // merged into 8 values, the second chain into 16
   auto chain = [&](std::initializer_list<int> order, int extra) {
     bool unset = true;
     for (int i : order) {
@@ -132,11 +133,11 @@ double cube_shape_ops(int shape) {
     }
     return !unset;
   };
-  chain({0, 1, 2, 3, 4, 5}, 3);
+  chain({1, 2, 3, 4, 5}, 3);
   if (chain({6, 7, 8, 9}, 8)) ops += 16;
-  if (chain({10, 11, 12}, -1)) ops += 16;
-  chain({13, 14, 15}, -1);
-  return ops + 24;  // differences over column 2, products with the last chain, sum
+  if (chain({10, 11, 12}, -1)) ops += 8;  // fused with the differences
+  chain({0, 13, 14, 15}, -1);
+  return ops + 8 + 8 + 3;  // differences over column 2, products with the last chain, sum
 }
 
 double cube_shape_cost(int shape) {

@@ -6,10 +6,10 @@
 // nonzero.  A row may also sit in the slot of any larger set (its extra
 // entries there are zeros), and unused slots hold rows of the constant 1, so
 // a few shapes per size serve every matrix whose four chosen columns fit.
-// The shapes were picked greedily from the class counts of random matrices of
-// density 0.15..0.95 (a third at 0.5): with 12 to 14 shapes per size the
-// cheapest that fits needs 1.07 to 1.11 times the operations of a
-// shape made for the matrix (one shape: 1.7 times, 6 shapes: 1.15).
+// The shapes were picked greedily, then improved by moving single slots, over
+// the class counts of random matrices of density 0.15..0.95 (half of them near
+// 0.5): with 22 shapes per size the cheapest that fits needs 1.07 to 1.09 times
+// the operations of a shape made for the matrix (one shape: 1.7 times).
 #pragma once
 #include <cstdint>
 
@@ -27,97 +27,103 @@ struct CubeShape {
 
 // Shapes of kCubeSizes[i] rows are kCubeShapes[kCubeFirst[i] .. kCubeFirst[i + 1]),
 // cheapest first; comments: row values and FP64 operations per 16 terms.
-constexpr int kCubeSizeCount = 6;
-constexpr int kCubeSizes[kCubeSizeCount] = {20, 24, 28, 32, 36, 40};
-constexpr int kCubeFirst[kCubeSizeCount + 1] = {0, 12, 24, 38, 52, 66, 80};
-constexpr int kCubeShapeCount = 80;
+constexpr int kCubeSizeCount = 4;
+constexpr int kCubeSizes[kCubeSizeCount] = {28, 32, 36, 40};
+constexpr int kCubeFirst[kCubeSizeCount + 1] = {0, 22, 44, 66, 88};
+constexpr int kCubeShapeCount = 88;
 constexpr CubeShape kCubeShapes[kCubeShapeCount] = {
-    // up to 20 rows
-    {{13, 3, 0, 1, 0, 0, 0, 0, 2, 1, 0, 0, 0, 0, 0, 0}},  // 31 values, 90 operations
-    {{13, 2, 0, 1, 2, 0, 0, 0, 2, 0, 0, 0, 0, 0, 0, 0}},  // 29 values, 100 operations
-    {{11, 2, 0, 1, 2, 0, 0, 0, 1, 1, 0, 0, 2, 0, 0, 0}},  // 37 values, 118 operations
-    {{9, 2, 2, 0, 0, 2, 2, 0, 1, 2, 0, 0, 0, 0, 0, 0}},  // 43 values, 136 operations
-    {{4, 3, 1, 1, 0, 2, 3, 0, 4, 1, 0, 1, 0, 0, 0, 0}},  // 56 values, 167 operations
-    {{3, 1, 3, 1, 0, 3, 2, 0, 2, 2, 1, 1, 0, 0, 1, 0}},  // 67 values, 194 operations
-    {{4, 1, 1, 1, 0, 3, 1, 2, 2, 2, 2, 0, 0, 0, 1, 0}},  // 72 values, 203 operations
-    {{2, 1, 0, 2, 1, 3, 2, 1, 0, 2, 3, 1, 1, 0, 1, 0}},  // 82 values, 235 operations
-    {{0, 2, 1, 2, 0, 3, 2, 1, 1, 3, 0, 2, 0, 1, 2, 0}},  // 96 values, 258 operations
-    {{3, 1, 0, 2, 0, 0, 0, 3, 0, 1, 0, 1, 2, 2, 3, 2}},  // 129 values, 314 operations
-    {{0, 1, 0, 1, 0, 0, 1, 4, 0, 0, 1, 2, 0, 5, 2, 3}},  // 166 values, 390 operations
-    {{0, 0, 0, 0, 0, 0, 2, 2, 0, 1, 0, 2, 0, 3, 1, 9}},  // 220 values, 492 operations
-    // up to 24 rows
-    {{18, 1, 0, 1, 2, 0, 0, 0, 2, 0, 0, 0, 0, 0, 0, 0}},  // 32 values, 105 operations
-    {{12, 2, 4, 0, 0, 1, 1, 0, 3, 1, 0, 0, 0, 0, 0, 0}},  // 42 values, 135 operations
-    {{6, 5, 4, 1, 0, 1, 3, 0, 3, 1, 0, 0, 0, 0, 0, 0}},  // 54 values, 165 operations
-    {{5, 3, 1, 1, 0, 2, 3, 0, 3, 3, 1, 0, 0, 0, 2, 0}},  // 75 values, 212 operations
-    {{3, 3, 3, 1, 0, 3, 2, 0, 4, 1, 1, 1, 0, 0, 2, 0}},  // 79 values, 222 operations
-    {{3, 0, 2, 2, 0, 3, 1, 1, 3, 4, 4, 0, 0, 0, 1, 0}},  // 85 values, 234 operations
-    {{2, 4, 2, 3, 0, 2, 3, 1, 2, 2, 0, 0, 2, 0, 1, 0}},  // 82 values, 237 operations
-    {{2, 2, 2, 2, 1, 3, 3, 1, 2, 2, 0, 1, 1, 0, 2, 0}},  // 92 values, 259 operations
-    {{1, 2, 0, 2, 2, 0, 0, 2, 0, 3, 1, 4, 2, 2, 3, 0}},  // 129 values, 326 operations
-    {{0, 0, 0, 3, 1, 3, 0, 3, 0, 3, 1, 3, 1, 1, 3, 2}},  // 158 values, 386 operations
-    {{0, 0, 0, 1, 0, 2, 0, 5, 0, 0, 1, 4, 0, 4, 3, 4}},  // 208 values, 476 operations
-    {{1, 0, 0, 1, 0, 0, 0, 4, 0, 0, 0, 3, 0, 4, 2, 9}},  // 253 values, 560 operations
     // up to 28 rows
-    {{18, 3, 3, 0, 2, 0, 0, 0, 2, 0, 0, 0, 0, 0, 0, 0}},  // 38 values, 135 operations
-    {{15, 3, 3, 1, 3, 0, 0, 0, 3, 0, 0, 0, 0, 0, 0, 0}},  // 43 values, 148 operations
-    {{8, 4, 4, 2, 5, 0, 0, 0, 3, 1, 0, 0, 1, 0, 0, 0}},  // 56 values, 181 operations
-    {{6, 4, 2, 4, 4, 0, 1, 0, 4, 1, 1, 0, 1, 0, 0, 0}},  // 66 values, 207 operations
-    {{4, 4, 1, 1, 0, 4, 3, 1, 6, 2, 1, 0, 0, 0, 1, 0}},  // 86 values, 239 operations
-    {{6, 4, 1, 3, 2, 0, 3, 1, 1, 2, 1, 0, 2, 1, 1, 0}},  // 90 values, 255 operations
-    {{5, 2, 4, 3, 0, 3, 1, 1, 2, 1, 1, 0, 2, 2, 1, 0}},  // 97 values, 272 operations
-    {{2, 5, 1, 2, 2, 0, 4, 1, 2, 3, 2, 1, 1, 1, 1, 0}},  // 102 values, 283 operations
-    {{2, 3, 1, 1, 0, 3, 4, 3, 1, 4, 3, 0, 2, 0, 1, 0}},  // 112 values, 305 operations
-    {{3, 2, 0, 2, 0, 2, 4, 2, 2, 1, 2, 3, 1, 2, 2, 0}},  // 131 values, 340 operations
-    {{0, 0, 3, 3, 0, 4, 2, 1, 0, 3, 3, 1, 2, 3, 2, 1}},  // 146 values, 370 operations
-    {{0, 1, 1, 2, 0, 1, 4, 3, 1, 4, 0, 3, 2, 2, 1, 3}},  // 178 values, 434 operations
-    {{0, 0, 0, 1, 0, 2, 1, 4, 0, 1, 2, 4, 0, 5, 4, 4}},  // 228 values, 528 operations
-    {{0, 0, 0, 0, 0, 0, 0, 5, 0, 0, 0, 4, 1, 3, 3, 12}},  // 316 values, 688 operations
+    {{19, 2, 0, 2, 3, 0, 0, 0, 2, 0, 0, 0, 0, 0, 0, 0}},  // 41 values, 113 operations
+    {{16, 2, 0, 3, 3, 0, 0, 0, 4, 0, 0, 0, 0, 0, 0, 0}},  // 46 values, 126 operations
+    {{12, 2, 0, 3, 5, 0, 0, 0, 5, 1, 0, 0, 0, 0, 0, 0}},  // 52 values, 142 operations
+    {{11, 4, 4, 1, 3, 0, 1, 0, 2, 1, 0, 0, 1, 0, 0, 0}},  // 53 values, 159 operations
+    {{9, 6, 3, 1, 2, 0, 2, 0, 3, 1, 1, 0, 0, 0, 0, 0}},  // 57 values, 173 operations
+    {{6, 0, 5, 3, 4, 2, 1, 0, 3, 3, 0, 0, 1, 0, 0, 0}},  // 70 values, 200 operations
+    {{5, 4, 2, 2, 2, 2, 3, 0, 2, 3, 0, 0, 2, 0, 1, 0}},  // 81 values, 225 operations
+    {{6, 3, 3, 2, 0, 2, 3, 1, 1, 2, 2, 0, 3, 0, 0, 0}},  // 84 values, 232 operations
+    {{5, 5, 1, 2, 3, 0, 3, 2, 2, 1, 0, 1, 2, 0, 1, 0}},  // 91 values, 241 operations
+    {{4, 3, 2, 2, 3, 4, 1, 0, 1, 1, 3, 1, 2, 1, 0, 0}},  // 90 values, 248 operations
+    {{4, 4, 2, 3, 3, 0, 2, 0, 1, 2, 1, 1, 3, 1, 1, 0}},  // 92 values, 248 operations
+    {{2, 3, 2, 4, 0, 2, 2, 1, 2, 3, 2, 0, 4, 0, 1, 0}},  // 100 values, 268 operations
+    {{3, 2, 2, 3, 2, 3, 1, 1, 2, 1, 2, 2, 2, 1, 1, 0}},  // 107 values, 283 operations
+    {{0, 5, 1, 2, 2, 2, 4, 1, 0, 2, 4, 1, 2, 2, 0, 0}},  // 112 values, 293 operations
+    {{2, 2, 4, 3, 0, 2, 2, 1, 2, 3, 1, 1, 1, 2, 2, 0}},  // 114 values, 296 operations
+    {{2, 1, 0, 4, 0, 4, 2, 2, 1, 3, 3, 1, 2, 0, 3, 0}},  // 126 values, 318 operations
+    {{2, 1, 2, 3, 1, 0, 3, 2, 1, 3, 0, 2, 2, 3, 3, 0}},  // 136 values, 334 operations
+    {{1, 0, 0, 3, 0, 1, 2, 3, 1, 2, 3, 2, 2, 5, 3, 0}},  // 159 values, 383 operations
+    {{1, 0, 0, 2, 0, 0, 3, 3, 1, 1, 1, 4, 2, 5, 2, 3}},  // 199 values, 459 operations
+    {{0, 1, 0, 1, 0, 1, 0, 5, 1, 1, 0, 4, 0, 4, 5, 5}},  // 240 values, 535 operations
+    {{1, 0, 0, 0, 0, 0, 2, 3, 1, 1, 0, 5, 0, 3, 3, 9}},  // 271 values, 591 operations
+    {{0, 0, 0, 0, 0, 0, 1, 3, 0, 0, 0, 3, 0, 5, 2, 14}},  // 332 values, 707 operations
     // up to 32 rows
-    {{18, 5, 4, 0, 0, 0, 1, 0, 4, 0, 0, 0, 0, 0, 0, 0}},  // 48 values, 145 operations
-    {{22, 2, 2, 0, 0, 2, 1, 0, 2, 1, 0, 0, 0, 0, 0, 0}},  // 50 values, 149 operations
-    {{17, 4, 3, 1, 3, 0, 0, 0, 3, 0, 0, 0, 1, 0, 0, 0}},  // 51 values, 166 operations
-    {{15, 2, 3, 2, 3, 1, 1, 0, 3, 1, 0, 0, 1, 0, 0, 0}},  // 61 values, 192 operations
-    {{7, 6, 4, 2, 4, 0, 2, 0, 3, 2, 1, 0, 1, 0, 0, 0}},  // 73 values, 224 operations
-    {{7, 3, 2, 1, 0, 4, 3, 2, 2, 3, 4, 0, 0, 0, 1, 0}},  // 105 values, 278 operations
-    {{3, 2, 3, 3, 4, 4, 2, 1, 3, 3, 0, 1, 2, 0, 1, 0}},  // 107 values, 296 operations
-    {{4, 3, 3, 4, 2, 2, 3, 0, 0, 3, 2, 0, 3, 2, 1, 0}},  // 112 values, 307 operations
-    {{4, 1, 3, 5, 1, 2, 3, 1, 2, 2, 1, 1, 2, 3, 1, 0}},  // 126 values, 337 operations
-    {{3, 1, 1, 4, 1, 1, 2, 2, 0, 2, 3, 1, 4, 3, 1, 3}},  // 177 values, 438 operations
-    {{2, 1, 0, 4, 1, 1, 3, 4, 0, 1, 1, 3, 2, 4, 3, 2}},  // 198 values, 479 operations
-    {{1, 1, 1, 3, 0, 2, 1, 2, 0, 1, 0, 5, 2, 2, 4, 7}},  // 257 values, 594 operations
-    {{0, 1, 1, 2, 0, 3, 2, 3, 0, 1, 0, 4, 1, 3, 4, 7}},  // 264 values, 608 operations
-    {{0, 0, 0, 1, 0, 0, 0, 5, 0, 0, 0, 5, 0, 4, 3, 14}},  // 364 values, 788 operations
+    {{23, 2, 0, 2, 3, 0, 0, 0, 2, 0, 0, 0, 0, 0, 0, 0}},  // 45 values, 121 operations
+    {{19, 3, 0, 2, 5, 0, 0, 0, 3, 0, 0, 0, 0, 0, 0, 0}},  // 49 values, 133 operations
+    {{19, 3, 4, 0, 3, 0, 0, 0, 2, 1, 0, 0, 0, 0, 0, 0}},  // 47 values, 143 operations
+    {{16, 3, 5, 1, 2, 0, 0, 0, 3, 1, 0, 0, 1, 0, 0, 0}},  // 54 values, 160 operations
+    {{11, 5, 6, 1, 5, 0, 0, 0, 2, 1, 0, 0, 1, 0, 0, 0}},  // 59 values, 175 operations
+    {{13, 4, 3, 1, 2, 0, 2, 0, 2, 2, 1, 0, 1, 1, 0, 0}},  // 71 values, 201 operations
+    {{6, 4, 6, 3, 2, 2, 2, 0, 2, 1, 1, 0, 2, 1, 0, 0}},  // 86 values, 242 operations
+    {{5, 3, 5, 3, 4, 1, 2, 0, 2, 3, 0, 0, 2, 1, 1, 0}},  // 93 values, 253 operations
+    {{5, 4, 2, 3, 2, 2, 3, 0, 3, 2, 2, 1, 2, 1, 0, 0}},  // 99 values, 269 operations
+    {{5, 3, 3, 3, 2, 2, 3, 1, 3, 1, 0, 2, 3, 0, 1, 0}},  // 107 values, 281 operations
+    {{4, 4, 3, 2, 0, 3, 4, 1, 2, 3, 0, 1, 3, 1, 1, 0}},  // 114 values, 294 operations
+    {{5, 2, 2, 3, 3, 2, 3, 0, 1, 3, 2, 1, 2, 1, 2, 0}},  // 113 values, 297 operations
+    {{2, 3, 2, 3, 3, 3, 1, 2, 3, 2, 2, 1, 3, 1, 1, 0}},  // 120 values, 314 operations
+    {{2, 3, 3, 3, 0, 3, 2, 2, 3, 3, 0, 1, 3, 1, 3, 0}},  // 132 values, 332 operations
+    {{2, 3, 1, 2, 2, 2, 2, 2, 1, 4, 3, 3, 3, 0, 2, 0}},  // 136 values, 346 operations
+    {{0, 2, 3, 3, 0, 3, 3, 2, 3, 2, 1, 3, 2, 3, 2, 0}},  // 152 values, 377 operations
+    {{3, 0, 0, 3, 0, 3, 1, 4, 1, 2, 4, 2, 3, 3, 2, 1}},  // 173 values, 413 operations
+    {{0, 0, 1, 4, 0, 2, 2, 6, 1, 4, 1, 2, 2, 2, 4, 1}},  // 192 values, 455 operations
+    {{0, 1, 1, 2, 1, 4, 1, 4, 1, 2, 2, 4, 2, 1, 3, 3}},  // 204 values, 483 operations
+    {{0, 0, 0, 0, 1, 1, 1, 5, 0, 2, 0, 5, 1, 4, 7, 5}},  // 270 values, 601 operations
+    {{0, 0, 0, 3, 0, 1, 1, 3, 0, 0, 0, 4, 0, 6, 5, 9}},  // 308 values, 671 operations
+    {{0, 0, 0, 0, 0, 0, 1, 5, 0, 0, 0, 4, 0, 4, 3, 15}},  // 372 values, 791 operations
     // up to 36 rows
-    {{24, 3, 3, 1, 0, 0, 2, 0, 3, 0, 0, 0, 0, 0, 0, 0}},  // 54 values, 155 operations
-    {{22, 3, 3, 1, 4, 0, 0, 0, 2, 1, 0, 0, 0, 0, 0, 0}},  // 54 values, 171 operations
-    {{20, 3, 3, 1, 4, 0, 1, 0, 2, 2, 0, 0, 0, 0, 0, 0}},  // 60 values, 185 operations
-    {{12, 6, 5, 1, 5, 0, 1, 0, 3, 1, 1, 0, 1, 0, 0, 0}},  // 70 values, 217 operations
-    {{10, 4, 1, 3, 4, 2, 2, 0, 2, 1, 3, 1, 2, 0, 1, 0}},  // 100 values, 283 operations
-    {{6, 3, 3, 5, 2, 3, 2, 1, 3, 1, 2, 0, 2, 2, 1, 0}},  // 120 values, 327 operations
-    {{4, 2, 3, 3, 2, 3, 4, 2, 4, 4, 0, 1, 2, 1, 1, 0}},  // 130 values, 345 operations
-    {{4, 2, 3, 5, 3, 2, 2, 2, 2, 4, 0, 2, 2, 1, 2, 0}},  // 140 values, 365 operations
-    {{3, 3, 2, 5, 3, 2, 1, 2, 0, 2, 4, 1, 2, 3, 2, 1}},  // 163 values, 414 operations
-    {{2, 2, 2, 3, 2, 3, 2, 3, 1, 1, 3, 3, 3, 3, 2, 1}},  // 180 values, 451 operations
-    {{0, 1, 1, 2, 1, 4, 1, 5, 0, 3, 4, 3, 1, 4, 4, 2}},  // 226 values, 542 operations
-    {{1, 1, 0, 1, 0, 0, 2, 6, 1, 3, 0, 5, 0, 5, 6, 5}},  // 285 values, 646 operations
-    {{0, 0, 0, 1, 0, 1, 1, 6, 0, 1, 0, 6, 0, 4, 4, 12}},  // 368 values, 812 operations
-    {{0, 0, 0, 0, 0, 1, 1, 4, 0, 0, 0, 5, 0, 3, 3, 19}},  // 432 values, 932 operations
+    {{25, 2, 0, 2, 4, 0, 0, 0, 3, 0, 0, 0, 0, 0, 0, 0}},  // 51 values, 135 operations
+    {{21, 5, 3, 0, 2, 0, 1, 0, 4, 0, 0, 0, 0, 0, 0, 0}},  // 53 values, 157 operations
+    {{19, 4, 3, 1, 3, 0, 1, 0, 5, 0, 0, 0, 0, 0, 0, 0}},  // 57 values, 167 operations
+    {{17, 4, 5, 1, 4, 0, 0, 0, 2, 2, 0, 0, 1, 0, 0, 0}},  // 63 values, 181 operations
+    {{7, 7, 5, 1, 5, 0, 1, 0, 5, 2, 0, 0, 3, 0, 0, 0}},  // 79 values, 223 operations
+    {{11, 4, 3, 3, 2, 0, 2, 1, 3, 2, 0, 0, 3, 1, 1, 0}},  // 99 values, 259 operations
+    {{7, 5, 4, 2, 4, 0, 3, 1, 2, 3, 1, 0, 2, 1, 1, 0}},  // 105 values, 279 operations
+    {{5, 2, 4, 4, 4, 3, 3, 0, 4, 2, 2, 0, 2, 1, 0, 0}},  // 105 values, 285 operations
+    {{5, 4, 6, 2, 2, 2, 3, 1, 2, 3, 0, 1, 3, 1, 1, 0}},  // 117 values, 305 operations
+    {{5, 3, 3, 4, 1, 4, 3, 0, 0, 3, 4, 1, 4, 1, 0, 0}},  // 123 values, 321 operations
+    {{3, 2, 4, 4, 2, 2, 3, 2, 3, 3, 2, 0, 4, 1, 1, 0}},  // 129 values, 335 operations
+    {{2, 0, 2, 6, 0, 4, 4, 1, 4, 4, 2, 1, 4, 1, 1, 0}},  // 142 values, 358 operations
+    {{3, 3, 3, 3, 1, 4, 3, 2, 1, 3, 4, 0, 2, 2, 2, 0}},  // 143 values, 363 operations
+    {{2, 2, 3, 6, 3, 2, 2, 2, 1, 3, 2, 1, 3, 3, 1, 0}},  // 148 values, 374 operations
+    {{3, 2, 1, 4, 3, 4, 2, 2, 2, 3, 4, 0, 1, 1, 3, 1}},  // 155 values, 387 operations
+    {{0, 1, 2, 2, 0, 1, 3, 7, 1, 5, 3, 2, 2, 4, 2, 1}},  // 208 values, 493 operations
+    {{0, 0, 2, 2, 0, 4, 2, 5, 0, 5, 3, 3, 1, 3, 4, 2}},  // 224 values, 521 operations
+    {{2, 1, 0, 3, 0, 2, 1, 5, 1, 3, 1, 4, 0, 5, 4, 4}},  // 254 values, 578 operations
+    {{0, 0, 0, 1, 1, 0, 5, 5, 0, 1, 2, 4, 2, 6, 3, 6}},  // 286 values, 641 operations
+    {{0, 0, 0, 2, 0, 2, 1, 5, 0, 2, 0, 5, 0, 3, 5, 11}},  // 348 values, 759 operations
+    {{0, 0, 0, 2, 0, 0, 0, 5, 0, 1, 0, 3, 0, 4, 5, 16}},  // 404 values, 863 operations
+    {{0, 0, 0, 0, 0, 1, 0, 4, 0, 0, 0, 5, 0, 3, 4, 19}},  // 436 values, 923 operations
     // up to 40 rows
-    {{25, 4, 4, 0, 3, 0, 0, 0, 3, 1, 0, 0, 0, 0, 0, 0}},  // 57 values, 178 operations
-    {{21, 5, 5, 0, 4, 0, 0, 0, 4, 1, 0, 0, 0, 0, 0, 0}},  // 61 values, 190 operations
-    {{18, 5, 4, 1, 5, 0, 1, 0, 3, 2, 0, 0, 1, 0, 0, 0}},  // 72 values, 215 operations
-    {{11, 6, 5, 2, 5, 2, 1, 0, 5, 1, 1, 0, 1, 0, 0, 0}},  // 85 values, 256 operations
-    {{6, 6, 4, 2, 2, 5, 2, 1, 4, 1, 4, 0, 3, 0, 0, 0}},  // 114 values, 319 operations
-    {{4, 4, 4, 3, 2, 5, 4, 1, 2, 4, 4, 0, 2, 0, 1, 0}},  // 132 values, 357 operations
-    {{4, 2, 4, 5, 3, 3, 4, 1, 3, 3, 2, 1, 3, 2, 0, 0}},  // 140 values, 373 operations
-    {{6, 4, 3, 3, 1, 3, 4, 1, 2, 3, 1, 2, 3, 1, 3, 0}},  // 150 values, 391 operations
-    {{3, 4, 1, 2, 3, 4, 5, 1, 2, 2, 4, 4, 2, 2, 1, 0}},  // 163 values, 420 operations
-    {{2, 1, 1, 3, 1, 4, 5, 4, 1, 5, 2, 3, 1, 3, 4, 0}},  // 202 values, 499 operations
-    {{4, 1, 2, 3, 1, 4, 3, 3, 1, 3, 2, 3, 2, 3, 3, 2}},  // 210 values, 513 operations
-    {{0, 2, 0, 3, 0, 4, 3, 3, 0, 1, 3, 6, 3, 3, 3, 6}},  // 288 values, 666 operations
-    {{0, 2, 0, 1, 0, 1, 0, 8, 0, 1, 1, 5, 0, 5, 7, 9}},  // 364 values, 810 operations
-    {{0, 0, 0, 1, 0, 0, 0, 6, 0, 0, 1, 4, 0, 5, 4, 19}},  // 464 values, 1000 operations
+    {{28, 4, 3, 0, 3, 0, 0, 0, 2, 0, 0, 0, 0, 0, 0, 0}},  // 52 values, 152 operations
+    {{23, 4, 4, 1, 4, 0, 0, 0, 4, 0, 0, 0, 0, 0, 0, 0}},  // 59 values, 171 operations
+    {{19, 6, 5, 0, 5, 0, 0, 0, 2, 1, 0, 0, 2, 0, 0, 0}},  // 67 values, 191 operations
+    {{17, 7, 4, 1, 4, 0, 2, 0, 3, 0, 0, 0, 2, 0, 0, 0}},  // 73 values, 205 operations
+    {{13, 6, 5, 3, 4, 0, 1, 0, 4, 1, 0, 0, 2, 1, 0, 0}},  // 87 values, 237 operations
+    {{10, 6, 4, 3, 4, 1, 2, 1, 4, 1, 2, 0, 1, 1, 0, 0}},  // 102 values, 278 operations
+    {{7, 5, 5, 3, 4, 2, 2, 0, 3, 2, 3, 1, 2, 1, 0, 0}},  // 113 values, 303 operations
+    {{6, 4, 3, 2, 3, 4, 4, 1, 3, 4, 3, 0, 2, 0, 1, 0}},  // 124 values, 326 operations
+    {{4, 4, 3, 2, 5, 4, 2, 1, 3, 3, 4, 1, 3, 0, 1, 0}},  // 130 values, 340 operations
+    {{4, 2, 6, 3, 3, 4, 3, 2, 3, 3, 3, 1, 2, 1, 0, 0}},  // 136 values, 352 operations
+    {{4, 3, 5, 3, 2, 3, 5, 1, 1, 5, 0, 2, 4, 1, 1, 0}},  // 146 values, 368 operations
+    {{4, 3, 2, 3, 3, 2, 3, 2, 4, 4, 2, 3, 3, 1, 1, 0}},  // 152 values, 384 operations
+    {{3, 4, 2, 3, 3, 2, 4, 2, 2, 1, 2, 4, 5, 1, 2, 0}},  // 165 values, 411 operations
+    {{0, 5, 4, 4, 2, 3, 3, 2, 1, 2, 3, 3, 3, 3, 2, 0}},  // 176 values, 435 operations
+    {{0, 2, 2, 3, 0, 5, 2, 4, 3, 3, 4, 3, 5, 1, 2, 1}},  // 198 values, 477 operations
+    {{2, 2, 1, 4, 2, 4, 3, 3, 1, 2, 3, 4, 3, 2, 2, 2}},  // 210 values, 502 operations
+    {{0, 1, 1, 3, 0, 3, 4, 4, 0, 3, 2, 6, 2, 5, 4, 2}},  // 256 values, 591 operations
+    {{3, 0, 0, 2, 0, 2, 2, 5, 1, 2, 2, 5, 0, 5, 5, 6}},  // 301 values, 673 operations
+    {{0, 0, 0, 1, 0, 0, 2, 9, 0, 0, 2, 6, 2, 6, 4, 8}},  // 356 values, 779 operations
+    {{1, 0, 0, 0, 0, 0, 0, 5, 1, 4, 2, 5, 0, 5, 5, 12}},  // 379 values, 819 operations
+    {{0, 0, 0, 3, 0, 1, 0, 5, 0, 0, 0, 4, 0, 4, 4, 19}},  // 456 values, 971 operations
+    {{1, 0, 0, 0, 0, 0, 1, 3, 0, 1, 0, 5, 0, 4, 4, 21}},  // 473 values, 1007 operations
 };
 
 // Classes in the order the kernel multiplies them (ryser_cube.cuh).
@@ -146,6 +152,21 @@ PERM_HD constexpr int cube_values(const CubeShape& s) {
   for (int t = 0; t < 16; t++) n += s.rows[t] << cube_bits(t);
   return n;
 }
-constexpr int kCubeMaxSums = 256;  // largest number of fast-column sums of a shape
+constexpr int kCubeMaxSums = 256;  // at least the fast-column sums of any shape
+// Integer walks: rows of a class outside its int32 runs of 4 and 3 rows,
+// their first FP64 sum (2^|T| / 2 per row), and the factors of a term (runs
+// and left-over rows).
+PERM_HD constexpr int cube_left(int rows) { return rows % 4 == 3 ? 0 : rows % 4; }
+PERM_HD constexpr int cube_left_sum(const CubeShape& s, int i) {
+  int n = 0;
+  for (int t = 0; t < i; t++) n += cube_left(s.rows[cube_class(t)]) * ((1 << cube_bits(cube_class(t))) / 2);
+  return n;
+}
+PERM_HD constexpr int cube_factors(const CubeShape& s) {
+  int n = 0;
+  for (int t = 0; t < 16; t++) n += (s.rows[t] + 1) / 4 + cube_left(s.rows[t]);
+  return n;
+}
+constexpr int kCubeMaxWide = 84;  // 2 rows in each of the 16 classes: 2 x 80 / 2
 
 }  // namespace perm

@@ -130,18 +130,19 @@ const void* sdd_3l_kernel_r20(int n, int r1);
 const void* sdd_3l_kernel_r24(int n, int r1);
 const void* sdd_3l_kernel_r28(int n, int r1);
 
-const void* cube_f64_n20(int i);
-const void* cube_f64_n24(int i);
-const void* cube_f64_n28(int i);
-const void* cube_f64_n32(int i);
-const void* cube_f64_n36(int i);
-const void* cube_f64_n40(int i);
-const void* cube_sdd_n20(int i);
-const void* cube_sdd_n24(int i);
-const void* cube_sdd_n28(int i);
-const void* cube_sdd_n32(int i);
-const void* cube_sdd_n36(int i);
-const void* cube_sdd_n40(int i);
+// ryser_cube_<kind>_n<size>.cu
+#define PERM_CUBE_KIND(kind)            \
+  const void* cube_##kind##_n28(int i); \
+  const void* cube_##kind##_n32(int i); \
+  const void* cube_##kind##_n36(int i); \
+  const void* cube_##kind##_n40(int i);
+PERM_CUBE_KIND(f64)
+PERM_CUBE_KIND(f64a)
+PERM_CUBE_KIND(sdd)
+PERM_CUBE_KIND(int)
+PERM_CUBE_KIND(inta)
+PERM_CUBE_KIND(intc)
+#undef PERM_CUBE_KIND
 const void* dense_tc_kernel_g3(int n);
 const void* dense_tc_kernel_g4(int n);
 const void* dense_tc_kernel_g5(int n);
@@ -152,14 +153,17 @@ static int cube_size(int shape) {
   while (shape >= kCubeFirst[i + 1]) i++;
   return i;
 }
-static const void* cube_kernel(int shape, bool pair) {
+// kinds of column-cube walks, in the order of their occupancy tables
+enum CubeKind { kCubeF64, kCubeF64Abs, kCubeSdd, kCubeInt, kCubeIntAbs, kCubeIntc, kCubeKinds };
+static const void* cube_kernel(int shape, int kind) {
   using Pick = const void* (*)(int);
-  static const Pick f64[kCubeSizeCount] = {cube_f64_n20, cube_f64_n24, cube_f64_n28,
-                                           cube_f64_n32, cube_f64_n36, cube_f64_n40};
-  static const Pick sdd[kCubeSizeCount] = {cube_sdd_n20, cube_sdd_n24, cube_sdd_n28,
-                                           cube_sdd_n32, cube_sdd_n36, cube_sdd_n40};
+#define PERM_CUBE_KIND(kind) \
+  {cube_##kind##_n28, cube_##kind##_n32, cube_##kind##_n36, cube_##kind##_n40}
+  static const Pick pick[kCubeKinds][kCubeSizeCount] = {PERM_CUBE_KIND(f64), PERM_CUBE_KIND(f64a), PERM_CUBE_KIND(sdd),
+                                                        PERM_CUBE_KIND(int), PERM_CUBE_KIND(inta), PERM_CUBE_KIND(intc)};
+#undef PERM_CUBE_KIND
   const int i = cube_size(shape);
-  return (pair ? sdd : f64)[i](shape - kCubeFirst[i]);
+  return pick[kind][i](shape - kCubeFirst[i]);
 }
 
 static const void* dense_tc_kernel(int n, int g) {
@@ -509,7 +513,7 @@ struct perm_ctx {
   // + ngo - 1] int32-X in the two-level row layout, [34 + 3 family + ngo - 1]
   // certified int32-X in the two-level layout
   int dense_occ[122][PERM_MAX_EXACT_N + 1] = {};
-  int cube_occ[2][kCubeShapeCount] = {};         // column-cube walks: [0] FP64, [1] split-dd
+  int cube_occ[kCubeKinds][kCubeShapeCount] = {};  // column-cube walks
   int batch_m[kBatchMaxOrder + 1] = {};          // autotuned lane-range exponents (0: default)
   int dense_pref[PERM_MAX_EXACT_N + 1] = {};     // autotuned kernel for integer inputs (0: built-in choice)
   double rel_target = 1e-10;                     // rerun in double-double above this estimate (<=0: never)
@@ -1130,7 +1134,7 @@ static void sdd_choose(const std::vector<double>& a, int n, int* inner, int* inn
 // instructions; G in 4..6 up to the one-level G; the cheapest layout below
 // `best_cost` whose groups provably fit int32.
 static bool int_three_level_layout(const std::vector<double>& a, int n, int g1, long best_cost, int* g_out,
-                                   int* ng1_out, int* ng2_out, std::vector<double>* perm) {
+                                   int* ng1_out, int* ng2_out, std::vector<double>* perm, long* cost_out) {
   if (g1 < 4) return false;
   long best = best_cost;
   for (int g = std::min(g1, 6); g >= 4; g--) {
@@ -1148,6 +1152,7 @@ static bool int_three_level_layout(const std::vector<double>& a, int n, int g1, 
     *ng2_out = ng2;
     *perm = std::move(p);
   }
+  *cost_out = best;
   return best != best_cost;
 }
 
@@ -1158,7 +1163,8 @@ static bool int_three_level_layout(const std::vector<double>& a, int n, int g1, 
 struct IntLayout {
   int g, ngo, ng1, ng2;
 };
-static IntLayout choose_int_layout(const std::vector<double>& a, int n, int G, std::vector<double>* perm) {
+static IntLayout choose_int_layout(const std::vector<double>& a, int n, int G, std::vector<double>* perm,
+                                   long* cost_out = nullptr) {
   IntLayout l = {G, 0, 0, 0};
   long cost = 8L * (2 * n + (n + G - 1) / G);
   int g2 = G, ngo2 = 0, g3 = G, a1 = 0, a2 = 0;
@@ -1167,13 +1173,14 @@ static IntLayout choose_int_layout(const std::vector<double>& a, int n, int G, s
     const int ri = n - g2 * ngo2;
     cost = 7L * (2 * ri + (ri + g2 - 1) / g2 + 1) + 2 * n + (n + g2 - 1) / g2 + ngo2;
   }
-  if (int_three_level_layout(a, n, G, cost, &g3, &a1, &a2, &three)) {
+  if (int_three_level_layout(a, n, G, cost, &g3, &a1, &a2, &three, &cost)) {
     l = {g3, 0, a1, a2};
     *perm = std::move(three);
   } else if (ngo2) {
     l = {g2, ngo2, 0, 0};
     *perm = std::move(two);
   }
+  if (cost_out) *cost_out = cost;
   return l;
 }
 
@@ -1294,7 +1301,7 @@ static bool intc_two_level_layout(const std::vector<double>& a, int n, long one_
 // c the level costs of intc_two_level_layout; the cheapest below
 // `best_cost` whose groups (< 2^31) and pairs (< 2^53) provably fit.
 static bool intc_three_level_layout(const std::vector<double>& a, int n, long best_cost, int* g_out, int* pair_out,
-                                    int* ng1_out, int* ng2_out, std::vector<double>* perm) {
+                                    int* ng1_out, int* ng2_out, std::vector<double>* perm, long* cost_out = nullptr) {
   long best = best_cost;
   const int fam_g[3] = {4, 5, 6};
   const bool fam_pair[3] = {true, false, true};
@@ -1336,6 +1343,7 @@ static bool intc_three_level_layout(const std::vector<double>& a, int n, long be
     *ng2_out = ng2;
     *perm = std::move(p);
   }
+  if (cost_out) *cost_out = best;
   return best != best_cost;
 }
 
@@ -1346,6 +1354,16 @@ static void build_fp64_image(const std::vector<double>& a, int n, DenseOperand* 
   double* img = reinterpret_cast<double*>(op->image.data());
   for (int k = 0; k < n; k++)
     for (int j = 0; j < n; j++) img[(size_t)k * np + j] = a[(size_t)j * n + k];
+}
+
+// Sum of a row's entries in the fast columns of set `cls`; bit b of `signs` is
+// the sign of the set's b-th column (1: plus).
+template <class Entry>
+static double fast_sum(int cls, int signs, Entry entry) {
+  double t = 0.0;
+  for (int k = 0, b = 0; k < 4; k++)
+    if ((cls >> k) & 1) t += ((signs >> b++) & 1) ? entry(k) : -entry(k);
+  return t;
 }
 
 // Turns the column-major image of a cube layout's matrix (`parts` column sets
@@ -1379,34 +1397,92 @@ static void build_cube_operand(const CubeLayout& l, int parts, DenseOperand* op)
         const int j = l.slot_row[cube_slot(shape, i) + r];
         if (j < 0) continue;
         for (int s = 0; s < half; s++) {
-          double t = 0.0;  // the last column of the set has sign plus
-          for (int k = 0, b = 0; k < 4; k++) {
-            if (!((cls >> k) & 1)) continue;
-            const double c = 0.5 * from[(size_t)k * np + j];
-            t += (s + half) >> b++ & 1 ? c : -c;
-          }
-          op->sums[(size_t)part * kCubeMaxSums + cube_sum(shape, i) + r * half + s] = t;
+          op->sums[(size_t)part * kCubeMaxSums + cube_sum(shape, i) + r * half + s] =
+              fast_sum(cls, s + half, [&](int k) { return 0.5 * from[(size_t)k * np + j]; });
         }
       }
     }
   }
 }
 
+// The integer walks' operand (int32 columns; slots without a row hold y = 1),
+// when the products that the kernel forms in int32 (runs of 4 and 3 rows,
+// below 2^31) and, for the certified walk, keeps in FP64 as exact (any
+// kCubeExactRows rows, below 2^53) provably fit.
+static bool build_cube_int_operand(const CubeLayout& l, DenseOperand* op) {
+  const int n = op->n, nc = n - 4;
+  const CubeShape& shape = kCubeShapes[l.shape];
+  const int N = cube_rows(shape);
+  std::vector<double> rowabs;
+  if (!int_row_abs(l.mat, n, rowabs)) return false;
+  for (int i = 0; i < 16; i++) {
+    const int rows = shape.rows[cube_class(i)], runs = rows - cube_left(rows);
+    for (int r = 0; r < runs; r += 4) {
+      double b = 1.0;
+      for (int t = r; t < std::min(r + 4, runs); t++) {
+        const int j = l.slot_row[cube_slot(shape, i) + t];
+        if (j >= 0) b *= std::max(rowabs[j], 1.0);
+      }
+      if (!(b < 2147483648.0)) return false;
+    }
+  }
+  if (op->variant == PERM_KERNEL_DENSE_INT_DD) {
+    std::vector<double> large = rowabs;
+    std::sort(large.begin(), large.end(), std::greater<double>());
+    double b = 1.0;
+    for (int t = 0; t < kCubeExactRows; t++) b *= std::max(large[t], 1.0);
+    if (!(b < 9007199254740992.0)) return false;
+  }
+  op->shape = l.shape;
+  op->image.assign(sizeof(int) * (size_t)nc * N, 0);
+  int* img = reinterpret_cast<int*>(op->image.data());
+  for (int slot = 0; slot < N; slot++) {
+    const int j = l.slot_row[slot];
+    for (int k = 0; k < nc; k++)
+      img[(size_t)k * N + slot] = j >= 0 ? (int)l.mat[(size_t)j * n + k + 4] : k == nc - 1 ? 1 : 0;
+  }
+  // every row's sums, then those of the rows left over from the runs
+  op->sums.assign(kCubeMaxSums + kCubeMaxWide, 0.0);
+  for (int i = 1; i < 16; i++) {
+    const int cls = cube_class(i), half = (1 << cube_bits(cls)) / 2, runs = shape.rows[cls] - cube_left(shape.rows[cls]);
+    for (int r = 0; r < shape.rows[cls]; r++) {
+      const int j = l.slot_row[cube_slot(shape, i) + r];
+      if (j < 0) continue;
+      for (int s = 0; s < half; s++) {
+        const double t = fast_sum(cls, s + half, [&](int k) { return l.mat[(size_t)j * n + k]; });
+        op->sums[cube_sum(shape, i) + r * half + s] = t;
+        if (r >= runs) op->sums[kCubeMaxSums + cube_left_sum(shape, i) + (r - runs) * half + s] = t;
+      }
+    }
+  }
+  return true;
+}
+
 static int build_sdd_operand(perm_ctx* ctx, const std::vector<double>& a, int n, DenseOperand* op) {
   if (n < 4 || n > 40) return fail(ctx, PERM_EUNSUPPORTED, "split-dd kernel covers orders 4..40 (got %d)", n);
+  // The column-cube walk (6 operations per row value, 2 per row and about 280
+  // for the class arrays and the sum, per 16 terms; 0.63 of the FP64 pipe)
+  // unless a row layout is cheaper (per 8 terms, 0.69 dense, 0.56..0.62 the
+  // others).  n = 30: 364 values 7.3 ms, dense layout 8.9 ms.  The smallest
+  // row layout (sparse, 6 rows) needs 320 + 6n operations per 8 terms.
   CubeLayout l;
-  // any shape that fits: 6 operations per row value at 0.63 of the FP64 pipe
-  // cost less than the row layouts' 6 per row and term at 0.56..0.69 (n = 30,
-  // 364 values: 7.3 ms against 8.9 ms in the dense layout)
-  if (n >= kCubeMinN && cube_layout(a, n, 1e9, &l)) {
+  int inner = 0, inner1 = 0;
+  std::vector<double> perm;
+  bool cube = n >= kCubeMinN && cube_layout(a, n, 1e9, &l);
+  if (cube) {
+    const double mine = (6.0 * cube_values(kCubeShapes[l.shape]) + 2.0 * n + 280.0) / 0.63;
+    if (mine > 2.0 * (320.0 + 6.0 * n) / 0.62) {
+      sdd_choose(a, n, &inner, &inner1, &perm);
+      cube = mine < 2.0 * (double)sdd_cost(n, inner, inner1, inner) / (inner ? 0.62 : 0.69);
+    }
+  }
+  if (cube) {
     const int rc = build_split_operand(ctx, l.mat, n, op);
     if (rc) return rc;
     op->variant = PERM_KERNEL_DENSE_SDD;
     build_cube_operand(l, 2, op);
     return PERM_OK;
   }
-  int inner = 0, inner1 = 0;
-  std::vector<double> perm;
   sdd_choose(a, n, &inner, &inner1, &perm);
   const int rc = build_split_operand(ctx, inner ? perm : a, n, op);
   if (rc) return rc;
@@ -1444,6 +1520,34 @@ static int build_operand(perm_ctx* ctx, const void* mat, int n, int dtype, int v
     op->ngo = 0;
     op->ng1 = op->ng2 = 0;
     std::vector<double> two;
+    CubeLayout cube;
+    const bool certified = op->variant == PERM_KERNEL_DENSE_INT_DD;
+    if (n >= kCubeMinN && op->variant != PERM_KERNEL_DENSE_TC && cube_layout(a, n, 1e9, &cube)) {
+      // Against the row layouts' instructions per 8 terms, in cycles per SM,
+      // warp and 16 terms: those issue 0.8 of 4 per cycle (0.77 each; the
+      // certified walk's, 0.95), the cube takes 0.47 per unit of its cost
+      // (certified: 100 + 0.68), measured over the shapes.  The several-level
+      // layouts need 0.6 of the one-level instructions at density 1/2, and
+      // the cube less still where they need less; only above that are they
+      // searched for (0.2 ms on the host at n = 30).
+      const double mine = certified ? 100.0 + 0.68 * cube.cost : 0.47 * cube.cost;
+      const double each = certified ? 0.95 : 0.77;
+      int pair = 0, cost1 = 0, g = 0, x = 0, y = 0;
+      if (certified) intc_layout(a, n, &pair, &cost1);
+      long cost = certified ? 8L * (n + cost1) : 8L * (2 * n + (n + G - 1) / G);
+      bool take = mine < each * 0.6 * (double)cost;
+      if (!take) {
+        std::vector<double> p;
+        if (certified) {
+          intc_two_level_layout(a, n, cost, &g, &pair, &x, &p, &cost);
+          intc_three_level_layout(a, n, cost, &g, &pair, &x, &y, &p, &cost);
+        } else {
+          choose_int_layout(a, n, G, &p, &cost);
+        }
+        take = mine < each * (double)cost;
+      }
+      if (take && build_cube_int_operand(cube, op)) return PERM_OK;
+    }
     if (op->variant == PERM_KERNEL_DENSE_INT_DD) {
       int cost1 = 0;
       op->group = intc_layout(a, n, &op->pair, &cost1);
@@ -1521,8 +1625,14 @@ struct perm_matrix {
   void* d_image = nullptr;
 };
 
+static int cube_kind(const DenseOperand& op) {
+  return op.variant == PERM_KERNEL_DENSE_SDD      ? kCubeSdd
+         : op.variant == PERM_KERNEL_DENSE_INT    ? kCubeInt
+         : op.variant == PERM_KERNEL_DENSE_INT_DD ? kCubeIntc
+                                                  : kCubeF64;
+}
 static const void* operand_kernel(const DenseOperand& op) {
-  if (op.shape >= 0) return cube_kernel(op.shape, op.variant == PERM_KERNEL_DENSE_SDD);
+  if (op.shape >= 0) return cube_kernel(op.shape, cube_kind(op));
   if (op.variant == PERM_KERNEL_DENSE_INT)
     return op.ng1 ? dense_int_3l_kernel(op.n, op.group, op.ng1, op.ng2)
            : op.ngo ? dense_int_sparse_kernel(op.n, op.group, op.ngo)
@@ -1540,11 +1650,14 @@ static const void* operand_kernel(const DenseOperand& op) {
                     : dense_kernel(op.n);
 }
 static int operand_threads(const DenseOperand& op) {
-  return op.shape >= 0 ? kCubeThreads : op.variant == PERM_KERNEL_DENSE_TC ? kTcThreads : 128;
+  if (op.shape >= 0) return kCubeThreads;
+  return op.variant == PERM_KERNEL_DENSE_TC ? kTcThreads : 128;
 }
 static size_t operand_smem(const DenseOperand& op) {
   if (op.shape >= 0)
-    return cube_smem_bytes(op.variant == PERM_KERNEL_DENSE_SDD, op.n, cube_rows(kCubeShapes[op.shape]));
+    return cube_smem_bytes(cube_rows(kCubeShapes[op.shape]),
+                           cube_kind(op) >= kCubeInt ? sizeof(int) : (cube_kind(op) == kCubeSdd ? 2 : 1) * sizeof(double),
+                           op.n, cube_kind(op) == kCubeSdd);
   if (op.variant == PERM_KERNEL_DENSE_INT || op.variant == PERM_KERNEL_DENSE_INT_DD) return dense_int_smem_bytes(op.n);
   if (op.variant == PERM_KERNEL_DENSE_SDD)
     return op.inner ? sparse_sdd_smem_bytes(op.n, op.inner, 128) : dense_sdd_smem_bytes(op.n);
@@ -1668,8 +1781,7 @@ static int dense_plan(perm_ctx* ctx, const DenseOperand& op, int shard, int nsha
   }
   for (int i = 0; i < 5; i++)
     if (op.inner1 && op.inner == kFp3lR2[i]) fp_slot = 102 + 4 * i + op.inner1 / 4 - 2;
-  const bool pair = op.variant == PERM_KERNEL_DENSE_SDD;
-  int& occ_slot = op.shape >= 0 ? ctx->cube_occ[pair][op.shape] : ctx->dense_occ[op.variant == PERM_KERNEL_DENSE_INT
+  int& occ_slot = op.shape >= 0 ? ctx->cube_occ[cube_kind(op)][op.shape] : ctx->dense_occ[op.variant == PERM_KERNEL_DENSE_INT
                                      ? (op.ng1 ? 50 + 6 * (op.group - 4) + 2 * (op.ng1 - 2) + op.ng2 - 1
                                         : op.ngo ? 25 + 3 * (op.group - 4) + op.ngo - 1
                                                  : op.group)
@@ -1718,7 +1830,7 @@ static int dense_plan(perm_ctx* ctx, const DenseOperand& op, int shard, int nsha
     // ranges of whole cubes.  A thread owns ceil(blocks / threads) blocks of
     // 2^m cubes at most; leaving a block costs about half a cube more, since
     // the lanes then flip different columns.
-    const uint64_t cubes = (last - first) >> 4, threads = (uint64_t)grid * kCubeThreads;
+    const uint64_t cubes = (last - first) >> 4, threads = (uint64_t)grid * operand_threads(op);
     double best = -1.0;
     for (int m = 0; m <= 10 && m <= (nshards == 1 ? n - 5 : ms - 4); m++) {
       const double each = std::ceil((double)(cubes >> m) / (double)threads);
@@ -1730,14 +1842,17 @@ static int dense_plan(perm_ctx* ctx, const DenseOperand& op, int shard, int nsha
     }
     p->block0 = first >> p->m;
     p->nblocks = (last - first) >> p->m;
-    p->grid = (int)std::min<uint64_t>((uint64_t)grid, std::max<uint64_t>(1, (p->nblocks + kCubeThreads - 1) / kCubeThreads));
+    p->grid = (int)std::min<uint64_t>((uint64_t)grid, std::max<uint64_t>(1, (p->nblocks + operand_threads(op) - 1) / operand_threads(op)));
     return PERM_OK;
   }
   // Alignment m <= ms: each thread should own >= 64 aligned blocks when possible.
   const uint64_t len = last - first;
   const uint64_t threads = (uint64_t)grid * 128;
+  // FP64 X is recomputed at block boundaries, at most every 2^12 steps (at
+  // 2^20 an order-40 walk drifted past its own error bound).
   int m = 3;
-  while (m < 20 && m < ms && (len >> (m + 1)) >= threads * 64) m++;
+  const int m_max = op.variant == PERM_KERNEL_DENSE ? 12 : 20;
+  while (m < m_max && m < ms && (len >> (m + 1)) >= threads * 64) m++;
   const uint64_t mine = len >> m;
   if (mine < (uint64_t)grid * 128) grid = (int)std::max<uint64_t>(1, (mine + 127) / 128);
   p->grid = grid;
@@ -1751,27 +1866,38 @@ static int dense_launch(perm_ctx* ctx, const DenseOperand& op, const void* d_ima
   const int n = op.n;
   CU(ctx, cudaEventRecord(ctx->ev0, ctx->stream));
   if (op.shape >= 0) {
-    CubeArgs args;
-    args.img = static_cast<const double*>(d_image);
+    const int kind = cube_kind(op);
+    union {
+      CubeArgs f64;
+      CubeSddArgs sdd;
+      CubeIntArgs integer;
+    } u;
+    CubeWalk& args = u.f64;  // every form begins with it
+    args.img = d_image;
     args.n = n;
     args.m = p.m - 4;
     args.block0 = p.block0;
     args.nblocks = p.nblocks;
-    args.seg = kCubeSegment;
+    args.seg = kind >= kCubeInt ? ~0ull : kCubeSegment;
     args.partials = ctx->partials;
     args.ticket = ctx->ticket;
     args.out = ctx->d_out;
     args.sums = ctx->d_est;
     args.err = ctx->d_err;
-    args.inject = ctx->inject_timeouts > 0 && op.variant == PERM_KERNEL_DENSE ? 16u : 0u;
+    args.inject = ctx->inject_timeouts > 0 && kind == kCubeF64 ? 16u : 0u;
     if (args.inject) ctx->inject_timeouts--;
-    memcpy(args.c, op.sums.data(), sizeof args.c);
-    if (op.variant == PERM_KERNEL_DENSE_SDD) {
-      memcpy(args.cl, op.sums.data() + kCubeMaxSums, sizeof args.cl);
-      CU(ctx, cudaMemsetAsync(ctx->d_est, 0, 2 * sizeof(double), ctx->stream));
+    if (kind >= kCubeInt) {
+      for (int i = 0; i < kCubeMaxSums; i++) u.integer.ci[i] = (int)op.sums[i];
+      memcpy(u.integer.cd, op.sums.data() + kCubeMaxSums, sizeof u.integer.cd);
+    } else {
+      memcpy(u.f64.c, op.sums.data(), sizeof u.f64.c);
+      if (kind == kCubeSdd) memcpy(u.sdd.cl, op.sums.data() + kCubeMaxSums, sizeof u.sdd.cl);
     }
-    void* kargs[] = {&args};
-    CU(ctx, cudaLaunchKernel(operand_kernel(op), dim3(p.grid), dim3(kCubeThreads), kargs, operand_smem(op), ctx->stream));
+    void* kargs[] = {&u};
+    if (kind == kCubeSdd || kind == kCubeIntc)
+      CU(ctx, cudaMemsetAsync(ctx->d_est, 0, 2 * sizeof(double), ctx->stream));
+    CU(ctx, cudaLaunchKernel(operand_kernel(op), dim3(p.grid), dim3(operand_threads(op)), kargs, operand_smem(op),
+                             ctx->stream));
   } else if (op.variant == PERM_KERNEL_DENSE_TC) {
     DenseTcArgs args;
     args.colI = static_cast<const int*>(d_image);
@@ -1950,7 +2076,8 @@ struct ErrEstimate {
 // bounds of `variant`'s rounding error from the sums of |term| and term^2
 // (sampled, or the walk's own); k_terms = the longest thread range of a
 // certified walk
-static void error_bounds(int variant, int group, int n, double value, ErrEstimate* e, uint64_t k_terms = 0) {
+static void error_bounds(int variant, int group, int n, double value, ErrEstimate* e, uint64_t k_terms = 0,
+                         int shape = -1) {
   const double u = std::ldexp(1.0, -53);
   const double av = std::fabs(value), s1 = e->s1, s2 = e->s2;
   if (av == 0.0) {
@@ -1959,10 +2086,13 @@ static void error_bounds(int variant, int group, int n, double value, ErrEstimat
   }
   if (variant == PERM_KERNEL_DENSE_INT_DD || variant == PERM_KERNEL_DENSE_SDD) {
     const double k = (double)k_terms;
-    const double prod = variant == PERM_KERNEL_DENSE_INT_DD ? 8.0 * std::ceil((double)n / group) : 8.0 * n;
+    // the column-cube walks take at most n + 5 factors (the rows and the
+    // class arrays they are merged through) and sum cubes of 16 terms first
+    const bool chain = variant == PERM_KERNEL_DENSE_INT_DD && shape < 0;
+    const double prod = chain ? 8.0 * std::ceil((double)n / group) : 8.0 * (shape < 0 ? n : n + 5);
     // low-part rounding: the int32-X walk adds every term to one (hi, lo),
     // split-dd adds groups of eight
-    const double lows = variant == PERM_KERNEL_DENSE_INT_DD ? k * k : (k / 4) * (k / 4);
+    const double lows = chain ? k * k : (k / 4) * (k / 4);
     const double drift = variant == PERM_KERNEL_DENSE_SDD ? 64.0 * n * n * k : 0.0;
     e->worst = e->random = (prod + 256.0 + lows + drift) * u * u * s1 / av;
   } else if (variant == PERM_KERNEL_DENSE_DD) {
@@ -1973,7 +2103,8 @@ static void error_bounds(int variant, int group, int n, double value, ErrEstimat
     e->worst = (2.0 * n + 16.0) * u * s1 / av;
     e->random = 4.0 * u * std::sqrt(2.0 * n / 3.0) * std::sqrt(s2) / av;
   } else if (variant == PERM_KERNEL_DENSE_INT || variant == PERM_KERNEL_DENSE_TC) {
-    const double groups = std::ceil((double)n / group);
+    // (one rounding more in the column-cube walk: the difference over column 2)
+    const double groups = shape >= 0 ? cube_factors(kCubeShapes[shape]) + 1.0 : std::ceil((double)n / group);
     e->worst = (groups + 16.0) * u * s1 / av;
     e->random = 4.0 * u * std::sqrt(std::max(1.0, groups - 1.0) / 3.0) * std::sqrt(s2) / av;
   } else {
@@ -1997,7 +2128,7 @@ static int estimate_error(perm_ctx* ctx, const void* d_col_fp64, int n, const De
   CU(ctx, cudaStreamSynchronize(ctx->stream));
   e->s1 = ctx->h_out[12] * 2.0;  // |factor| = 2
   e->s2 = ctx->h_out[13] * 4.0;
-  error_bounds(op.variant, op.group, n, value, e);
+  error_bounds(op.variant, op.group, n, value, e, 0, op.shape);
   return PERM_OK;
 }
 
@@ -2088,7 +2219,7 @@ static int refine_result(perm_ctx* ctx, const void* mat, int n, int dtype, const
       out->steps == out->total_steps) {
     ErrEstimate c;
     c.s1 = ctx->walk_m1;
-    error_bounds(op.variant, op.group, n, out->value, &c, ctx->walk_terms_per_thread);
+    error_bounds(op.variant, op.group, n, out->value, &c, ctx->walk_terms_per_thread, op.shape);
     out->abs_term_sum = c.s1;
     out->rel_error_estimate = c.worst;
     return PERM_OK;
@@ -2162,7 +2293,7 @@ static int refine_result(perm_ctx* ctx, const void* mat, int n, int dtype, const
     if ((rc = estimate_error(ctx, ctx->d_stage, n, c_op, out->value, &e))) return rc;
   } else {
     e.s1 = ctx->walk_m1;
-    error_bounds(cv, c_op.group, n, out->value, &e, ctx->walk_terms_per_thread);
+    error_bounds(cv, c_op.group, n, out->value, &e, ctx->walk_terms_per_thread, c_op.shape);
   }
   out->abs_term_sum = e.s1;
   out->rel_error_estimate = e.worst;

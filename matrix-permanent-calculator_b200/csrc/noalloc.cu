@@ -171,7 +171,7 @@ extern "C" int perm_exact_dense_noalloc(const double* d_mat, int n, double* d_ou
     if (grid > kNoAllocMaxBlocks) grid = kNoAllocMaxBlocks;
     const uint64_t threads = (uint64_t)grid * 128;
     int m = 3;
-    while (m < 20 && m < n - 1 && (total >> (m + 1)) >= threads * 64) m++;
+    while (m < 12 && m < n - 1 && (total >> (m + 1)) >= threads * 64) m++;
     const uint64_t blocks = total >> m;
     if (blocks < threads) grid = (int)((blocks + 127) / 128);
     args.m = m;

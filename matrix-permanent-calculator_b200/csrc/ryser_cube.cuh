@@ -15,9 +15,11 @@
 // of 16.  The products of a class are an array over the signs of T, which is
 // copied (widened) into the array of a larger class or multiplied into it:
 //
-//   {} > {0} > {01} (x {02}) > {012} > {0123} = top
-//   {1} > {12} (x {13}) > {123}, {2} > {23} > {023}      multiplied into top
-//   {3} > {03} > {013}: top is summed over s_2 first, then multiplied
+//   {0} > {01} (x {02}) > {012} > {0123} = top, {1} > {12} (x {13}) > {123}
+//   {2} > {23} > {023}, {} > {3} > {03} > {013}
+//
+// The first two are multiplied into top, the third with the difference over
+// the sign of column 2, the last with the sum of the rest.
 //
 // The host picks the four columns, of the matrix or of its transpose, whose
 // rows fit the cheapest of the compiled shapes (cube_shapes.h).  At density
@@ -41,6 +43,7 @@
 
 #include "cube_shapes.h"
 #include "ryser_cube.h"
+#include "ryser_dense_int.cuh"
 #include "ryser_dense_sdd.cuh"
 
 namespace perm {
@@ -57,170 +60,331 @@ __device__ constexpr int cube_drop(int s, int set, int sub) {
   return r;
 }
 
-// Product arrays and row values of a walk: FP64, or split x with
-// double-double products (pair).
-template <bool kPair>
-struct CubeNum;
-template <>
-struct CubeNum<false> {
+// A product: FP64, or a double-double pair.  kRows template arguments count
+// the rows multiplied so far: 0 means unset, and products of up to kExact rows
+// are exact in FP64 (lo is 0 and not kept).
+struct CubeF64 {
   double hi;
-  __device__ __forceinline__ void mul(const CubeNum& x) { hi = hi * x.hi; }
-};
-template <>
-struct CubeNum<true> {
-  double hi, lo;
-  __device__ __forceinline__ void mul(const CubeNum& x) {
-    dd t = {hi, lo};
-    pair_mul(t, x.hi, x.lo);
-    hi = t.hi;
-    lo = t.lo;
+  template <int kRows>
+  __device__ __forceinline__ void mul(double x) {
+    hi = hi * x;
+  }
+  template <int kRows, int kOther>
+  __device__ __forceinline__ void mul(const CubeF64& x) {
+    hi = hi * x.hi;
   }
 };
 
-template <int kSet, bool kPair>
+template <int kExact>
+struct CubeDd {
+  double hi, lo;
+  // by an exact value x of one or more rows, kRows in all afterwards
+  template <int kRows, int kBefore>
+  __device__ __forceinline__ void mul_exact(double x) {
+    const double h = __dmul_rn(hi, x);
+    if constexpr (kRows > kExact) {
+      const double e = __fma_rn(hi, x, -h);
+      lo = kBefore <= kExact ? e : __fma_rn(lo, x, e);
+    }
+    hi = h;
+  }
+  // by another product of kOther rows
+  template <int kRows, int kOther>
+  __device__ __forceinline__ void mul(const CubeDd& x) {
+    if constexpr (kOther <= kExact) {
+      mul_exact<kRows + kOther, kRows>(x.hi);
+    } else {
+      const double h = __dmul_rn(hi, x.hi);
+      double l = __fma_rn(hi, x.hi, -h);
+      l = __fma_rn(hi, x.lo, l);
+      if constexpr (kRows > kExact) l = __fma_rn(lo, x.hi, l);
+      hi = h;
+      lo = l;
+    }
+  }
+};
+
+template <int kSet, class Num>
 struct CubeArray {
   static constexpr int kW = 1 << cube_bits(kSet);
-  CubeNum<kPair> v[kW];
+  Num v[kW];
 };
 
 // to = from widened to a larger set, or multiplied into it
-template <int kTo, int kFrom, bool kPair>
-__device__ __forceinline__ void cube_widen(CubeArray<kTo, kPair>& to, const CubeArray<kFrom, kPair>& from) {
+template <int kTo, int kFrom, class Num>
+__device__ __forceinline__ void cube_widen(CubeArray<kTo, Num>& to, const CubeArray<kFrom, Num>& from) {
 #pragma unroll
-  for (int s = 0; s < CubeArray<kTo, kPair>::kW; s++) to.v[s] = from.v[cube_drop(s, kTo, kFrom)];
+  for (int s = 0; s < CubeArray<kTo, Num>::kW; s++) to.v[s] = from.v[cube_drop(s, kTo, kFrom)];
 }
-template <int kTo, int kFrom, bool kPair>
-__device__ __forceinline__ void cube_merge(CubeArray<kTo, kPair>& to, const CubeArray<kFrom, kPair>& from) {
+template <int kRows, int kOther, int kTo, int kFrom, class Num>
+__device__ __forceinline__ void cube_merge(CubeArray<kTo, Num>& to, const CubeArray<kFrom, Num>& from) {
 #pragma unroll
-  for (int s = 0; s < CubeArray<kTo, kPair>::kW; s++) to.v[s].mul(from.v[cube_drop(s, kTo, kFrom)]);
+  for (int s = 0; s < CubeArray<kTo, Num>::kW; s++)
+    to.v[s].template mul<kRows, kOther>(from.v[cube_drop(s, kTo, kFrom)]);
 }
 
-// The products of one cube, and their signed sum.  `row(slot)` returns a
-// row's b; `kShape` gives the class sizes.
-template <int kShape, bool kPair, class Row>
+// The products of one cube.  `src` multiplies the rows of a class into an
+// array: src.rows<kI, kDone>(p), kDone rows being in p already.
+template <int kShape, class Num, class Source>
 struct Cube {
-  using Num = CubeNum<kPair>;
-  const CubeArgs& a;
-  Row row;
+  const Source& src;
 
   template <int kI>
   static constexpr int count() {
-    return kCubeShapes[kShape].rows[cube_class(kI)];
+    return kI < 0 ? 0 : kCubeShapes[kShape].rows[cube_class(kI < 0 ? 0 : kI)];
   }
 
-  // multiplies the rows of class kI into p (which is unset when kFirst)
-  template <int kI, bool kFirst>
-  __device__ __forceinline__ void rows(CubeArray<cube_class(kI), kPair>& p) const {
-    constexpr int W = CubeArray<cube_class(kI), kPair>::kW, H = W / 2;
+  // {k} > {kl} (x another pair) > {klm}: classes kI0, kI1, kX (-1: none) and
+  // kI2 of the kernel order, starting from an array of kDone rows
+  template <int kI0, int kI1, int kX, int kI2>
+  static constexpr int total() {
+    return count<kI0>() + count<kI1>() + count<kX>() + count<kI2>();
+  }
+  template <int kI0, int kI1, int kX, int kI2, int kFrom, int kDone>
+  __device__ __forceinline__ void chain(CubeArray<cube_class(kI2), Num>& p3, const CubeArray<kFrom, Num>& from) const {
+    constexpr int n1 = kDone + count<kI0>(), n2 = n1 + count<kI1>(), n3 = n2 + count<kX>();
+    CubeArray<cube_class(kI0), Num> p1;
+    if constexpr (kDone > 0) cube_widen(p1, from);
+    src.template rows<kI0, kDone>(p1);
+    CubeArray<cube_class(kI1), Num> p2;
+    if constexpr (n1 > 0) cube_widen(p2, p1);
+    src.template rows<kI1, n1>(p2);
+    if constexpr (n2 > 0) cube_widen(p3, p2);
+    if constexpr (n3 > n2) {
+      CubeArray<cube_class(kX < 0 ? 0 : kX), Num> x;
+      src.template rows<(kX < 0 ? 0 : kX), 0>(x);
+      if constexpr (n2 == 0)
+        cube_widen(p3, x);
+      else
+        cube_merge<n2, n3 - n2>(p3, x);
+    }
+    src.template rows<kI2, n3>(p3);
+  }
+
+  static constexpr int kFirst = total<1, 2, 3, 4>() + count<5>();  // rows of top
+  static constexpr int kSecond = total<6, 7, 8, 9>();
+  static constexpr int kThird = total<10, 11, -1, 12>();
+  static constexpr int kLast = count<0>() + total<13, 14, -1, 15>();
+  static_assert(total<1, 2, 3, 4>() > 0 && kLast > 0, "shapes have rows in the first and the last chain");
+
+  // top[16]: the first and second chain and the rows of {0123}; the arrays of
+  // the third ({0, 2, 3}; unset without rows) and the last chain ({0, 1, 3}),
+  // which also takes the rows of {}: the chains are about as long then, and
+  // more of their products stay below 2^53 for integers
+  __device__ __forceinline__ void products(CubeArray<15, Num>& top, CubeArray<13, Num>& third,
+                                           CubeArray<11, Num>& last) const {
+    const CubeArray<0, Num> none = {};
+    {
+      CubeArray<7, Num> p3;
+      chain<1, 2, 3, 4, 0, 0>(p3, none);
+      cube_widen(top, p3);
+      src.template rows<5, total<1, 2, 3, 4>()>(top);
+    }
+    if constexpr (kSecond > 0) {
+      CubeArray<14, Num> p3;
+      chain<6, 7, 8, 9, 0, 0>(p3, none);
+      cube_merge<kFirst, kSecond>(top, p3);
+    }
+    if constexpr (kThird > 0) chain<10, 11, -1, 12, 0, 0>(third, none);
+    CubeArray<0, Num> p0;
+    src.template rows<0, 0>(p0);
+    chain<13, 14, -1, 15, 0, count<0>()>(last, p0);
+  }
+};
+
+// Rows of FP64 x: b + c with c a constant operand.  `row(slot)` returns b.
+template <int kShape, class Row>
+struct CubeRowsF64 {
+  const CubeArgs& a;
+  Row row;
+  template <int kI, int kDone>
+  __device__ __forceinline__ void rows(CubeArray<cube_class(kI), CubeF64>& p) const {
+    constexpr int W = CubeArray<cube_class(kI), CubeF64>::kW, H = W / 2;
     constexpr int kSlot = cube_slot(kCubeShapes[kShape], kI), kSum = cube_sum(kCubeShapes[kShape], kI);
+    constexpr int K = kCubeShapes[kShape].rows[cube_class(kI)];
 #pragma unroll
-    for (int r = 0; r < count<kI>(); r++) {
-      const Num b = row(kSlot + r);
+    for (int r = 0; r < K; r++) {
+      const double b = row(kSlot + r);
 #pragma unroll
       for (int s = 0; s < W; s++) {
-        Num x = b;
+        double x = b;
+        // the sums with the last column's sign plus; minus is their mirror image
+        if constexpr (W > 1)
+          x = s >= H ? __dadd_rn(b, a.c[kSum + r * H + s - H]) : __dsub_rn(b, a.c[kSum + r * H + H - 1 - s]);
+        if (kDone == 0 && r == 0)
+          p.v[s].hi = x;
+        else
+          p.v[s].hi = p.v[s].hi * x;
+      }
+    }
+  }
+};
+
+// Rows of split x: pairs with exact coarse parts.  `row(slot)` returns (b, its remainder).
+template <int kShape, class Row>
+struct CubeRowsSdd {
+  const CubeSddArgs& a;
+  Row row;
+  template <int kI, int kDone>
+  __device__ __forceinline__ void rows(CubeArray<cube_class(kI), CubeDd<0>>& p) const {
+    constexpr int W = CubeArray<cube_class(kI), CubeDd<0>>::kW, H = W / 2;
+    constexpr int kSlot = cube_slot(kCubeShapes[kShape], kI), kSum = cube_sum(kCubeShapes[kShape], kI);
+    constexpr int K = kCubeShapes[kShape].rows[cube_class(kI)];
+#pragma unroll
+    for (int r = 0; r < K; r++) {
+      const CubeDd<0> b = row(kSlot + r);
+#pragma unroll
+      for (int s = 0; s < W; s++) {
+        CubeDd<0> x = b;
         if constexpr (W > 1) {
-          // the sums with the last column's sign plus; minus is their mirror image
           const int q = kSum + r * H + (s >= H ? s - H : H - 1 - s);
           x.hi = s >= H ? __dadd_rn(b.hi, a.c[q]) : __dsub_rn(b.hi, a.c[q]);
-          if constexpr (kPair) x.lo = s >= H ? __dadd_rn(b.lo, a.cl[q]) : __dsub_rn(b.lo, a.cl[q]);
+          x.lo = s >= H ? __dadd_rn(b.lo, a.cl[q]) : __dsub_rn(b.lo, a.cl[q]);
         }
-        if (kFirst && r == 0)
+        if (kDone == 0 && r == 0)
           p.v[s] = x;
         else
-          p.v[s].mul(x);
+          p.v[s].template mul<1, 1>(x);
       }
     }
   }
+};
 
-  // {k} > {kl} (x extra) > {klm}: classes kI, kI + 1, (kX), kL of the kernel
-  // order; true when it has any rows
-  template <int kI0, int kI1, int kX, int kI2>
-  static constexpr bool any() {
-    return count<kI0>() + count<kI1>() + (kX >= 0 ? count<(kX >= 0 ? kX : 0)>() : 0) + count<kI2>() > 0;
+// Rows of an integer matrix, y = 2x in int32 (registers).  Runs of 4 rows of
+// a class (and a last run of 3) are multiplied in int32 and converted once per
+// value: the host checks |product| < 2^31.  The one or two rows left over are
+// converted once and added and multiplied in FP64: a run that short costs
+// more in conversions (two cycles each per warp and SM) than it saves.  Both
+// are exact.
+template <int kShape, class Num, class Row>
+struct CubeRowsInt {
+  const CubeIntArgs& a;
+  Row row;
+
+  template <int kRows, int kBefore>
+  __device__ __forceinline__ static void put(Num& p, double x) {
+    if constexpr (kBefore == 0)
+      p.hi = x;
+    else if constexpr (std::is_same_v<Num, CubeF64>)
+      p.hi = p.hi * x;
+    else
+      p.template mul_exact<kRows, kBefore>(x);
   }
-  template <int kI0, int kI1, int kX, int kI2, int kFrom, bool kUnset>
-  __device__ __forceinline__ void chain(CubeArray<cube_class(kI2), kPair>& p3,
-                                        const CubeArray<kFrom, kPair>& from) const {
-    constexpr int A = cube_class(kI0), B = cube_class(kI1), C = cube_class(kI2);
-    constexpr bool f1 = kUnset && count<kI0>() == 0, f2 = f1 && count<kI1>() == 0;
-    CubeArray<A, kPair> p1;
-    if constexpr (!kUnset) cube_widen(p1, from);
-    rows<kI0, kUnset>(p1);
-    CubeArray<B, kPair> p2;
-    if constexpr (!f1) cube_widen(p2, p1);
-    rows<kI1, f1>(p2);
-    if constexpr (!f2) cube_widen(p3, p2);
-    if constexpr (kX >= 0) {
-      constexpr int kXi = kX >= 0 ? kX : 0;
-      if constexpr (count<kXi>() > 0) {
-        CubeArray<cube_class(kXi), kPair> x;
-        rows<kXi, true>(x);
-        if constexpr (f2)
-          cube_widen(p3, x);
-        else
-          cube_merge(p3, x);
-        rows<kI2, false>(p3);
-        return;
+  template <int kI, int kR, int kDone>
+  __device__ __forceinline__ void from(CubeArray<cube_class(kI), Num>& p) const {
+    constexpr int W = CubeArray<cube_class(kI), Num>::kW, H = W / 2;
+    constexpr int K = kCubeShapes[kShape].rows[cube_class(kI)], kLeft = K - kR;
+    constexpr int kSlot = cube_slot(kCubeShapes[kShape], kI), kSum = cube_sum(kCubeShapes[kShape], kI);
+    if constexpr (kLeft >= 3) {
+      constexpr int G = kLeft >= 4 ? 4 : 3;
+#pragma unroll
+      for (int s = 0; s < W; s++) {
+        uint32_t y[4];
+#pragma unroll
+        for (int t = 0; t < G; t++) {
+          const int b = row(kSlot + kR + t), q = kSum + (kR + t) * H;
+          if constexpr (W > 1)
+            y[t] = (uint32_t)(s >= H ? b + a.ci[q + s - H] : b - a.ci[q + H - 1 - s]);
+          else
+            y[t] = (uint32_t)b;
+        }
+        const uint32_t v = G == 4 ? (y[0] * y[1]) * (y[2] * y[3]) : (y[0] * y[1]) * y[2];
+        put<kDone + G, kDone>(p.v[s], __int2double_rn((int)v));
       }
+      from<kI, kR + G, kDone + G>(p);
+    } else if constexpr (kLeft > 0) {
+      constexpr int kLeftSum = cube_left_sum(kCubeShapes[kShape], kI) + (kR - (K - cube_left(K))) * H;
+      const double b = __int2double_rn(row(kSlot + kR));
+#pragma unroll
+      for (int s = 0; s < W; s++) {
+        double x = b;
+        if constexpr (W > 1) x = s >= H ? __dadd_rn(b, a.cd[kLeftSum + s - H]) : __dsub_rn(b, a.cd[kLeftSum + H - 1 - s]);
+        put<kDone + 1, kDone>(p.v[s], x);
+      }
+      from<kI, kR + 1, kDone + 1>(p);
     }
-    rows<kI2, f2>(p3);
   }
-
-  // top[16] and the last chain's array over {0, 1, 3}
-  __device__ __forceinline__ void products(CubeArray<15, kPair>& top, CubeArray<11, kPair>& last) const {
-    static_assert(count<13>() + count<14>() + count<15>() > 0 && count<0>() + count<1>() + count<2>() + count<4>() > 0,
-                  "shapes have rows in the first and the last chain");
-    {
-      CubeArray<0, kPair> p0;
-      rows<0, true>(p0);
-      CubeArray<7, kPair> p3;
-      chain<1, 2, 3, 4, 0, count<0>() == 0>(p3, p0);
-      cube_widen(top, p3);
-      rows<5, false>(top);
-    }
-    const CubeArray<0, kPair> none = {};
-    if constexpr (any<6, 7, 8, 9>()) {
-      CubeArray<14, kPair> p3;
-      chain<6, 7, 8, 9, 0, true>(p3, none);
-      cube_merge(top, p3);
-    }
-    if constexpr (any<10, 11, -1, 12>()) {
-      CubeArray<13, kPair> p3;
-      chain<10, 11, -1, 12, 0, true>(p3, none);
-      cube_merge(top, p3);
-    }
-    chain<13, 14, -1, 15, 0, true>(last, none);
+  template <int kI, int kDone>
+  __device__ __forceinline__ void rows(CubeArray<cube_class(kI), Num>& p) const {
+    from<kI, 0, kDone>(p);
   }
 };
 
 // Adds the 16 signed terms last x top to (H, L) (Sum2, over column 2's sign
 // first) and their absolute values to m1.
-__device__ __forceinline__ void cube_sum_dd(const CubeArray<15, true>& top, const CubeArray<11, true>& last, bool odd,
+template <bool kLastExact, class Num>
+__device__ __forceinline__ void cube_sum_dd(const CubeArray<15, Num>& top, const CubeArray<11, Num>& last, bool odd,
                                             double& H, double& L, double& m1) {
-  double gs = 0.0, gc = 0.0;
+  dd t[8];
 #pragma unroll
   for (int s = 0; s < 8; s++) {
     const int lo = (s & 3) | ((s & 4) << 1);  // sign of column 2 minus
-    const CubeNum<true>&t0 = top.v[lo], &t1 = top.v[lo | 4];
+    const Num &t0 = top.v[lo], &t1 = top.v[lo | 4];
     dd d = two_sum(t0.hi, -t1.hi);
     d.lo = __dadd_rn(d.lo, __dsub_rn(t0.lo, t1.lo));
     m1 = __fma_rn(fabs(last.v[s].hi), __dadd_rn(fabs(t0.hi), fabs(t1.hi)), m1);
-    pair_mul(d, last.v[s].hi, last.v[s].lo);
+    if constexpr (kLastExact) {
+      const double h = __dmul_rn(d.hi, last.v[s].hi);
+      d.lo = __fma_rn(d.lo, last.v[s].hi, __fma_rn(d.hi, last.v[s].hi, -h));
+      d.hi = h;
+    } else {
+      pair_mul(d, last.v[s].hi, last.v[s].lo);
+    }
     if (__popc(s) & 1) d = {-d.hi, -d.lo};
-    if (s == 0)
-      gs = d.hi, gc = d.lo;
-    else
-      sum2_add(gs, gc, d.hi, d.lo);
+    t[s] = d;
   }
-  sum2_add(H, L, odd ? -gs : gs, odd ? -gc : gc);
+  // pairwise: every rounding error of the high parts goes to the low part
+#pragma unroll
+  for (int w = 4; w >= 1; w >>= 1) {
+#pragma unroll
+    for (int s = 0; s < w; s++) {
+      dd r = two_sum(t[s].hi, t[s + w].hi);
+      r.lo = __dadd_rn(r.lo, __dadd_rn(t[s].lo, t[s + w].lo));
+      t[s] = r;
+    }
+  }
+  sum2_add(H, L, odd ? -t[0].hi : t[0].hi, odd ? -t[0].lo : t[0].lo);
+}
+
+// The signed sum of the 16 terms top x third x last: over column 2's sign
+// first, then column 0's, then the other two.  Neighbouring terms mostly
+// cancel, so what is rounded stays small, and the differences of products are
+// fused (one rounding less per term; errors over integer matrices then match
+// those of the row layouts).
+// kAbs: their absolute values are added to m1.
+template <bool kThird, bool kAbs>
+__device__ __forceinline__ double cube_sum_f64(const CubeArray<15, CubeF64>& top, const CubeArray<13, CubeF64>& third,
+                                               const CubeArray<11, CubeF64>& last, double& m1) {
+  double d[8];
+#pragma unroll
+  for (int s = 0; s < 8; s++) {
+    const int t0 = (s & 3) | ((s & 4) << 1), t1 = t0 | 4;  // column 2 minus, plus
+    if constexpr (kThird) {
+      const int a0 = (s & 1) | (s & 4), a1 = a0 | 2;
+      const double p = __dmul_rn(top.v[t1].hi, third.v[a1].hi);
+      d[s] = __fma_rn(top.v[t0].hi, third.v[a0].hi, -p);
+      if constexpr (kAbs)
+        m1 = __fma_rn(fabs(last.v[s].hi), __fma_rn(fabs(top.v[t0].hi), fabs(third.v[a0].hi), fabs(p)), m1);
+    } else {
+      d[s] = __dsub_rn(top.v[t0].hi, top.v[t1].hi);
+      if constexpr (kAbs)
+        m1 = __fma_rn(fabs(last.v[s].hi), __dadd_rn(fabs(top.v[t0].hi), fabs(top.v[t1].hi)), m1);
+    }
+  }
+  double t[4];
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    const int s = 2 * q + (__popc(q) & 1), r = s ^ 1;  // plus term, minus term
+    t[q] = __fma_rn(last.v[s].hi, d[s], -__dmul_rn(last.v[r].hi, d[r]));
+  }
+  return __dadd_rn(__dadd_rn(t[0], t[1]), __dadd_rn(t[2], t[3]));
 }
 
 // Range of outer Gray indices of this thread, and the loop over it:
 // start(h) sets b for outer index h, flip(h) moves it from h - 1 to h,
 // cube(h) adds the 16 terms of h.
 template <class Start, class Flip, class Eval>
-__device__ __forceinline__ void cube_walk(const CubeArgs& a, Start start, Flip flip, Eval cube) {
+__device__ __forceinline__ void cube_walk(const CubeWalk& a, Start start, Flip flip, Eval cube) {
   const uint64_t TT = (uint64_t)gridDim.x * blockDim.x;
   const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const uint64_t q = a.nblocks / TT, r = a.nblocks % TT;
@@ -240,8 +404,19 @@ __device__ __forceinline__ void cube_walk(const CubeArgs& a, Start start, Flip f
   }
 }
 
-// FP64 walk.
-template <int kShape>
+// Sum of m1 over the grid to *sums, and the thread totals to *out.
+__device__ __forceinline__ void cube_finish(const CubeWalk& a, dd total, bool abs_sum, double m1, double factor, dd* red) {
+  if (abs_sum) {
+#pragma unroll
+    for (int d = 16; d >= 1; d >>= 1) m1 += __shfl_down_sync(0xffffffffu, m1, d);
+    if ((threadIdx.x & 31) == 0 && m1 > 0.0) atomicAdd(a.sums, m1);
+  }
+  const dd bt = block_reduce_dd(total, red);
+  grid_finish_dd(bt, a.partials, a.ticket, a.out, factor, red);
+}
+
+// FP64 walk; kAbs: sums[0] += sum |term| as well (16 of some 250 operations).
+template <int kShape, bool kAbs>
 __global__ void __launch_bounds__(kCubeThreads, 1) ryser_cube_kernel(const __grid_constant__ CubeArgs a) {
   constexpr int N = cube_rows(kCubeShapes[kShape]);
   static_assert(N % 2 == 0, "columns are read two rows at a time");
@@ -252,6 +427,7 @@ __global__ void __launch_bounds__(kCubeThreads, 1) ryser_cube_kernel(const __gri
   uint64_t* bar = reinterpret_cast<uint64_t*>(red + 32);
   const bool staged = stage_to_smem(sC, a.img, (uint32_t)(sizeof(double) * nc * N), bar, a.err, a.inject);
   Acc acc;
+  double m1 = 0.0;
   if (staged) {
     double b[N];
     auto add = [&](const double* c, double s) {
@@ -262,8 +438,9 @@ __global__ void __launch_bounds__(kCubeThreads, 1) ryser_cube_kernel(const __gri
         b[j + 1] = __fma_rn(s, v.y, b[j + 1]);
       }
     };
-    auto row = [&](int j) { return CubeNum<false>{b[j]}; };
-    const Cube<kShape, false, decltype(row)> cube{a, row};
+    auto row = [&](int j) { return b[j]; };
+    const CubeRowsF64<kShape, decltype(row)> src{a, row};
+    const Cube<kShape, CubeF64, decltype(src)> cube{src};
     cube_walk(
         a,
         [&](uint64_t h) {
@@ -279,23 +456,15 @@ __global__ void __launch_bounds__(kCubeThreads, 1) ryser_cube_kernel(const __gri
           add(sC + (size_t)k * N, ((h >> (k + 1)) & 1) ? -1.0 : 1.0);
         },
         [&](uint64_t h) {
-          CubeArray<15, false> top;
-          CubeArray<11, false> last;
-          cube.products(top, last);
-          double even = 0.0, odd = 0.0;
-#pragma unroll
-          for (int s = 0; s < 8; s++) {
-            const int lo = (s & 3) | ((s & 4) << 1);  // sign of column 2 minus
-            const double d = top.v[lo].hi - top.v[lo | 4].hi;
-            double& t = (__popc(s) & 1) ? odd : even;
-            t = s < 2 ? last.v[s].hi * d : __fma_rn(last.v[s].hi, d, t);
-          }
-          const double t = even - odd;
+          CubeArray<15, CubeF64> top;
+          CubeArray<13, CubeF64> third;
+          CubeArray<11, CubeF64> last;
+          cube.products(top, third, last);
+          const double t = cube_sum_f64<(decltype(cube)::kThird > 0), kAbs>(top, third, last, m1);
           acc.add((h & 1) ? -t : t);
         });
   }
-  const dd bt = block_reduce_dd(acc.value(), red);
-  grid_finish_dd(bt, a.partials, a.ticket, a.out, (a.n & 1) ? 2.0 : -2.0, red);
+  cube_finish(a, acc.value(), kAbs, m1, (a.n & 1) ? 2.0 : -2.0, red);
 }
 
 // Split-dd walk (ryser_dense_sdd.cuh): b's exact coarse parts in registers,
@@ -306,7 +475,7 @@ __global__ void __launch_bounds__(kCubeThreads, 1) ryser_cube_kernel(const __gri
 // and updated in one pass, it was 9% slower (more wavefronts), with 12 warps
 // of 168 registers 9% (spills).
 template <int kShape>
-__global__ void __launch_bounds__(kCubeThreads, 1) ryser_cube_sdd_kernel(const __grid_constant__ CubeArgs a) {
+__global__ void __launch_bounds__(kCubeThreads, 1) ryser_cube_sdd_kernel(const __grid_constant__ CubeSddArgs a) {
   constexpr int N = cube_rows(kCubeShapes[kShape]);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int nc = a.n - 4;
@@ -330,8 +499,9 @@ __global__ void __launch_bounds__(kCubeThreads, 1) ryser_cube_sdd_kernel(const _
         bl[(j + 1) * kCubeThreads] = __fma_rn(s, w.y, bl[(j + 1) * kCubeThreads]);
       }
     };
-    auto row = [&](int j) { return CubeNum<true>{b[j], bl[j * kCubeThreads]}; };
-    const Cube<kShape, true, decltype(row)> cube{a, row};
+    auto row = [&](int j) { return CubeDd<0>{b[j], bl[j * kCubeThreads]}; };
+    const CubeRowsSdd<kShape, decltype(row)> src{a, row};
+    const Cube<kShape, CubeDd<0>, decltype(src)> cube{src};
     cube_walk(
         a,
         [&](uint64_t h) {
@@ -347,18 +517,90 @@ __global__ void __launch_bounds__(kCubeThreads, 1) ryser_cube_sdd_kernel(const _
           add(k, ((h >> (k + 1)) & 1) ? -1.0 : 1.0);
         },
         [&](uint64_t h) {
-          CubeArray<15, true> top;
-          CubeArray<11, true> last;
-          cube.products(top, last);
-          cube_sum_dd(top, last, (h & 1) != 0, H, L, m1);
+          using C = decltype(cube);
+          CubeArray<15, CubeDd<0>> top;
+          CubeArray<13, CubeDd<0>> third;
+          CubeArray<11, CubeDd<0>> last;
+          cube.products(top, third, last);
+          if constexpr (C::kThird > 0) cube_merge<C::kFirst + C::kSecond, C::kThird>(top, third);
+          cube_sum_dd<false>(top, last, (h & 1) != 0, H, L, m1);
         });
   }
-  DenseSddArgs f = {};  // the shared tail's destinations
-  f.partials = a.partials;
-  f.ticket = a.ticket;
-  f.out = a.out;
-  f.sums = a.sums;
-  sdd_finish(H, L, m1, f, red, (a.n & 1) ? 2.0 : -2.0);
+  cube_finish(a, two_sum(H, L), true, m1, (a.n & 1) ? 2.0 : -2.0, red);
+}
+
+// Integer walks: y in int32 registers, columns as int32 in shared memory.
+// FP64 products (kDd false), or double-double products and sum with a
+// certified error (ryser_dense_intc.cuh), where products of up to
+// kCubeExactRows rows are kept in FP64 exactly (checked by the host).
+// FP64 products, order-40 shape of 140 values: 182 cycles per warp and cube,
+// 0.66 instructions issued per cycle and scheduler, FP64 pipe 46%, conversions
+// 30% (n = 40, density 1/2: 375 in the three-level row layout before).
+// Constants of both signs instead of mirrored ones: 200 (the compiler loads
+// them to registers early); left-over rows added to the bit pattern of 2^52 + b
+// instead of converted: 187; 12 warps of 168 registers: 185 and spills in the
+// larger shapes.  Certified: 364 cycles, of which the double-double arrays and
+// sum are two thirds of the FP64 operations (12 warps: 381).
+template <int kShape, bool kDd, bool kAbs>
+__global__ void __launch_bounds__(kCubeThreads, 1) ryser_cube_int_kernel(const __grid_constant__ CubeIntArgs a) {
+  using Num = std::conditional_t<kDd, CubeDd<kCubeExactRows>, CubeF64>;
+  constexpr int N = cube_rows(kCubeShapes[kShape]);
+  static_assert(N % 4 == 0, "columns are read four rows at a time");
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int nc = a.n - 4;
+  int* sC = reinterpret_cast<int*>(smem_raw);
+  dd* red = reinterpret_cast<dd*>(sC + (size_t)nc * N);
+  uint64_t* bar = reinterpret_cast<uint64_t*>(red + 32);
+  const bool staged = stage_to_smem(sC, a.img, (uint32_t)(sizeof(int) * nc * N), bar, a.err, a.inject);
+  Acc acc;
+  double H = 0.0, L = 0.0, m1 = 0.0;
+  if (staged) {
+    int b[N];
+    auto add = [&](int k, int s) {
+#pragma unroll
+      for (int j = 0; j < N; j += 4) {
+        const int4 v = lds4i(sC + (size_t)k * N + j);
+        b[j] += s * v.x;
+        b[j + 1] += s * v.y;
+        b[j + 2] += s * v.z;
+        b[j + 3] += s * v.w;
+      }
+    };
+    auto row = [&](int j) { return b[j]; };
+    const CubeRowsInt<kShape, Num, decltype(row)> src{a, row};
+    const Cube<kShape, Num, decltype(src)> cube{src};
+    cube_walk(
+        a,
+        [&](uint64_t h) {
+          const uint64_t g = h ^ (h >> 1);
+#pragma unroll
+          for (int j = 0; j < N; j++) b[j] = 0;
+          add(nc - 1, 1);
+#pragma unroll 1
+          for (int k = 0; k < nc - 1; k++) add(k, ((g >> k) & 1) ? 1 : -1);
+        },
+        [&](uint64_t h) {
+          const int k = __ffsll((long long)h) - 1;
+          add(k, ((h >> (k + 1)) & 1) ? -2 : 2);
+        },
+        [&](uint64_t h) {
+          using C = decltype(cube);
+          CubeArray<15, Num> top;
+          CubeArray<13, Num> third;
+          CubeArray<11, Num> last;
+          cube.products(top, third, last);
+          if constexpr (kDd) {
+            if constexpr (C::kThird > 0) cube_merge<C::kFirst + C::kSecond, C::kThird>(top, third);
+            cube_sum_dd<C::kLast <= kCubeExactRows>(top, last, (h & 1) != 0, H, L, m1);
+          } else {
+            const double t = cube_sum_f64<(C::kThird > 0), kAbs>(top, third, last, m1);
+            acc.add((h & 1) ? -t : t);
+          }
+        });
+  }
+  // prod y = 2^n prod x
+  const double factor = ((a.n & 1) ? 2.0 : -2.0) * ldexp(1.0, -a.n);
+  cube_finish(a, kDd ? two_sum(H, L) : acc.value(), kDd || kAbs, m1, factor, red);
 }
 
 }  // namespace perm

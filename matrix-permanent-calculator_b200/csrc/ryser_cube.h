@@ -9,10 +9,13 @@ namespace perm {
 
 struct dd;
 
-constexpr int kCubeThreads = 256;  // per CTA, one CTA per SM (ryser_cube.cuh)
+// Threads per CTA, one CTA per SM (ryser_cube.cuh).
+constexpr int kCubeThreads = 256;
+// Rows whose product the certified integer walk keeps in FP64 exactly.
+constexpr int kCubeExactRows = 8;
 
-struct CubeArgs {
-  const double* img;  // columns 4..n-1 in slot order (split-dd: coarse parts, then remainders)
+struct CubeWalk {
+  const void* img;  // columns 4..n-1 in slot order: FP64, split-dd coarse parts then remainders, or int32
   int n;
   int m;                     // log2 of the range alignment, in outer Gray indices
   uint64_t block0, nblocks;  // aligned blocks of 2^m outer indices of this launch
@@ -20,16 +23,27 @@ struct CubeArgs {
   dd* partials;
   unsigned* ticket;
   double* out;
-  double* sums;  // certified walks: sums[0] += sum |term| (zeroed by the host)
+  double* sums;  // sums[0] += sum |term| (zeroed by the host; walks that sum it)
   int* err;
   uint32_t inject;  // failure injection (tests): staging expects this many extra bytes
-  double c[kCubeMaxSums];   // sums of the fast columns over their signs, halved (plus last
-                            // column: row of class T has 2^|T| / 2), kernel order
-  double cl[kCubeMaxSums];  // split-dd: of their remainders
 };
 
-inline size_t cube_smem_bytes(bool pair, int n, int rows) {
-  return sizeof(double) * (size_t)rows * ((pair ? 2 : 1) * (size_t)(n - 4) + (pair ? kCubeThreads : 0)) + 32 * 16 + 16;
+// The sums of the fast columns over their signs, with the last column of a
+// row's set plus (2^|T| / 2 per row), in kernel order: of x, of split x, of
+// y = 2x.
+struct CubeArgs : CubeWalk {
+  double c[kCubeMaxSums];  // halved
+};
+struct CubeSddArgs : CubeWalk {
+  double c[kCubeMaxSums], cl[kCubeMaxSums];  // halved: of the coarse parts, of the remainders
+};
+struct CubeIntArgs : CubeWalk {
+  int ci[kCubeMaxSums];
+  double cd[kCubeMaxWide];  // of the rows left over from the int32 products
+};
+
+inline size_t cube_smem_bytes(int rows, size_t column_bytes, int n, bool remainders) {
+  return (size_t)rows * (column_bytes * (size_t)(n - 4) + (remainders ? sizeof(double) * kCubeThreads : 0)) + 32 * 16 + 16;
 }
 
 }  // namespace perm

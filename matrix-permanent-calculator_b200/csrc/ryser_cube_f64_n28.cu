@@ -2,7 +2,5 @@
 #include "cube_inst.cuh"
 
 namespace perm {
-const void* cube_f64_n28(int i) {
-  return cube_f64_pick<cube_first<28>()>(i, std::make_index_sequence<cube_count<28>()>());
-}
+const void* cube_f64_n28(int i) { return cube_pick<0, 28>(i); }
 }  // namespace perm

@@ -2,7 +2,5 @@
 #include "cube_inst.cuh"
 
 namespace perm {
-const void* cube_f64_n32(int i) {
-  return cube_f64_pick<cube_first<32>()>(i, std::make_index_sequence<cube_count<32>()>());
-}
+const void* cube_f64_n32(int i) { return cube_pick<0, 32>(i); }
 }  // namespace perm

@@ -2,7 +2,5 @@
 #include "cube_inst.cuh"
 
 namespace perm {
-const void* cube_f64_n36(int i) {
-  return cube_f64_pick<cube_first<36>()>(i, std::make_index_sequence<cube_count<36>()>());
-}
+const void* cube_f64_n36(int i) { return cube_pick<0, 36>(i); }
 }  // namespace perm

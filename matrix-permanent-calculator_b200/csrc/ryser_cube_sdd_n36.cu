@@ -2,7 +2,5 @@
 #include "cube_inst.cuh"
 
 namespace perm {
-const void* cube_sdd_n36(int i) {
-  return cube_sdd_pick<cube_first<36>()>(i, std::make_index_sequence<cube_count<36>()>());
-}
+const void* cube_sdd_n36(int i) { return cube_pick<2, 36>(i); }
 }  // namespace perm

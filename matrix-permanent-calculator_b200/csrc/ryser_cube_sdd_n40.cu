@@ -2,7 +2,5 @@
 #include "cube_inst.cuh"
 
 namespace perm {
-const void* cube_sdd_n40(int i) {
-  return cube_sdd_pick<cube_first<40>()>(i, std::make_index_sequence<cube_count<40>()>());
-}
+const void* cube_sdd_n40(int i) { return cube_pick<2, 40>(i); }
 }  // namespace perm

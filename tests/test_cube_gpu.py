@@ -77,3 +77,37 @@ def test_cube_transposed_and_permuted_inputs_agree(engine, pb):
     got = [engine.exact_dense(M, variant=pb.PERM_KERNEL_DENSE_SDD) for M in (A, A.T.copy(), A[::-1, ::-1].copy())]
     for g in got[1:]:
         assert abs(g.value - got[0].value) <= (g.rel_error_estimate + got[0].rel_error_estimate + 2 * U) * got[0].value
+
+
+def _integers(n, d, top, seed, signed=False):
+    rng = np.random.default_rng([n, seed, top])
+    mask = (rng.random((n, n)) < d) | (np.eye(n)[rng.permutation(n)] > 0)
+    vals = rng.integers(1, top + 1, (n, n))
+    return (mask * (vals * rng.choice([-1, 1], (n, n)) if signed else mask * vals)).astype(np.float64)
+
+
+@pytest.mark.parametrize("n,d,top,signed", [(25, 0.12, 4, False), (25, 0.5, 1, False), (26, 0.4, 3, True),
+                                            (27, 0.5, 4, False), (28, 0.7, 4, False), (29, 0.3, 1, False),
+                                            # row sums at the int32 runs' limit (four of about 215) and beyond it
+                                            (25, 0.5, 33, False), (25, 0.5, 60, False)])
+def test_cube_integer_walks_vs_exact(engine, orc, pb, n, d, top, signed):
+    """int32 walks, FP64 and double-double products: against the exact
+    multi-modular oracle within their bounds; shards add up."""
+    A = _integers(n, d, top, 6, signed)
+    want = float(orc.perm_exact_int(A)[0])
+    _check(engine, A, want, U * abs(want), (pb.PERM_KERNEL_DENSE_INT, pb.PERM_KERNEL_DENSE_INT_DD))
+    r = engine.exact_dense(A, variant=pb.PERM_KERNEL_DENSE_INT_DD)
+    assert abs(r.value - want) <= 2 * U * abs(want) + r.rel_error_estimate * abs(want)
+
+
+@pytest.mark.parametrize("n,k", [(36, 19), (33, 20)])
+def test_cube_integer_walks_vs_product(engine, orc, pb, n, k):
+    rng = np.random.default_rng(n)
+    B, C = _integers(k, 0.8, 4, 7), _integers(n - k, 0.8, 4, 8)
+    A = np.zeros((n, n))
+    A[:k, :k], A[k:, k:] = B, C
+    A = A[rng.permutation(n)][:, rng.permutation(n)]
+    want = float(orc.perm_exact_int(B)[0] * orc.perm_exact_int(C)[0])
+    for variant in (pb.PERM_KERNEL_DENSE_INT, pb.PERM_KERNEL_DENSE_INT_DD):
+        r = engine.exact_dense(A, variant=variant)
+        assert abs(r.value - want) <= (r.rel_error_estimate + 2 * U) * want, variant
