@@ -24,7 +24,8 @@ struct UpSets {
   int count = 0;
   uint64_t lo[kPad], hi[kPad];                 // byte masks over classes 0..7 and 8..15
   uint8_t caps[kCubeShapeCount][kPad];
-  uint8_t perm[24][16];
+  uint8_t perm[24][16];   // class under each order of the columns
+  uint8_t column[24][4];  // new place of each column
   UpSets() {
     memset(lo, 0, sizeof lo);
     memset(hi, 0, sizeof hi);
@@ -50,6 +51,7 @@ struct UpSets {
           if ((t >> k) & 1) r |= 1 << p[k];
         perm[i][t] = (uint8_t)r;
       }
+      for (int k = 0; k < 4; k++) column[i][k] = (uint8_t)p[k];
       i++;
     } while (std::next_permutation(p, p + 4));
   }
@@ -153,12 +155,19 @@ bool cube_layout(const std::vector<double>& a, int n, double max_cost, CubeLayou
   static const struct Costs {
     double v[kCubeShapeCount];
     int values[kCubeShapeCount], at_least[kCubeShapeCount][5] = {};
+    uint8_t both[kCubeShapeCount][16] = {};    // slots of the classes with columns k and l
+    uint8_t fullest[kCubeShapeCount][4] = {};  // of those with column k, ascending
     Costs() {
       for (int s = 0; s < kCubeShapeCount; s++) {
         v[s] = cube_shape_cost(s);
         values[s] = cube_values(kCubeShapes[s]);
         for (int t = 0; t < 16; t++)
           for (int b = cube_bits(t); b >= 0; b--) at_least[s][b] += kCubeShapes[s].rows[t];
+        for (int kl = 0; kl < 16; kl++)
+          for (int t = 0; t < 16; t++)
+            if (((t >> (kl / 4)) & 1) && ((t >> (kl % 4)) & 1)) both[s][kl] += kCubeShapes[s].rows[t];
+        for (int k = 0; k < 4; k++) fullest[s][k] = both[s][5 * k];
+        std::sort(fullest[s], fullest[s] + 4);
       }
     }
   } costs;
@@ -199,21 +208,42 @@ bool cube_layout(const std::vector<double>& a, int n, double max_cost, CubeLayou
       count[t]++;
       for (int b = cube_bits(t); b >= 0; b--) at_least[b]++;
     }
+    // rows nonzero in column k, and in columns k and l
+    uint8_t need[16], fullest[4];
+    for (int k = 0; k < 4; k++)
+      for (int l = 0; l < 4; l++) need[4 * k + l] = (uint8_t)__builtin_popcountll(sup[q.c[k]] & sup[q.c[l]]);
+    for (int k = 0; k < 4; k++) fullest[k] = need[5 * k];
+    std::sort(fullest, fullest + 4);
     // shapes that could beat the best and have room in every layer of the
-    // lattice; only those are tried under the 24 orders of the columns
+    // lattice and for every column; only those are tried under the 24 orders
     int tryable[kCubeShapeCount], tries = 0;
     for (int s = first; s < last; s++) {
       if (costs.v[s] > best || (layout->shape >= 0 && costs.v[s] >= best) || costs.values[s] < q.values) continue;
       bool room = true;
       for (int t = 1; t <= 4; t++) room = room && at_least[t] <= costs.at_least[s][t];
+      for (int k = 0; k < 4; k++) room = room && fullest[k] <= costs.fullest[s][k];
       if (room) tryable[tries++] = s;
     }
     for (int p = 0; p < 24 && tries; p++) {
-      uint8_t have[16], sum[UpSets::kPad] = {};
-      for (int t = 0; t < 16; t++) have[U.perm[p][t]] = count[t];
-      U.sums(have, sum);
+      uint8_t have[16], sum[UpSets::kPad];
+      bool summed = false;
       for (int i = 0; i < tries; i++) {
         const int s = tryable[i];
+        // the columns' and pairs' own counts first: most orders fail here
+        bool fits = true;
+        for (int k = 0; k < 4 && fits; k++)
+          for (int l = 0; l <= k; l++)
+            if (need[4 * k + l] > costs.both[s][4 * U.column[p][k] + U.column[p][l]]) {
+              fits = false;
+              break;
+            }
+        if (!fits) continue;
+        if (!summed) {
+          for (int t = 0; t < 16; t++) have[U.perm[p][t]] = count[t];
+          memset(sum, 0, sizeof sum);
+          U.sums(have, sum);
+          summed = true;
+        }
         uint8_t over = 0;
         for (int u = 0; u < UpSets::kPad; u++) over |= (uint8_t)(sum[u] > U.caps[s][u]);
         if (over) continue;

@@ -25,6 +25,8 @@
 #include <functional>
 #include <mutex>
 #include <string>
+#include <system_error>
+#include <thread>
 #include <vector>
 
 #include "../../include/perman_b200.h"
@@ -480,6 +482,16 @@ struct perm_matrix;
 // whole cubes of 16 terms from here on, and below it the search for four
 // columns (some 30 us on the host) costs what the walk gains.
 constexpr int kCubeMinN = 25;
+// In a batch's graph the column-cube walks run in kBatchBranches parallel
+// branches, largest first, each with a CTA per 64 cubes of its threads, so
+// that small ones share the device: smallest order, and at most so many walks
+// (the largest orders), since a graph node takes some 10 us to instantiate.
+// 1024 matrices of orders 12..28: 24.9 ms from order 25 on, 23.4 from 24, 22.7
+// from 23, 22.3 from 22, 21.9 from 21 (and 3 ms more of set-up); 8 branches
+// 22.4, 32 branches 22.1.
+constexpr int kBatchCubeMinN = 22;
+constexpr int kBatchBranches = 16;
+constexpr size_t kBatchMaxCubes = 4096;
 
 struct perm_ctx {
   int device = 0;
@@ -1458,6 +1470,63 @@ static bool build_cube_int_operand(const CubeLayout& l, DenseOperand* op) {
   return true;
 }
 
+// The FP64 walk's operand in column cubes; false where a row layout needs
+// fewer operations: their walks reach 0.93 (one level) and 0.87 of the FP64
+// pipe against 0.82.  One level is 32 n operations per 16 terms.  The smallest
+// row layout (levels of 8 and 20 rows) needs 394 + 4n, so cheaper cubes skip
+// the search for one.
+static bool cube_operand_f64(const std::vector<double>& a, int n, DenseOperand* op) {
+  CubeLayout l;
+  if (!cube_layout(a, n, 32.0 * n * 0.82 / 0.93, &l)) return false;
+  if (l.cost > (394.0 + 4.0 * n) * 0.82 / 0.87) {
+    int inner = 0, inner1 = 0;
+    long cost8 = 0;  // operations per 8 terms
+    std::vector<double> perm;
+    fp64_choose(a, n, &inner, &inner1, &perm, &cost8);
+    if (l.cost / 0.82 > 2.0 * (double)cost8 / (inner ? 0.87 : 0.93)) return false;
+  }
+  op->n = n;
+  op->variant = PERM_KERNEL_DENSE;
+  op->group = 0;
+  op->inner = op->inner1 = 0;
+  build_fp64_image(l.mat, n, op);
+  build_cube_operand(l, 1, op);
+  return true;
+}
+
+// The int32 walks' operand (op->variant: plain or certified) in column cubes,
+// for product groups of G (int_group_size); false where a row layout is
+// cheaper or the products need not fit.
+static bool cube_operand_int(const std::vector<double>& a, int n, int G, DenseOperand* op) {
+  CubeLayout cube;
+  if (!cube_layout(a, n, 1e9, &cube)) return false;
+  op->n = n;
+  const bool certified = op->variant == PERM_KERNEL_DENSE_INT_DD;
+  // Against the row layouts' instructions per 8 terms, in cycles per SM, warp
+  // and 16 terms: those issue 0.8 of 4 per cycle (0.77 each; the certified
+  // walk's, 0.95), the cube takes 0.47 per unit of its cost (certified: 100 +
+  // 0.68), measured over the shapes.  The several-level layouts need 0.6 of
+  // the one-level instructions at density 1/2, and the cube less still where
+  // they need less; only above that are they searched for (0.2 ms on the host
+  // at n = 30).
+  const double mine = certified ? 100.0 + 0.68 * cube.cost : 0.47 * cube.cost;
+  const double each = certified ? 0.95 : 0.77;
+  int pair = 0, cost1 = 0, g = 0, x = 0, y = 0;
+  if (certified) intc_layout(a, n, &pair, &cost1);
+  long cost = certified ? 8L * (n + cost1) : 8L * (2 * n + (n + G - 1) / G);
+  if (mine >= each * 0.6 * (double)cost) {
+    std::vector<double> p;
+    if (certified) {
+      intc_two_level_layout(a, n, cost, &g, &pair, &x, &p, &cost);
+      intc_three_level_layout(a, n, cost, &g, &pair, &x, &y, &p, &cost);
+    } else {
+      choose_int_layout(a, n, G, &p, &cost);
+    }
+    if (mine >= each * (double)cost) return false;
+  }
+  return build_cube_int_operand(cube, op);
+}
+
 static int build_sdd_operand(perm_ctx* ctx, const std::vector<double>& a, int n, DenseOperand* op) {
   if (n < 4 || n > 40) return fail(ctx, PERM_EUNSUPPORTED, "split-dd kernel covers orders 4..40 (got %d)", n);
   // The column-cube walk (6 operations per row value, 2 per row and about 280
@@ -1520,34 +1589,7 @@ static int build_operand(perm_ctx* ctx, const void* mat, int n, int dtype, int v
     op->ngo = 0;
     op->ng1 = op->ng2 = 0;
     std::vector<double> two;
-    CubeLayout cube;
-    const bool certified = op->variant == PERM_KERNEL_DENSE_INT_DD;
-    if (n >= kCubeMinN && op->variant != PERM_KERNEL_DENSE_TC && cube_layout(a, n, 1e9, &cube)) {
-      // Against the row layouts' instructions per 8 terms, in cycles per SM,
-      // warp and 16 terms: those issue 0.8 of 4 per cycle (0.77 each; the
-      // certified walk's, 0.95), the cube takes 0.47 per unit of its cost
-      // (certified: 100 + 0.68), measured over the shapes.  The several-level
-      // layouts need 0.6 of the one-level instructions at density 1/2, and
-      // the cube less still where they need less; only above that are they
-      // searched for (0.2 ms on the host at n = 30).
-      const double mine = certified ? 100.0 + 0.68 * cube.cost : 0.47 * cube.cost;
-      const double each = certified ? 0.95 : 0.77;
-      int pair = 0, cost1 = 0, g = 0, x = 0, y = 0;
-      if (certified) intc_layout(a, n, &pair, &cost1);
-      long cost = certified ? 8L * (n + cost1) : 8L * (2 * n + (n + G - 1) / G);
-      bool take = mine < each * 0.6 * (double)cost;
-      if (!take) {
-        std::vector<double> p;
-        if (certified) {
-          intc_two_level_layout(a, n, cost, &g, &pair, &x, &p, &cost);
-          intc_three_level_layout(a, n, cost, &g, &pair, &x, &y, &p, &cost);
-        } else {
-          choose_int_layout(a, n, G, &p, &cost);
-        }
-        take = mine < each * (double)cost;
-      }
-      if (take && build_cube_int_operand(cube, op)) return PERM_OK;
-    }
+    if (n >= kCubeMinN && op->variant != PERM_KERNEL_DENSE_TC && cube_operand_int(a, n, G, op)) return PERM_OK;
     if (op->variant == PERM_KERNEL_DENSE_INT_DD) {
       int cost1 = 0;
       op->group = intc_layout(a, n, &op->pair, &cost1);
@@ -1595,24 +1637,9 @@ static int build_operand(perm_ctx* ctx, const void* mat, int n, int dtype, int v
     op->inner = 0;
     op->inner1 = 0;
     if (op->variant == PERM_KERNEL_DENSE) {
-      // The column-cube walk unless a row layout needs fewer operations: their
-      // walks reach 0.93 (one level) and 0.87 of the FP64 pipe against 0.82.
-      // The smallest row layout (levels of 8 and 20 rows) needs 394 + 4n
-      // operations per 16 terms, so cheaper cubes skip the search for one.
-      CubeLayout l;
-      const bool cube = n >= kCubeMinN && cube_layout(a, n, 32.0 * n * 0.82 / 0.93, &l);
+      if (n >= kCubeMinN && cube_operand_f64(a, n, op)) return PERM_OK;
       std::vector<double> perm;
-      if (!cube || l.cost > (394.0 + 4.0 * n) * 0.82 / 0.87) {
-        long cost8 = 0;  // operations per 8 terms
-        fp64_choose(a, n, &op->inner, &op->inner1, &perm, &cost8);
-        if (cube && l.cost / 0.82 > 2.0 * (double)cost8 / (op->inner ? 0.87 : 0.93)) l.shape = -1;
-      }
-      if (l.shape >= 0) {
-        op->inner = op->inner1 = 0;
-        build_fp64_image(l.mat, n, op);
-        build_cube_operand(l, 1, op);
-        return PERM_OK;
-      }
+      fp64_choose(a, n, &op->inner, &op->inner1, &perm);
       if (op->inner) a.swap(perm);  // walk the permuted matrix (same permanent)
     }
     build_fp64_image(a, n, op);
@@ -1767,6 +1794,53 @@ extern "C" int perm_shard_range(int n, int shard, int nshards, uint64_t* first, 
   return PERM_OK;
 }
 
+// Range alignment (log2, in cubes, at most m_max) of a column-cube walk: a
+// thread owns ceil(blocks / threads) blocks of 2^m cubes at most, and leaving a
+// block costs about half a cube more, since the lanes then flip different
+// columns.
+static int cube_align(uint64_t cubes, uint64_t threads, int m_max) {
+  double best = -1.0;
+  int best_m = 0;
+  for (int m = 0; m <= 10 && m <= m_max; m++) {
+    const double each = std::ceil((double)(cubes >> m) / (double)threads);
+    const double cost = each * (std::ldexp(1.0, m) + 0.5);
+    if (best < 0.0 || cost < best) best = cost, best_m = m;
+  }
+  return best_m;
+}
+
+// Launch arguments of a column-cube walk over blocks [block0, block0 +
+// nblocks) of 2^m cubes, without its destinations; the walk's own form begins
+// with CubeWalk.
+union CubeLaunch {
+  CubeWalk walk;
+  CubeArgs f64;
+  CubeSddArgs sdd;
+  CubeIntArgs integer;
+  CubeLaunch() {}
+};
+static void cube_args(const DenseOperand& op, const void* d_image, int m, uint64_t block0, uint64_t nblocks,
+                      CubeLaunch* u) {
+  const int kind = cube_kind(op);
+  CubeWalk& w = u->walk;
+  w.img = d_image;
+  w.n = op.n;
+  w.m = m;
+  w.block0 = block0;
+  w.nblocks = nblocks;
+  w.seg = kind >= kCubeInt ? ~0ull : kCubeSegment;
+  w.inject = 0;
+  if (kind >= kCubeInt) {
+    for (int i = 0; i < kCubeMaxSums; i++) u->integer.ci[i] = (int)op.sums[i];
+    memcpy(u->integer.cd, op.sums.data() + kCubeMaxSums, sizeof u->integer.cd);
+  } else if (kind == kCubeSdd) {
+    memcpy(u->sdd.c, op.sums.data(), sizeof u->sdd.c);
+    memcpy(u->sdd.cl, op.sums.data() + kCubeMaxSums, sizeof u->sdd.cl);
+  } else {
+    memcpy(u->f64.c, op.sums.data(), sizeof u->f64.c);
+  }
+}
+
 static int dense_plan(perm_ctx* ctx, const DenseOperand& op, int shard, int nshards, DensePlan* p) {
   const int n = op.n;
   const void* fn = operand_kernel(op);
@@ -1827,19 +1901,7 @@ static int dense_plan(perm_ctx* ctx, const DenseOperand& op, int shard, int nsha
   }
   int grid = std::min(kMaxBlocks, ctx->num_sms * occ_slot);
   if (op.shape >= 0) {
-    // ranges of whole cubes.  A thread owns ceil(blocks / threads) blocks of
-    // 2^m cubes at most; leaving a block costs about half a cube more, since
-    // the lanes then flip different columns.
-    const uint64_t cubes = (last - first) >> 4, threads = (uint64_t)grid * operand_threads(op);
-    double best = -1.0;
-    for (int m = 0; m <= 10 && m <= (nshards == 1 ? n - 5 : ms - 4); m++) {
-      const double each = std::ceil((double)(cubes >> m) / (double)threads);
-      const double cost = each * (std::ldexp(1.0, m) + 0.5);
-      if (best < 0.0 || cost < best) {
-        best = cost;
-        p->m = 4 + m;
-      }
-    }
+    p->m = 4 + cube_align((last - first) >> 4, (uint64_t)grid * operand_threads(op), nshards == 1 ? n - 5 : ms - 4);
     p->block0 = first >> p->m;
     p->nblocks = (last - first) >> p->m;
     p->grid = (int)std::min<uint64_t>((uint64_t)grid, std::max<uint64_t>(1, (p->nblocks + operand_threads(op) - 1) / operand_threads(op)));
@@ -1867,31 +1929,17 @@ static int dense_launch(perm_ctx* ctx, const DenseOperand& op, const void* d_ima
   CU(ctx, cudaEventRecord(ctx->ev0, ctx->stream));
   if (op.shape >= 0) {
     const int kind = cube_kind(op);
-    union {
-      CubeArgs f64;
-      CubeSddArgs sdd;
-      CubeIntArgs integer;
-    } u;
-    CubeWalk& args = u.f64;  // every form begins with it
-    args.img = d_image;
-    args.n = n;
-    args.m = p.m - 4;
-    args.block0 = p.block0;
-    args.nblocks = p.nblocks;
-    args.seg = kind >= kCubeInt ? ~0ull : kCubeSegment;
+    CubeLaunch u;
+    cube_args(op, d_image, p.m - 4, p.block0, p.nblocks, &u);
+    CubeWalk& args = u.walk;
     args.partials = ctx->partials;
     args.ticket = ctx->ticket;
     args.out = ctx->d_out;
     args.sums = ctx->d_est;
     args.err = ctx->d_err;
-    args.inject = ctx->inject_timeouts > 0 && kind == kCubeF64 ? 16u : 0u;
-    if (args.inject) ctx->inject_timeouts--;
-    if (kind >= kCubeInt) {
-      for (int i = 0; i < kCubeMaxSums; i++) u.integer.ci[i] = (int)op.sums[i];
-      memcpy(u.integer.cd, op.sums.data() + kCubeMaxSums, sizeof u.integer.cd);
-    } else {
-      memcpy(u.f64.c, op.sums.data(), sizeof u.f64.c);
-      if (kind == kCubeSdd) memcpy(u.sdd.cl, op.sums.data() + kCubeMaxSums, sizeof u.sdd.cl);
+    if (ctx->inject_timeouts > 0 && kind == kCubeF64) {
+      args.inject = 16u;
+      ctx->inject_timeouts--;
     }
     void* kargs[] = {&u};
     if (kind == kCubeSdd || kind == kCubeIntc)
@@ -3024,6 +3072,14 @@ extern "C" int perm_approx_scaling_sparse_range(perm_ctx* ctx, int n, const int*
 // ---------------------------------------------------------------------------
 // batched exact permanents (one persistent launch, captured in a CUDA graph)
 // ---------------------------------------------------------------------------
+// One matrix of a batch that walks in column cubes, by a launch of its own in
+// the batch's graph.
+struct BatchCube {
+  DenseOperand op;
+  int index = 0;        // position in the caller's batch
+  uint64_t offset = 0;  // of its image in d_cubes, bytes
+};
+
 struct perm_batch {
   int count = 0;
   uint64_t total_tiles = 0;
@@ -3037,7 +3093,12 @@ struct perm_batch {
   unsigned* d_mat_done = nullptr;
   unsigned long long* d_next = nullptr;
   double* d_results = nullptr;
-  double* h_results = nullptr;  // pinned: (hi, lo, sum |term|) per matrix
+  double* h_results = nullptr;  // pinned: (hi, lo, sum |term|) per matrix, then the error flag
+  unsigned char* d_cubes = nullptr;  // column images of the column-cube walks
+  dd* d_cube_partials = nullptr;     // per branch of the graph: partials, tickets
+  unsigned* d_cube_tickets = nullptr;
+  std::vector<double> roundings;  // per matrix: roundings per term
+  std::vector<double> abs_scale;  // per matrix: factor of its sum |term|
   std::vector<int> groups;       // per matrix: 0 = FP64 X, else the int32-X group size
   std::vector<int> orders;       // host copies for double-double reruns
   std::vector<uint64_t> offsets;
@@ -3057,16 +3118,77 @@ static void batch_free(perm_batch* b) {
   cudaFree(b->d_mat_done);
   cudaFree(b->d_next);
   cudaFree(b->d_results);
+  cudaFree(b->d_cubes);
+  cudaFree(b->d_cube_partials);
+  cudaFree(b->d_cube_tickets);
   if (b->h_results) cudaFreeHost(b->h_results);
   delete b;
 }
 
+// The matrices of a batch that walk in column cubes, with their operands.  The
+// searches (some 30 us each) are shared out over up to 8 host threads.
+static void batch_cubes(int count, const int* orders, const double* values, std::vector<BatchCube>* out) {
+  std::vector<BatchCube> found;
+  std::vector<uint64_t> offset;
+  uint64_t off = 0;
+  for (int i = 0; i < count; i++) {
+    if (orders[i] < 1 || orders[i] > kBatchMaxOrder) return;  // refused by the caller
+    if (orders[i] >= kBatchCubeMinN) {
+      found.emplace_back();
+      found.back().index = i;
+      offset.push_back(off);
+    }
+    off += (uint64_t)orders[i] * orders[i];
+  }
+  if (found.size() > kBatchMaxCubes) {
+    std::vector<size_t> by_order(found.size());
+    for (size_t k = 0; k < by_order.size(); k++) by_order[k] = k;
+    std::stable_sort(by_order.begin(), by_order.end(),
+                     [&](size_t x, size_t y) { return orders[found[x].index] > orders[found[y].index]; });
+    std::sort(by_order.begin(), by_order.begin() + kBatchMaxCubes);
+    size_t kept = 0;
+    for (; kept < kBatchMaxCubes; kept++) {
+      offset[kept] = offset[by_order[kept]];
+      found[kept].index = found[by_order[kept]].index;
+    }
+    found.resize(kept);
+  }
+  std::atomic<size_t> next{0};
+  auto work = [&]() {
+    for (size_t k; (k = next.fetch_add(1)) < found.size();) {
+      const int n = orders[found[k].index];
+      const std::vector<double> a(values + offset[k], values + offset[k] + (size_t)n * n);
+      const int G = int_group_size(a, n);
+      DenseOperand& op = found[k].op;
+      op.variant = G ? PERM_KERNEL_DENSE_INT : PERM_KERNEL_DENSE;
+      if (!(G ? cube_operand_int(a, n, G, &op) : cube_operand_f64(a, n, &op))) op.shape = -1;
+    }
+  };
+  std::vector<std::thread> threads;
+  const size_t want = std::min<size_t>({found.size() / 8, std::thread::hardware_concurrency(), 8});
+  try {
+    while (threads.size() + 1 < want) threads.emplace_back(work);
+  } catch (const std::system_error&) {  // no more threads: the ones there do the work
+  }
+  work();
+  for (std::thread& t : threads) t.join();
+  for (BatchCube& c : found)
+    if (c.op.shape >= 0) out->push_back(std::move(c));
+}
+
 static int batch_create_locked(perm_ctx* ctx, int count, const int* orders, const double* values,
-                               const int* m_override, perm_batch** out, int variant_override = -1) {
+                               const int* m_override, perm_batch** out, int variant_override = -1,
+                               bool cubes = true) {
   if (count < 1 || !orders || !values || !out) return fail(ctx, PERM_EINVAL, "empty batch or null pointer");
   std::vector<BatchMatrix> mats(count);
   std::vector<uint64_t> src_off(count);
   std::vector<std::vector<double>> sparse_images(count);  // permuted matrices of the sparse layout
+  // Larger matrices walk in column cubes where that is cheaper.
+  std::vector<BatchCube> cube;
+  std::vector<int> cube_of(count, -1);
+  if (cubes) batch_cubes(count, orders, values, &cube);
+  for (size_t k = 0; k < cube.size(); k++) cube_of[cube[k].index] = (int)k;
+  uint64_t cube_bytes = 0;
   uint64_t off = 0, img = 0;
   for (int i = 0; i < count; i++) {
     const int n = orders[i];
@@ -3091,6 +3213,14 @@ static int batch_create_locked(perm_ctx* ctx, int count, const int* orders, cons
       std::vector<double> a(values + src_off[i], values + src_off[i] + (size_t)n * n);
       const int G = int_group_size(a, n);
       if (G >= 5) M.g = G;
+      if (cube_of[i] >= 0) {
+        BatchCube& c = cube[cube_of[i]];
+        c.offset = cube_bytes;
+        cube_bytes += (c.op.image.size() + 255) & ~(uint64_t)255;
+        M.g = G;
+        img -= (uint64_t)n * np;
+        continue;
+      }
       // two-level (sparse) layout (orders 12..32) when three columns have
       // their nonzeros in few rows: FP64 X with 8, 16, 20 or 24 inner rows,
       // int32 X (groups of 6) with 6, 12, 18 or 24; taken while the inner
@@ -3118,18 +3248,22 @@ static int batch_create_locked(perm_ctx* ctx, int count, const int* orders, cons
     }
   }
   // queue order: most Gray work first (longest-processing-time scheduling)
-  std::vector<int> order(count);
-  for (int i = 0; i < count; i++) order[i] = i;
+  std::vector<int> order;
+  for (int i = 0; i < count; i++)
+    if (cube_of[i] < 0) order.push_back(i);
   std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return mats[x].n > mats[y].n; });
-  std::vector<BatchMatrix> q(count);
+  std::stable_sort(cube.begin(), cube.end(), [](const BatchCube& x, const BatchCube& y) { return x.op.n > y.op.n; });
+  const int queued = (int)order.size();
+  std::vector<BatchMatrix> q(queued);
   uint64_t tiles = 0;
-  for (int r = 0; r < count; r++) {
+  for (int r = 0; r < queued; r++) {
     q[r] = mats[order[r]];
     q[r].first_tile = tiles;
     tiles += q[r].ntiles;
   }
   std::vector<double> image(img);
   for (int i = 0; i < count; i++) {
+    if (cube_of[i] >= 0) continue;
     const int n = mats[i].n, np = (n + 1) & ~1;
     const double* a = mats[i].r ? sparse_images[i].data() : values + src_off[i];
     double* dst = image.data() + mats[i].offset;
@@ -3156,6 +3290,7 @@ static int batch_create_locked(perm_ctx* ctx, int count, const int* orders, cons
   b->total_tiles = tiles;
   int max_n = 0;
   for (int i = 0; i < count; i++) {
+    if (cube_of[i] >= 0) continue;
     max_n = std::max(max_n, mats[i].n);
     if (mats[i].r) b->sparse++;
   }
@@ -3165,7 +3300,17 @@ static int batch_create_locked(perm_ctx* ctx, int count, const int* orders, cons
   const BatchVariant& V = kBatchVariants[vi];
   b->orders.assign(orders, orders + count);
   b->groups.resize(count);
-  for (int i = 0; i < count; i++) b->groups[i] = mats[i].g;
+  b->roundings.resize(count);
+  b->abs_scale.assign(count, 1.0);
+  for (int i = 0; i < count; i++) {
+    b->groups[i] = mats[i].g;
+    b->roundings[i] = mats[i].g ? std::ceil((double)mats[i].n / mats[i].g) : 2.0 * mats[i].n;
+  }
+  for (const BatchCube& c : cube) {
+    // |factor| = 2, of prod y = 2^n prod x in the int32 walk
+    b->abs_scale[c.index] = c.op.variant == PERM_KERNEL_DENSE_INT ? std::ldexp(1.0, 1 - c.op.n) : 2.0;
+    if (c.op.variant == PERM_KERNEL_DENSE_INT) b->roundings[c.index] = cube_factors(kCubeShapes[c.op.shape]) + 1.0;
+  }
   b->offsets = src_off;
   b->values.assign(values, values + off);
   cudaError_t e;
@@ -3178,15 +3323,30 @@ static int batch_create_locked(perm_ctx* ctx, int count, const int* orders, cons
     }                                               \
   } while (0)
   BT(cudaMalloc(&b->d_operands, sizeof(double) * std::max<uint64_t>(img, 1)));
-  BT(cudaMalloc(&b->d_mats, sizeof(BatchMatrix) * count));
-  BT(cudaMalloc(&b->d_tile_partials, sizeof(dd) * tiles));
-  BT(cudaMalloc(&b->d_tile_abs, sizeof(double) * tiles));
+  BT(cudaMalloc(&b->d_mats, sizeof(BatchMatrix) * std::max(queued, 1)));
+  BT(cudaMalloc(&b->d_tile_partials, sizeof(dd) * std::max<uint64_t>(tiles, 1)));
+  BT(cudaMalloc(&b->d_tile_abs, sizeof(double) * std::max<uint64_t>(tiles, 1)));
   BT(cudaMalloc(&b->d_mat_done, sizeof(unsigned) * count));
   BT(cudaMalloc(&b->d_next, sizeof(unsigned long long)));
-  BT(cudaMalloc(&b->d_results, sizeof(double) * 3 * count));
-  BT(cudaMallocHost(&b->h_results, sizeof(double) * 3 * count));
+  const size_t result_bytes = sizeof(double) * (3 * (size_t)count + 1);
+  BT(cudaMalloc(&b->d_results, result_bytes));
+  BT(cudaMallocHost(&b->h_results, result_bytes));
+  if (!cube.empty()) {
+    std::vector<unsigned char> images(cube_bytes);
+    for (const BatchCube& c : cube) memcpy(images.data() + c.offset, c.op.image.data(), c.op.image.size());
+    BT(cudaMalloc(&b->d_cubes, cube_bytes));
+    BT(cudaMemcpy(b->d_cubes, images.data(), cube_bytes, cudaMemcpyHostToDevice));
+    BT(cudaMalloc(&b->d_cube_partials, sizeof(dd) * kMaxBlocks * kBatchBranches));
+    BT(cudaMalloc(&b->d_cube_tickets, sizeof(unsigned) * kBatchBranches));
+    BT(cudaMemset(b->d_cube_tickets, 0, sizeof(unsigned) * kBatchBranches));
+    for (const BatchCube& c : cube)
+      if (int rc2 = allow_smem(ctx, cube_kernel(c.op.shape, cube_kind(c.op) + 1), operand_smem(c.op))) {
+        batch_free(b);
+        return rc2;
+      }
+  }
   BT(cudaMemcpy(b->d_operands, image.data(), sizeof(double) * img, cudaMemcpyHostToDevice));
-  BT(cudaMemcpy(b->d_mats, q.data(), sizeof(BatchMatrix) * count, cudaMemcpyHostToDevice));
+  if (queued) BT(cudaMemcpy(b->d_mats, q.data(), sizeof(BatchMatrix) * queued, cudaMemcpyHostToDevice));
   BT(cudaMemset(b->d_mat_done, 0, sizeof(unsigned) * count));
   if (!ctx->batch_occ[vi]) {
     if (int rc2 = allow_smem(ctx, V.fn, batch_smem_bytes(V))) {
@@ -3201,11 +3361,13 @@ static int batch_create_locked(perm_ctx* ctx, int count, const int* orders, cons
   const uint64_t warps = (uint64_t)ctx->num_sms * ctx->batch_occ[vi] * wpb;
   const uint64_t want = std::min<uint64_t>(warps, tiles);
   b->grid = (int)std::max<uint64_t>(1, (want + wpb - 1) / wpb);
-  // capture: reset the queue head, run, read the results back
+  // capture: reset the queue head and the results, run, read the results back.
+  // The column-cube walks are dealt to parallel branches beside the persistent
+  // kernel's: the next walk's CTAs fill the SMs that one leaves.
   BatchArgs args;
   args.operands = b->d_operands;
   args.mats = b->d_mats;
-  args.count = count;
+  args.count = queued;
   args.total_tiles = tiles;
   args.next_tile = b->d_next;
   args.tile_partials = b->d_tile_partials;
@@ -3213,10 +3375,52 @@ static int batch_create_locked(perm_ctx* ctx, int count, const int* orders, cons
   args.mat_done = b->d_mat_done;
   args.results = b->d_results;
   void* kargs[] = {&args};
+  struct Branches {
+    cudaStream_t stream[kBatchBranches] = {};
+    cudaEvent_t fork = nullptr, join[kBatchBranches] = {};
+    ~Branches() {
+      for (auto st : stream)
+        if (st) cudaStreamDestroy(st);
+      for (auto ev : join)
+        if (ev) cudaEventDestroy(ev);
+      if (fork) cudaEventDestroy(fork);
+    }
+  } br;
+  const int branches = (int)std::min<size_t>(kBatchBranches, cube.size());
+  if (branches) BT(cudaEventCreateWithFlags(&br.fork, cudaEventDisableTiming));
+  for (int i = 0; i < branches; i++) {
+    BT(cudaStreamCreateWithFlags(&br.stream[i], cudaStreamNonBlocking));
+    BT(cudaEventCreateWithFlags(&br.join[i], cudaEventDisableTiming));
+  }
   BT(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
   cudaMemsetAsync(b->d_next, 0, sizeof(unsigned long long), ctx->stream);
-  cudaLaunchKernel(V.fn, dim3(b->grid), dim3(V.block), kargs, batch_smem_bytes(V), ctx->stream);
-  cudaMemcpyAsync(b->h_results, b->d_results, sizeof(double) * 3 * count, cudaMemcpyDeviceToHost, ctx->stream);
+  cudaMemsetAsync(b->d_results, 0, result_bytes, ctx->stream);
+  if (branches) cudaEventRecord(br.fork, ctx->stream);
+  for (int i = 0; i < branches; i++) cudaStreamWaitEvent(br.stream[i], br.fork, 0);
+  for (size_t i = 0; i < cube.size(); i++) {
+    const BatchCube& c = cube[i];
+    const int branch = (int)(i % branches);
+    const uint64_t cubes_n = 1ull << (c.op.n - 5);
+    const int grid = (int)std::min<uint64_t>((uint64_t)ctx->num_sms, std::max<uint64_t>(1, cubes_n / (64 * kCubeThreads)));
+    const int m = cube_align(cubes_n, (uint64_t)grid * kCubeThreads, c.op.n - 5);
+    CubeLaunch u;
+    cube_args(c.op, b->d_cubes + c.offset, m, 0, cubes_n >> m, &u);
+    u.walk.partials = b->d_cube_partials + (size_t)branch * kMaxBlocks;
+    u.walk.ticket = b->d_cube_tickets + branch;
+    u.walk.out = b->d_results + 3 * c.index;
+    u.walk.sums = b->d_results + 3 * c.index + 2;
+    u.walk.err = reinterpret_cast<int*>(b->d_results + 3 * (size_t)count);
+    void* cargs[] = {&u};
+    cudaLaunchKernel(cube_kernel(c.op.shape, cube_kind(c.op) + 1), dim3(grid), dim3(kCubeThreads), cargs,
+                     operand_smem(c.op), br.stream[branch]);
+  }
+  if (tiles)
+    cudaLaunchKernel(V.fn, dim3(b->grid), dim3(V.block), kargs, batch_smem_bytes(V), ctx->stream);
+  for (int i = 0; i < branches; i++) {
+    cudaEventRecord(br.join[i], br.stream[i]);
+    cudaStreamWaitEvent(ctx->stream, br.join[i], 0);
+  }
+  cudaMemcpyAsync(b->h_results, b->d_results, result_bytes, cudaMemcpyDeviceToHost, ctx->stream);
   BT(cudaStreamEndCapture(ctx->stream, &b->graph));
   BT(cudaGraphInstantiate(&b->exec, b->graph, 0));
 #undef BT
@@ -3240,6 +3444,9 @@ static int batch_run_locked(perm_ctx* ctx, perm_batch* b, double* results, doubl
   CU(ctx, cudaGetLastError());
   float ms = 0;
   CU(ctx, cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));
+  int errflag = 0;
+  memcpy(&errflag, b->h_results + 3 * (size_t)b->count, sizeof errflag);
+  if (errflag) return fail(ctx, PERM_ETIMEOUT, "shared-memory staging wait timed out on device %d", ctx->device);
   if (kernel_ms) *kernel_ms = ms;
   if (results)
     for (int i = 0; i < b->count; i++) {
@@ -3264,9 +3471,9 @@ extern "C" int perm_batch_run_ex(perm_ctx* ctx, perm_batch* b, double* results, 
   for (int i = 0; i < b->count; i++) {
     const int n = b->orders[i];
     const double v = b->h_results[3 * i] + b->h_results[3 * i + 1];
-    const double sa = b->h_results[3 * i + 2];
+    const double sa = b->h_results[3 * i + 2] * b->abs_scale[i];
     const int G = b->groups[i];
-    const double rounds = G ? std::ceil((double)n / G) : 2.0 * n;  // roundings per term
+    const double rounds = b->roundings[i];
     double est = v != 0.0 ? (rounds + 16.0) * u * sa / std::fabs(v) : (sa > 0 ? INFINITY : 0.0);
     if (ctx->rel_target > 0 && est > ctx->rel_target && n >= 2) {
       const double* mat = b->values.data() + b->offsets[i];
@@ -3345,7 +3552,7 @@ extern "C" int perm_batch_autotune(perm_ctx* ctx, int n_lo, int n_hi, int* m_out
       int mo[kBatchMaxOrder + 1] = {};
       mo[n] = m;
       perm_batch* b = nullptr;
-      int rc = batch_create_locked(ctx, count, orders.data(), vals.data(), mo, &b);
+      int rc = batch_create_locked(ctx, count, orders.data(), vals.data(), mo, &b, -1, false);
       if (rc) return rc;
       double ms = 1e30, t = 0;
       for (int rep = 0; rep < 3; rep++) {
@@ -3391,7 +3598,7 @@ extern "C" int perm_batch_autotune(perm_ctx* ctx, int n_lo, int n_hi, int* m_out
     for (int v = 0; v < kBatchVariantCount; v++) {
       if (kBatchVariants[v].max_n < n_hi) continue;
       perm_batch* b = nullptr;
-      int rc = batch_create_locked(ctx, (int)orders.size(), orders.data(), vals.data(), nullptr, &b, v);
+      int rc = batch_create_locked(ctx, (int)orders.size(), orders.data(), vals.data(), nullptr, &b, v, false);
       if (rc) return rc;
       double ms = 1e30, t = 0;
       for (int rep = 0; rep < 3; rep++) {

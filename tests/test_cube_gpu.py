@@ -111,3 +111,27 @@ def test_cube_integer_walks_vs_product(engine, orc, pb, n, k):
     for variant in (pb.PERM_KERNEL_DENSE_INT, pb.PERM_KERNEL_DENSE_INT_DD):
         r = engine.exact_dense(A, variant=variant)
         assert abs(r.value - want) <= (r.rel_error_estimate + 2 * U) * want, variant
+
+
+def test_cube_walks_in_a_batch(engine, orc, pb):
+    """From order 25 a batch's matrices walk in column cubes, by launches of
+    their own beside the persistent kernel: values and error estimates in the
+    caller's order, for real, binary and dense matrices mixed with small ones,
+    the same on every run."""
+    rng = np.random.default_rng(21)
+    mats = []
+    for n, d in ((12, 0.5), (25, 0.3), (26, 0.95), (9, 0.6), (27, 0.5), (25, 0.8), (28, 0.4), (24, 0.5)):
+        mats += [_real(n, d, 31), _integers(n, d, 1, 32), _integers(n, d, 4, 33)]
+    mats = [mats[i] for i in rng.permutation(len(mats))]
+    b = engine.batch(mats)
+    try:
+        plain, _ = b.run()
+        again, _ = b.run()
+        values, estimates, _, _ = b.run_ex()
+    finally:
+        b.free()
+    assert np.array_equal(plain, again)
+    for M, p, v, e in zip(mats, plain, values, estimates):
+        r = engine.exact_dense(M)
+        assert abs(v - r.value) <= (e + r.rel_error_estimate + 2 * U) * abs(r.value), M.shape
+        assert abs(p - r.value) <= 1e-10 * abs(r.value), M.shape
