@@ -311,8 +311,8 @@ struct CubeRowsInt {
 };
 
 // Adds the 16 signed terms last x top to (H, L) (Sum2, over column 2's sign
-// first) and their absolute values to m1.
-template <bool kLastExact, class Num>
+// first) and their absolute values to m1.  Exact products keep no low part.
+template <bool kTopExact, bool kLastExact, class Num>
 __device__ __forceinline__ void cube_sum_dd(const CubeArray<15, Num>& top, const CubeArray<11, Num>& last, bool odd,
                                             double& H, double& L, double& m1) {
   dd t[8];
@@ -321,7 +321,7 @@ __device__ __forceinline__ void cube_sum_dd(const CubeArray<15, Num>& top, const
     const int lo = (s & 3) | ((s & 4) << 1);  // sign of column 2 minus
     const Num &t0 = top.v[lo], &t1 = top.v[lo | 4];
     dd d = two_sum(t0.hi, -t1.hi);
-    d.lo = __dadd_rn(d.lo, __dsub_rn(t0.lo, t1.lo));
+    if constexpr (!kTopExact) d.lo = __dadd_rn(d.lo, __dsub_rn(t0.lo, t1.lo));
     m1 = __fma_rn(fabs(last.v[s].hi), __dadd_rn(fabs(t0.hi), fabs(t1.hi)), m1);
     if constexpr (kLastExact) {
       const double h = __dmul_rn(d.hi, last.v[s].hi);
@@ -523,7 +523,7 @@ __global__ void __launch_bounds__(kCubeThreads, 1) ryser_cube_sdd_kernel(const _
           CubeArray<11, CubeDd<0>> last;
           cube.products(top, third, last);
           if constexpr (C::kThird > 0) cube_merge<C::kFirst + C::kSecond, C::kThird>(top, third);
-          cube_sum_dd<false>(top, last, (h & 1) != 0, H, L, m1);
+          cube_sum_dd<false, false>(top, last, (h & 1) != 0, H, L, m1);
         });
   }
   cube_finish(a, two_sum(H, L), true, m1, (a.n & 1) ? 2.0 : -2.0, red);
@@ -591,7 +591,8 @@ __global__ void __launch_bounds__(kCubeThreads, 1) ryser_cube_int_kernel(const _
           cube.products(top, third, last);
           if constexpr (kDd) {
             if constexpr (C::kThird > 0) cube_merge<C::kFirst + C::kSecond, C::kThird>(top, third);
-            cube_sum_dd<C::kLast <= kCubeExactRows>(top, last, (h & 1) != 0, H, L, m1);
+            cube_sum_dd<C::kFirst + C::kSecond + C::kThird <= kCubeExactRows, C::kLast <= kCubeExactRows>(
+                top, last, (h & 1) != 0, H, L, m1);
           } else {
             const double t = cube_sum_f64<(C::kThird > 0), kAbs>(top, third, last, m1);
             acc.add((h & 1) ? -t : t);

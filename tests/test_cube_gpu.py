@@ -88,6 +88,8 @@ def _integers(n, d, top, seed, signed=False):
 
 @pytest.mark.parametrize("n,d,top,signed", [(25, 0.12, 4, False), (25, 0.5, 1, False), (26, 0.4, 3, True),
                                             (27, 0.5, 4, False), (28, 0.7, 4, False), (29, 0.3, 1, False),
+                                            # so few rows in the first chains that their products are exact
+                                            (26, 0.05, 3, True),
                                             # row sums at the int32 runs' limit (four of about 215) and beyond it
                                             (25, 0.5, 33, False), (25, 0.5, 60, False)])
 def test_cube_integer_walks_vs_exact(engine, orc, pb, n, d, top, signed):
