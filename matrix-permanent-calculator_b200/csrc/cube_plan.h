@@ -16,10 +16,13 @@ struct CubeLayout {
   std::vector<int> slot_row;  // row of `mat` in each slot, -1: a row of the constant 1
 };
 
-// The cheapest compiled shape, of at most max_cost, that holds the rows of some four columns of the n x n row-major
-// matrix or of its transpose; false when there is none (orders outside
-// 9..40 among them).
-bool cube_layout(const std::vector<double>& a, int n, double max_cost, CubeLayout* layout);
+// The cheapest compiled shape, of at most max_cost, that holds the rows of some
+// four columns of the n x n row-major matrix or, with `transpose`, of its
+// transpose; false when there is none (orders outside 9..40 among them).  The
+// transpose has the same permanent and saves another 3..6% of the operations,
+// but other terms, whose absolute sum (the scale of every error) was 1.7 times
+// larger in a test: only for walks that certify their error.
+bool cube_layout(const std::vector<double>& a, int n, double max_cost, bool transpose, CubeLayout* layout);
 
 // FP64 operations per 16 terms of a shape's FP64 walk, and the same weighted
 // by the rate its size reaches: measured 0.80..0.85 of the FP64 pipe up to 130

@@ -1470,20 +1470,30 @@ static bool build_cube_int_operand(const CubeLayout& l, DenseOperand* op) {
   return true;
 }
 
+// The FP64 walk's row layout, searched for at most once (the search takes 65 us
+// at n = 25, 0.2 ms at n = 33).
+struct Fp64Rows {
+  int inner = 0, inner1 = 0;
+  long cost8 = 0;  // operations per 8 terms; 0: not searched yet
+  std::vector<double> perm;
+  void choose(const std::vector<double>& a, int n) {
+    if (!cost8) fp64_choose(a, n, &inner, &inner1, &perm, &cost8);
+  }
+};
+
 // The FP64 walk's operand in column cubes; false where a row layout needs
 // fewer operations: their walks reach 0.93 (one level) and 0.87 of the FP64
 // pipe against 0.82.  One level is 32 n operations per 16 terms.  The smallest
 // row layout (levels of 8 and 20 rows) needs 394 + 4n, so cheaper cubes skip
-// the search for one.
-static bool cube_operand_f64(const std::vector<double>& a, int n, DenseOperand* op) {
+// the search for one; below order 30 the search costs more than it could find
+// where the cube needs less than 0.6 of the one-level operations (n = 28,
+// density 0.6, 0.25 ms: 0.29 ms with the host's part, 0.34 with the search).
+static bool cube_operand_f64(const std::vector<double>& a, int n, Fp64Rows* rows, DenseOperand* op) {
   CubeLayout l;
-  if (!cube_layout(a, n, 32.0 * n * 0.82 / 0.93, &l)) return false;
-  if (l.cost > (394.0 + 4.0 * n) * 0.82 / 0.87) {
-    int inner = 0, inner1 = 0;
-    long cost8 = 0;  // operations per 8 terms
-    std::vector<double> perm;
-    fp64_choose(a, n, &inner, &inner1, &perm, &cost8);
-    if (l.cost / 0.82 > 2.0 * (double)cost8 / (inner ? 0.87 : 0.93)) return false;
+  if (!cube_layout(a, n, 32.0 * n * 0.82 / 0.93, false, &l)) return false;
+  if (l.cost > (n < 30 ? 0.6 * 32.0 * n : (394.0 + 4.0 * n) * 0.82 / 0.87)) {
+    rows->choose(a, n);
+    if (l.cost / 0.82 > 2.0 * (double)rows->cost8 / (rows->inner ? 0.87 : 0.93)) return false;
   }
   op->n = n;
   op->variant = PERM_KERNEL_DENSE;
@@ -1494,36 +1504,67 @@ static bool cube_operand_f64(const std::vector<double>& a, int n, DenseOperand* 
   return true;
 }
 
-// The int32 walks' operand (op->variant: plain or certified) in column cubes,
-// for product groups of G (int_group_size); false where a row layout is
-// cheaper or the products need not fit.
-static bool cube_operand_int(const std::vector<double>& a, int n, int G, DenseOperand* op) {
-  CubeLayout cube;
-  if (!cube_layout(a, n, 1e9, &cube)) return false;
-  op->n = n;
-  const bool certified = op->variant == PERM_KERNEL_DENSE_INT_DD;
-  // Against the row layouts' instructions per 8 terms, in cycles per SM, warp
-  // and 16 terms: those issue 0.8 of 4 per cycle (0.77 each; the certified
-  // walk's, 0.95), the cube takes 0.47 per unit of its cost (certified: 100 +
-  // 0.68), measured over the shapes.  The several-level layouts need 0.6 of
-  // the one-level instructions at density 1/2, and the cube less still where
-  // they need less; only above that are they searched for (0.2 ms on the host
-  // at n = 30).
-  const double mine = certified ? 100.0 + 0.68 * cube.cost : 0.47 * cube.cost;
-  const double each = certified ? 0.95 : 0.77;
-  int pair = 0, cost1 = 0, g = 0, x = 0, y = 0;
-  if (certified) intc_layout(a, n, &pair, &cost1);
-  long cost = certified ? 8L * (n + cost1) : 8L * (2 * n + (n + G - 1) / G);
-  if (mine >= each * 0.6 * (double)cost) {
-    std::vector<double> p;
-    if (certified) {
-      intc_two_level_layout(a, n, cost, &g, &pair, &x, &p, &cost);
-      intc_three_level_layout(a, n, cost, &g, &pair, &x, &y, &p, &cost);
-    } else {
-      choose_int_layout(a, n, G, &p, &cost);
+// The int32 walks' row layout, searched for at most once (0.25 ms at n = 30).
+struct IntRows {
+  int group = 0, pair = 0, ngo = 0, ng1 = 0, ng2 = 0;
+  long cost = 0;  // instructions per 8 terms; 0: not searched yet
+  std::vector<double> mat;  // the permuted matrix; empty: the matrix as it is
+  void choose(const std::vector<double>& a, int n, int G, bool certified) {
+    if (cost) return;
+    if (!certified) {
+      const IntLayout l = choose_int_layout(a, n, G, &mat, &cost);
+      group = l.g;
+      ngo = l.ngo;
+      ng1 = l.ng1;
+      ng2 = l.ng2;
+      if (!ngo && !ng1) mat.clear();
+      return;
     }
-    if (mine >= each * (double)cost) return false;
+    int cost1 = 0;
+    group = intc_layout(a, n, &pair, &cost1);
+    cost = 8L * (n + cost1);
+    int g2 = group, p2 = pair, ngo2 = 0;
+    std::vector<double> two, three;
+    if (intc_two_level_layout(a, n, cost, &g2, &p2, &ngo2, &two, &cost)) {
+      group = g2;
+      pair = p2;
+      ngo = ngo2;
+      mat.swap(two);
+    }
+    int g3 = 0, p3 = 0, a1 = 0, a2 = 0;
+    if (intc_three_level_layout(a, n, cost, &g3, &p3, &a1, &a2, &three, &cost)) {
+      group = g3;
+      pair = p3;
+      ngo = 0;
+      ng1 = a1;
+      ng2 = a2;
+      mat.swap(three);
+    }
   }
+};
+
+// The int32 walks' operand (op->variant: plain or certified) in column cubes,
+// where that is the cheaper walk.  Cycles per SM, warp and 16 terms, fitted to
+// both walks at orders 30..34 and densities 0.35..0.9 (the fits are good to
+// 5%): 40 + 0.39 of the cube's cost against 0.77 of the row layout's
+// instructions per 8 terms; certified, 90 + 0.65 against 105 + 0.74.  The
+// several-level row layouts need no less than about 0.55 (certified) and 0.6
+// of the one-level instructions; only above that are they searched for.
+static bool cube_operand_int(const std::vector<double>& a, int n, int G, IntRows* rows, DenseOperand* op) {
+  const bool certified = op->variant == PERM_KERNEL_DENSE_INT_DD;
+  const double base = certified ? 90.0 : 40.0, per = certified ? 0.65 : 0.39;
+  const double row_base = certified ? 105.0 : 0.0, row_per = certified ? 0.74 : 0.77;
+  int pair = 0, cost1 = 0;
+  if (certified) intc_layout(a, n, &pair, &cost1);
+  const double one_level = certified ? 8.0 * (n + cost1) : 8.0 * (2 * n + (n + G - 1) / G);
+  CubeLayout cube;
+  if (!cube_layout(a, n, (row_base + row_per * one_level - base) / per, certified && n >= 28, &cube)) return false;
+  const double mine = base + per * cube.cost;
+  if (mine > row_base + row_per * (certified ? 0.55 : 0.6) * one_level) {
+    rows->choose(a, n, G, certified);
+    if (mine >= row_base + row_per * (double)rows->cost) return false;
+  }
+  op->n = n;
   return build_cube_int_operand(cube, op);
 }
 
@@ -1533,15 +1574,19 @@ static int build_sdd_operand(perm_ctx* ctx, const std::vector<double>& a, int n,
   // for the class arrays and the sum, per 16 terms; 0.63 of the FP64 pipe)
   // unless a row layout is cheaper (per 8 terms, 0.69 dense, 0.56..0.62 the
   // others).  n = 30: 364 values 7.3 ms, dense layout 8.9 ms.  The smallest
-  // row layout (sparse, 6 rows) needs 320 + 6n operations per 8 terms.
+  // row layout (sparse, 6 rows) needs 320 + 6n operations per 8 terms; below
+  // order 30 it is searched for (50 us) only where the cube needs more than 0.7
+  // of the dense layout's time.
   CubeLayout l;
   int inner = 0, inner1 = 0;
   std::vector<double> perm;
-  bool cube = n >= kCubeMinN && cube_layout(a, n, 1e9, &l);
+  bool cube = n >= kCubeMinN && cube_layout(a, n, 1e9, true, &l);
+  bool searched = false;
   if (cube) {
     const double mine = (6.0 * cube_values(kCubeShapes[l.shape]) + 2.0 * n + 280.0) / 0.63;
-    if (mine > 2.0 * (320.0 + 6.0 * n) / 0.62) {
+    if (mine > (n < 30 ? 0.7 * 2.0 * (double)sdd_cost(n, 0) / 0.69 : 2.0 * (320.0 + 6.0 * n) / 0.62)) {
       sdd_choose(a, n, &inner, &inner1, &perm);
+      searched = true;
       cube = mine < 2.0 * (double)sdd_cost(n, inner, inner1, inner) / (inner ? 0.62 : 0.69);
     }
   }
@@ -1552,7 +1597,7 @@ static int build_sdd_operand(perm_ctx* ctx, const std::vector<double>& a, int n,
     build_cube_operand(l, 2, op);
     return PERM_OK;
   }
-  sdd_choose(a, n, &inner, &inner1, &perm);
+  if (!searched) sdd_choose(a, n, &inner, &inner1, &perm);
   const int rc = build_split_operand(ctx, inner ? perm : a, n, op);
   if (rc) return rc;
   op->variant = PERM_KERNEL_DENSE_SDD;
@@ -1588,38 +1633,16 @@ static int build_operand(perm_ctx* ctx, const void* mat, int n, int dtype, int v
     op->pair = 0;
     op->ngo = 0;
     op->ng1 = op->ng2 = 0;
-    std::vector<double> two;
-    if (n >= kCubeMinN && op->variant != PERM_KERNEL_DENSE_TC && cube_operand_int(a, n, G, op)) return PERM_OK;
-    if (op->variant == PERM_KERNEL_DENSE_INT_DD) {
-      int cost1 = 0;
-      op->group = intc_layout(a, n, &op->pair, &cost1);
-      long cost = 8L * (n + cost1);
-      int g2 = op->group, p2 = op->pair, ngo2 = 0;
-      std::vector<double> three;
-      if (intc_two_level_layout(a, n, cost, &g2, &p2, &ngo2, &two, &cost)) {
-        op->group = g2;
-        op->pair = p2;
-        op->ngo = ngo2;
-      }
-      int g3 = 0, p3 = 0, a1 = 0, a2 = 0;
-      if (intc_three_level_layout(a, n, cost, &g3, &p3, &a1, &a2, &three)) {
-        op->group = g3;
-        op->pair = p3;
-        op->ngo = 0;
-        op->ng1 = a1;
-        op->ng2 = a2;
-        a.swap(three);  // walk the permuted matrix (same permanent)
-      } else if (op->ngo) {
-        a.swap(two);
-      }
-    }
-    if (op->variant == PERM_KERNEL_DENSE_INT) {
-      const IntLayout l = choose_int_layout(a, n, G, &two);
-      op->group = l.g;
-      op->ngo = l.ngo;
-      op->ng1 = l.ng1;
-      op->ng2 = l.ng2;
-      if (l.ngo || l.ng1) a.swap(two);  // walk the permuted matrix (same permanent)
+    if (op->variant != PERM_KERNEL_DENSE_TC) {
+      IntRows rows;
+      if (n >= kCubeMinN && cube_operand_int(a, n, G, &rows, op)) return PERM_OK;
+      rows.choose(a, n, G, op->variant == PERM_KERNEL_DENSE_INT_DD);
+      op->group = rows.group;
+      op->pair = rows.pair;
+      op->ngo = rows.ngo;
+      op->ng1 = rows.ng1;
+      op->ng2 = rows.ng2;
+      if (!rows.mat.empty()) a.swap(rows.mat);  // walk the permuted matrix (same permanent)
     }
     op->image.assign(sizeof(int) * (size_t)(n + 1) * np4, 0);
     int* img = reinterpret_cast<int*>(op->image.data());
@@ -1637,10 +1660,12 @@ static int build_operand(perm_ctx* ctx, const void* mat, int n, int dtype, int v
     op->inner = 0;
     op->inner1 = 0;
     if (op->variant == PERM_KERNEL_DENSE) {
-      if (n >= kCubeMinN && cube_operand_f64(a, n, op)) return PERM_OK;
-      std::vector<double> perm;
-      fp64_choose(a, n, &op->inner, &op->inner1, &perm);
-      if (op->inner) a.swap(perm);  // walk the permuted matrix (same permanent)
+      Fp64Rows rows;
+      if (n >= kCubeMinN && cube_operand_f64(a, n, &rows, op)) return PERM_OK;
+      rows.choose(a, n);
+      op->inner = rows.inner;
+      op->inner1 = rows.inner1;
+      if (op->inner) a.swap(rows.perm);  // walk the permuted matrix (same permanent)
     }
     build_fp64_image(a, n, op);
   }
@@ -3161,7 +3186,9 @@ static void batch_cubes(int count, const int* orders, const double* values, std:
       const int G = int_group_size(a, n);
       DenseOperand& op = found[k].op;
       op.variant = G ? PERM_KERNEL_DENSE_INT : PERM_KERNEL_DENSE;
-      if (!(G ? cube_operand_int(a, n, G, &op) : cube_operand_f64(a, n, &op))) op.shape = -1;
+      IntRows int_rows;
+      Fp64Rows rows;
+      if (!(G ? cube_operand_int(a, n, G, &int_rows, &op) : cube_operand_f64(a, n, &rows, &op))) op.shape = -1;
     }
   };
   std::vector<std::thread> threads;

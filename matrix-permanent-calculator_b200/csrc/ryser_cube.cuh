@@ -21,8 +21,9 @@
 // The first two are multiplied into top, the third with the difference over
 // the sign of column 2, the last with the sum of the rest.
 //
-// The host picks the four columns, of the matrix or of its transpose, whose
-// rows fit the cheapest of the compiled shapes (cube_shapes.h).  At density
+// The host picks the four columns (for the certified walks, of the matrix or of
+// its transpose) whose rows fit the cheapest of the compiled shapes
+// (cube_shapes.h).  At density
 // 1/2 that leaves about 0.2 x 16 n row values per 16 terms: for an order-32
 // matrix 284 FP64 operations instead of 1024 for the plain walk, and 640 for
 // the three-level row layout this replaced (n = 32, density 1/2: 6.38 ms
