@@ -2669,6 +2669,23 @@ static int run_skipper(perm_ctx* ctx, int n, const int* rptrs, const int* cols, 
   for (int p = cptrs[n - 1]; p < cptrs[n]; p++) x0[rows[p]] += cvals[p];
 
   SkipArgs a;
+  a.wide = 4;
+  a.exact = 1;
+  double size = 0;
+  for (int k = 0; k < n; k++) {
+    uint64_t seen = 0;
+    for (int p = cptrs[k]; p < cptrs[k + 1]; p++) {
+      if ((seen >> rows[p]) & 1) a.wide = 1;
+      seen |= 1ull << rows[p];
+      if (cvals[p] != std::floor(cvals[p])) a.exact = 0;
+      size += std::fabs(cvals[p]);
+    }
+  }
+  for (int p = 0; p < nnz; p++) {
+    if (rvals[p] != std::floor(rvals[p])) a.exact = 0;
+    size += std::fabs(rvals[p]);
+  }
+  if (!(size < 0x1p50)) a.exact = 0;
   uint32_t off = align16(sizeof(double) * n);
   a.off_cvals = off;
   off = align16(off + sizeof(double) * nnz);
@@ -2702,7 +2719,10 @@ static int run_skipper(perm_ctx* ctx, int n, const int* rptrs, const int* cols, 
   const uint64_t total = 1ull << (n - 1);
   int grid = std::min(kMaxBlocks, ctx->num_sms * occ);
   const uint64_t threads = (uint64_t)grid * block;
-  uint64_t chunk = 256;
+  // 64 indices or more, 32..64 chunks a thread (n = 36, three nonzeros a row:
+  // 8 chunks 2.3..5.1 ms, 32 1.4..2.6, 128 2.3..2.6; n = 27: chunks of 32
+  // indices 0.15 ms, 128 0.09; n = 24: 0.06, 0.09)
+  uint64_t chunk = 64;
   while (chunk < (1ull << 24) && total / (chunk * 2) >= threads * 32) chunk *= 2;
   a.n = n;
   a.total = total;

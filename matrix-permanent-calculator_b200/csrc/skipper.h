@@ -15,6 +15,8 @@ struct SkipArgs {
   uint32_t pack_bytes;  // multiple of 16
   uint32_t off_cvals, off_rptrs, off_cptrs, off_cols, off_rows;
   int n;
+  int wide;         // rows of a column updated at once: 4, or 1 where a column lists a row twice
+  int exact;        // every x is exact in FP64 (integers): it is carried from chunk to chunk
   uint64_t total;    // 2^(n-1) Gray indices
   uint64_t chunk;    // Gray indices per queue entry
   uint64_t nchunks;  // ceil(total / chunk)

@@ -100,3 +100,27 @@ def test_automatic_choice(engine, pb):
     rb = engine.exact_sparse(cb["n"], cb["rptrs"], cb["cols"], cb["rvals"], cb["cptrs"], cb["rows"], cb["cvals"])
     assert rb.kernel == pb.PERM_KERNEL_SKIPPER
     assert rel_err(rb.value, engine.exact_dense(cb["mat"]).value) < 1e-13
+
+
+@pytest.mark.parametrize("n,repeat", [(9, False), (13, False), (17, False), (12, True), (18, True)])
+def test_columns_of_every_length(engine, orc, pb, n, repeat):
+    """Columns of 1..n rows (every remainder of the four taken at once), and
+    arrays that list an entry in two parts: parts add up."""
+    rng = np.random.default_rng(n)
+    A = np.zeros((n, n))
+    for k in range(n):
+        A[(k + np.arange(1 + k % (n // 2 - 1))) % n, k] = rng.integers(1, 4, 1 + k % (n // 2 - 1))
+    c = pb.compress(0, A)
+    if repeat:
+        c = {"n": n, "rptrs": 2 * c["rptrs"], "cptrs": 2 * c["cptrs"], "cols": np.repeat(c["cols"], 2),
+             "rows": np.repeat(c["rows"], 2), "rvals": np.repeat(c["rvals"], 2) / 2,
+             "cvals": np.repeat(c["cvals"], 2) / 2}
+    r = engine.exact_sparse(c["n"], c["rptrs"], c["cols"], c["rvals"], c["cptrs"], c["rows"], c["cvals"],
+                           variant=pb.PERM_KERNEL_SKIPPER)
+    # n roundings of every term, and the terms' absolute sum; one of the result
+    sign = 1.0 - 2.0 * ((np.arange(2 ** (n - 1))[:, None] >> np.arange(n - 1)) & 1)
+    x = A[:, n - 1] + sign @ A[:, :n - 1].T
+    s1 = np.abs(np.prod(x, axis=1)).sum() * 2.0 ** (1 - n)
+    exact = float(orc.perm_exact_int(A)[0])
+    assert abs(r.value - exact) <= 2.0 ** -53 * (n * s1 + abs(exact))
+    assert r.kernel == pb.PERM_KERNEL_SKIPPER
