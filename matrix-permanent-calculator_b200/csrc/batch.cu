@@ -368,19 +368,19 @@ __device__ __noinline__ void walk_range_xs(const double* col, int np, const doub
   }
 }
 
-// Orders below 9 have fewer than 256 Gray indices: lane 0 walks them all.
-__device__ void walk_small(const double* col, int np, const double* x0s, int n, Acc& acc, double& abs_sum) {
-  double x[8];
-  for (int j = 0; j < n; j++) x[j] = x0s[j];
-  const uint64_t total = 1ull << (n - 1);
-  for (uint64_t i = 0; i < total; i++) {
-    if (i) {
-      const int k = __ffsll((long long)i) - 1;
-      const double s = ((i >> (k + 1)) & 1) ? -1.0 : 1.0;
-      for (int j = 0; j < n; j++) x[j] = fma(s, col[k * np + j], x[j]);
+// Orders below 9 have at most 128 Gray indices: each lane takes every 32nd and
+// builds its x from the columns (walked by one lane, x in local memory, order 8
+// took 80 us and was what small batches waited for).
+__device__ void walk_small(const double* col, int np, const double* x0s, int n, int lane, Acc& acc, double& abs_sum) {
+  for (unsigned i = lane; i < 1u << (n - 1); i += 32) {
+    const unsigned g = i ^ (i >> 1);
+    double p = 1.0;
+    for (int j = 0; j < n; j++) {
+      double x = x0s[j];
+      for (int k = 0; k < n - 1; k++)
+        if ((g >> k) & 1) x += col[k * np + j];
+      p *= x;
     }
-    double p = x[0];
-    for (int j = 1; j < n; j++) p *= x[j];
     acc.add((i & 1) ? -p : p);
     abs_sum += fabs(p);
   }
@@ -544,7 +544,7 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) batch_kernel(BatchArgs a) 
     Acc acc;
     double abs_sum = 0.0;
     if (n < 9) {
-      if (lane == 0) walk_small(slot, np, x0, n, acc, abs_sum);
+      walk_small(slot, np, x0, n, lane, acc, abs_sum);
     } else {
       const uint64_t q = t - M.first_tile;
       const uint64_t L = 1ull << M.m;

@@ -482,6 +482,8 @@ struct perm_matrix;
 // whole cubes of 16 terms from here on, and below it the search for four
 // columns (some 30 us on the host) costs what the walk gains.
 constexpr int kCubeMinN = 25;
+// Shortest lane range, as a power of two, that small batches are cut to.
+constexpr int kBatchMinM = 7;
 // In a batch's graph the column-cube walks run in kBatchBranches parallel
 // branches, largest first, each with a CTA per 64 cubes of its threads, so
 // that small ones share the device: smallest order, and at most so many walks
@@ -3357,6 +3359,28 @@ static int batch_create_locked(perm_ctx* ctx, int count, const int* orders, cons
   std::vector<int> order;
   for (int i = 0; i < count; i++)
     if (cube_of[i] < 0) order.push_back(i);
+  // A tile of 2^12 indices per lane takes 0.27 ms whatever else the chip does,
+  // so where the batch has few of them the lane ranges are cut, the longest
+  // first, until there are 16 tiles an SM (32 and 64 are no better), down to
+  // 2^kBatchMinM indices (with 2^6 the columns' staging shows, 2^8 leaves warps
+  // idle).  16 matrices of order 18: 285 -> 43 us, 130 of order 18: 286 -> 100,
+  // of order 21: 495 -> 422, of orders 15..21: 305 -> 190.
+  if (!m_override) {
+    int cap = 0;
+    for (int i : order) cap = std::max(cap, mats[i].m);
+    for (;; cap--) {
+      uint64_t have = 0;
+      for (int i : order) {
+        BatchMatrix& M = mats[i];
+        if (M.n >= 9 && M.m > cap) {
+          M.m = cap;
+          M.ntiles = (uint32_t)((1ull << (M.n - 1)) >> (cap + 5));
+        }
+        have += M.ntiles;
+      }
+      if (cap <= kBatchMinM || have >= 16ull * ctx->num_sms) break;
+    }
+  }
   std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return mats[x].n > mats[y].n; });
   std::stable_sort(cube.begin(), cube.end(), [](const BatchCube& x, const BatchCube& y) { return x.op.n > y.op.n; });
   const int queued = (int)order.size();
@@ -3436,6 +3460,7 @@ static int batch_create_locked(perm_ctx* ctx, int count, const int* orders, cons
   BT(cudaMalloc(&b->d_next, sizeof(unsigned long long)));
   const size_t result_bytes = sizeof(double) * (3 * (size_t)count + 1);
   BT(cudaMalloc(&b->d_results, result_bytes));
+  BT(cudaMemset(b->d_results, 0, result_bytes));
   BT(cudaMallocHost(&b->h_results, result_bytes));
   if (!cube.empty()) {
     std::vector<unsigned char> images(cube_bytes);
@@ -3500,8 +3525,12 @@ static int batch_create_locked(perm_ctx* ctx, int count, const int* orders, cons
   }
   BT(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
   cudaMemsetAsync(b->d_next, 0, sizeof(unsigned long long), ctx->stream);
-  cudaMemsetAsync(b->d_results, 0, result_bytes, ctx->stream);
-  if (branches) cudaEventRecord(br.fork, ctx->stream);
+  // only the column-cube walks add to their results (a node of the graph takes
+  // 10 us: 350 us for 130 matrices of orders 15..21)
+  if (branches) {
+    cudaMemsetAsync(b->d_results, 0, result_bytes, ctx->stream);
+    cudaEventRecord(br.fork, ctx->stream);
+  }
   for (int i = 0; i < branches; i++) cudaStreamWaitEvent(br.stream[i], br.fork, 0);
   for (size_t i = 0; i < cube.size(); i++) {
     const BatchCube& c = cube[i];

@@ -224,3 +224,21 @@ def test_batch_variants_agree_and_autotune_picks_one(pb):
         tuned, _ = eng.batch_exact(mats)
         for a, b in zip(base, tuned):
             assert abs(a - b) <= 1e-11 * abs(b) or abs(a - b) < 1e-12
+
+
+@pytest.mark.parametrize("orders", [[20], [12, 13, 18], [1, 2, 3, 4, 5, 6, 7, 8, 9], [17] * 12 + [8, 14]])
+def test_small_batches_cut_lane_ranges(engine, orc, orders):
+    """Few matrices: tiles down to 2^7 indices a lane, and orders below 9 over
+    the warp's lanes; within the walk's own bound."""
+    rng = np.random.default_rng(len(orders))
+    mats = [(rng.random((n, n)) < 0.7) * (rng.random((n, n)) if i % 2 else 1.0) for i, n in enumerate(orders)]
+    for m in mats:
+        np.fill_diagonal(m, 1.0)
+    b = engine.batch(mats)
+    values, est, _, _ = b.run_ex()
+    again, _ = b.run()
+    b.free()
+    for m, v, e, w in zip(mats, values, est, again):
+        hi, lo = orc.perm_dd(m)[:2]
+        tol = (e + 2.0 ** -52) * abs(hi + lo)
+        assert abs(v - (hi + lo)) <= tol and abs(w - (hi + lo)) <= tol
