@@ -185,10 +185,10 @@ def run_reference_arm(args):
 # a recorded ncu count is only valid for the same template instance compiled
 # from the same text.
 KERNEL_SOURCES = {
-    "int32x": ["ryser_dense_int_sparse.cuh", "ryser_dense_int.cuh", "ryser_dense.cuh", "perman_common.cuh"],
-    "fp64x": ["ryser_dense_2l.cuh", "ryser_dense.cuh", "perman_common.cuh"],
-    "int32x_dd": ["ryser_dense_intc_sparse.cuh", "ryser_dense_intc.cuh", "ryser_dense_int_sparse.cuh",
-                  "ryser_dense_int.cuh", "ryser_dense.cuh", "perman_common.cuh"],
+    "int32x": ["ryser_cube.cuh", "cube_shapes.h", "cube_plan.cpp", "ryser_dense_int.cuh", "ryser_dense.cuh",
+               "perman_common.cuh"],
+    "int32x_dd": ["ryser_cube.cuh", "cube_shapes.h", "cube_plan.cpp", "ryser_dense_sdd.cuh", "ryser_dense_int.cuh",
+                  "ryser_dense.cuh", "perman_common.cuh"],
 }
 
 
@@ -204,6 +204,10 @@ def source_sha16(kname: str) -> str | None:
 
 def kernel_template(kname: str, A: np.ndarray) -> str:
     n = A.shape[0]
+    if n >= 25 and kname in ("int32x", "int32x_dd"):
+        # column-cube walk: the shape depends on the pattern of zeros
+        sha = hashlib.sha256(np.ascontiguousarray(A, dtype=np.float64).tobytes()).hexdigest()[:8]
+        return f"ryser_cube_int_kernel<shape, {'true' if kname == 'int32x_dd' else 'false'}, false>, matrix {sha}"
     if kname == "int32x":
         g, ngo, ng1, ng2 = (sys.modules.get("perman_b200") or load_pkg()).int_layout(A)
         if ng1:
@@ -495,9 +499,9 @@ def main():
         if prof_stale:
             line["roofline"]["frac_stale"] = True
             line["roofline"]["stale_reason"] = prof_stale
-    line["config"]["kernel"] = {1: "FP64-X register kernel", 3: "int32-X register kernel",
+    line["config"]["kernel"] = {1: "FP64-X column-cube kernel", 3: "int32-X column-cube kernel",
                                 5: "tensor-core row sums (tcgen05 kind::i8) + int32 products",
-                                7: "int32-X register kernel, double-double products and sum"}.get(r.kernel, r.kernel)
+                                7: "int32-X column-cube kernel, double-double products and sum"}.get(r.kernel, r.kernel)
     if r.kernel == pb.PERM_KERNEL_DENSE_INT:
         line["config"]["kernel_instance"] = kernel_template("int32x", A)
     if rank == 0 and not args.no_secondary:
@@ -516,20 +520,10 @@ def main():
         f64.run()
         fr = f64.run()
         f64.free()
-        # FP64 operations the walk executes per Gray step: n updates and n - 1
-        # multiplies (one level); in the two-level layout R inner rows at
-        # seven of eight steps (R updates, R - 1 multiplies, times P_out); in
-        # the three-level layout 2 R1 at four steps in eight, 2 R2 at three
-        r1, r2l = pb.fp64_levels(A)
-        if r1:
-            executed = (4 * 2 * r1 + 3 * 2 * r2l + 2 * n - 1) / 8
-        else:
-            executed = (7 * 2 * r2l + 2 * n - 1) / 8 if r2l else 2 * n - 1
         line["secondary"]["dense_n40_fp64x_same_matrix"] = {
             "kernel_ms": fr.kernel_ms, "steps_per_s": total_steps / (fr.kernel_ms * 1e-3),
-            "levels": [r1, r2l],
+            "layout": "column cubes",
             "fp64_equivalent_frac_of_measured_peak": total_steps * ops_per_step / (fr.kernel_ms * 1e-3) / peak_ops,
-            "fp64_pipe_frac_of_measured_peak": total_steps * executed / (fr.kernel_ms * 1e-3) / peak_ops,
             "rel_diff_vs_headline": abs(fr.value - perm_value) / abs(perm_value)}
         line["secondary"]["reference_gpu_same_box"] = reference_gpu(
             A, mean_ms, line["secondary"]["sparse_n36_d020_real"].get("auto_kernel_ms"),
