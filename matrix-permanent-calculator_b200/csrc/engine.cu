@@ -482,6 +482,11 @@ struct perm_matrix;
 // whole cubes of 16 terms from here on, and below it the search for four
 // columns (some 30 us on the host) costs what the walk gains.
 constexpr int kCubeMinN = 25;
+// ... and of the accuracy policy's whole FP64 walks: the cube sums its own
+// |term|, the row layouts pay for a sample (20..60 us; real, density 1/2: n = 20
+// 95 against 57 us, n = 23 115 and 60).  Below 20 every FP64 walk is the
+// one-level one, as perm_exact_dense_noalloc's is.
+constexpr int kCubeSumMinN = 20;
 // Shortest lane range, as a power of two, that small batches are cut to.
 constexpr int kBatchMinM = 7;
 // In a batch's graph the column-cube walks run in kBatchBranches parallel
@@ -1611,7 +1616,16 @@ static int build_sdd_operand(perm_ctx* ctx, const std::vector<double>& a, int n,
   return PERM_OK;
 }
 
-static int build_operand(perm_ctx* ctx, const void* mat, int n, int dtype, int variant, DenseOperand* op) {
+// No cube beats the row layouts above density 0.8 or so at orders 20..24.
+static bool sparse_enough(const std::vector<double>& a) {
+  size_t nonzeros = 0;
+  for (double v : a) nonzeros += v != 0.0;
+  return nonzeros <= a.size() * 8 / 10;
+}
+
+// `own_sum`: the operand is walked in one piece under the accuracy policy.
+static int build_operand(perm_ctx* ctx, const void* mat, int n, int dtype, int variant, DenseOperand* op,
+                         bool own_sum = false) {
   std::vector<double> a((size_t)n * n);
   for (size_t i = 0; i < a.size(); i++) a[i] = elem(mat, dtype, i);
   op->n = n;
@@ -1666,7 +1680,8 @@ static int build_operand(perm_ctx* ctx, const void* mat, int n, int dtype, int v
     op->inner1 = 0;
     if (op->variant == PERM_KERNEL_DENSE) {
       Fp64Rows rows;
-      if (n >= kCubeMinN && cube_operand_f64(a, n, &rows, op)) return PERM_OK;
+      if (n >= (own_sum && sparse_enough(a) ? kCubeSumMinN : kCubeMinN) && cube_operand_f64(a, n, &rows, op))
+        return PERM_OK;
       rows.choose(a, n);
       op->inner = rows.inner;
       op->inner1 = rows.inner1;
@@ -2531,7 +2546,8 @@ extern "C" int perm_exact_dense_ex(perm_ctx* ctx, const void* mat, int n, int dt
   int first = 0;
   if (variant == 0 && nshards == 1 && ctx->rel_target > 0 && (rc = policy_plan(ctx, mat, n, dtype, &first)))
     return rc;
-  if ((rc = build_operand(ctx, mat, n, dtype, first ? first : variant, &op))) return rc;
+  if ((rc = build_operand(ctx, mat, n, dtype, first ? first : variant, &op,
+                          nshards == 1 && variant == 0 && ctx->rel_target > 0))) return rc;
   // shards are Gray-index ranges of the walking kernels; the tensor-core
   // kernel's operand image is the int32-X one
   if (nshards > 1 && op.variant == PERM_KERNEL_DENSE_TC) op.variant = PERM_KERNEL_DENSE_INT;

@@ -137,3 +137,18 @@ def test_cube_walks_in_a_batch(engine, orc, pb):
         r = engine.exact_dense(M)
         assert abs(v - r.value) <= (e + r.rel_error_estimate + 2 * U) * abs(r.value), M.shape
         assert abs(p - r.value) <= 1e-10 * abs(r.value), M.shape
+
+
+@pytest.mark.parametrize("n,d", [(19, 0.5), (20, 0.3), (20, 0.7), (21, 0.5), (24, 0.6), (22, 0.95)])
+def test_whole_walks_with_own_term_sum(engine, orc, n, d):
+    """Policy calls below order 25: value within the reported bound, and the
+    sum of the absolute terms against direct evaluation."""
+    A = _real(n, d, 17)
+    r = engine.exact_dense(A)
+    hi, lo = orc.perm_dd(A)[:2]
+    assert abs(r.value - (hi + lo)) <= (r.rel_error_estimate + 2 * U) * abs(hi + lo)
+    if n == 20:
+        sign = 1.0 - 2.0 * ((np.arange(2 ** (n - 1))[:, None] >> np.arange(n - 1)) & 1)
+        s1 = np.abs(np.prod(A[:, n - 1] + sign @ A[:, :n - 1].T, axis=1)).sum() * 2.0 ** (1 - n)
+        # x carries n roundings, the product n more, either way
+        assert abs(r.abs_term_sum - s1) <= 1e-9 * s1
