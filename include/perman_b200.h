@@ -175,7 +175,7 @@ int perm_exact_dense_ex(perm_ctx* ctx, const void* mat, int n, int dtype, int va
  * policy; < 0 also skips the estimate):
  *  - a zero pattern without a perfect matching returns exactly 0;
  *  - whole walks of integer matrices whose group products fit in int32 run
- *    PERM_KERNEL_DENSE_INT_DD at once (about 1.4 int32-X walks), and real
+ *    PERM_KERNEL_DENSE_INT_DD at once (1.4 int32-X walks in rows, 1.9 in cubes), and real
  *    matrices of order 12..40 whose three sparsest columns touch so few rows
  *    R that the sparse layout's (7 (6R + 9) + 6n + 5) / 8 FP64 operations
  *    per Gray step are at most FP64 X's 2n run PERM_KERNEL_DENSE_SDD in
@@ -183,8 +183,8 @@ int perm_exact_dense_ex(perm_ctx* ctx, const void* mat, int n, int dtype, int va
  *  - for other nonnegative real matrices of order 28..40 the FP64-X walk's
  *    bound is predicted on the device before any walk (stratified sample of
  *    sum |term| and a weighted-Rasmussen estimate of perm, 4096 trials); when
- *    it is above 1.5x the target PERM_KERNEL_DENSE_SDD (about 4.2 FP64-X
- *    walks in the dense layout, less in the sparse one) runs at once and
+ *    it is above 1.5x the target PERM_KERNEL_DENSE_SDD (about 3.6 FP64-X
+ *    walks in column cubes, 4.2 in the dense row layout) runs at once and
  *    alone;
  *  - a result whose bound exceeds the target is cross-checked against
  *    B = A^T with its first row times 3 (perm(B) = 3 perm(A), independent
@@ -195,7 +195,7 @@ int perm_exact_dense_ex(perm_ctx* ctx, const void* mat, int n, int dtype, int va
  *    (orders 4..40), since it rarely passes there;
  *  - otherwise it is recomputed by a certified kernel: PERM_KERNEL_DENSE_INT_DD
  *    (integer, orders 8..64, directly after an int32-X first pass),
- *    PERM_KERNEL_DENSE_SDD (orders 4..40, about 4.2 FP64-X walks) or the
+ *    PERM_KERNEL_DENSE_SDD (orders 4..40, about 4 FP64-X walks) or the
  *    double-double kernel (orders <= 40, where neither applies).
  * kernel_ms covers every launch.  PERM_KERNEL_DENSE_DD forces that kernel. */
 int perm_ctx_set_rel_target(perm_ctx* ctx, double rel_target);
@@ -222,6 +222,11 @@ int perm_exact_dense_plan(perm_ctx* ctx, const void* mat, int n, int dtype, int*
  * the device, and the context stays usable.  0 switches it off.  No
  * counterpart in the reference (which has no device waits to bound). */
 int perm_ctx_inject_wait_timeout(perm_ctx* ctx, int launches);
+
+/* The layout queries below describe the row layouts: what the walks use below
+ * order 25 (the accuracy policy's whole FP64 walks: below order 20), and from
+ * there on for matrices too dense for the column-cube walk, which sums the 16
+ * sign choices of four columns at once. */
 
 /* Host only (no device): the layout PERM_KERNEL_DENSE_SDD uses for the
  * row-major n x n matrix `mat`: the number of inner rows R of the sparse
@@ -333,8 +338,8 @@ int perm_exact_dense_tc_rounds(perm_ctx* ctx, const void* mat, int n, int dtype,
  *    decomposition and X re-anchoring of perm_exact_dense_ex(PERM_KERNEL_DENSE)'s
  *    one-level walks, so its value equals that call's to the last bit on the
  *    same device wherever that call also walks one level (orders below 20,
- *    and matrices without a sparse enough column triple); where that call
- *    walks a two- or three-level row layout the two agree to rounding.
+ *    and matrices without sparse enough columns); where that call walks a
+ *    two- or three-level row layout or column cubes the two agree to rounding.
  *    Unlike perm_exact_dense it returns no error estimate and applies no
  *    accuracy policy (no int32-X, split-dd or double-double pass), so on
  *    matrices with heavy cancellation its error is that of one FP64-X walk;
@@ -385,7 +390,9 @@ int perm_batch_exact(perm_ctx* ctx, int count, const int* orders, const double* 
  * whose nonzeros lie in at most 8 / 16 rows for FP64 X, 6 / 12 rows for
  * int32 X; those rows are walked alone at seven of eight Gray steps, and in
  * int32 X a group whose other rows' product is 0 skips its seven vanishing
- * terms). */
+ * terms), gives matrices from order 22 that walk in column cubes a launch of
+ * their own in the graph, and cuts lane ranges where a batch is too small to
+ * fill the device. */
 int perm_batch_autotune(perm_ctx* ctx, int n_lo, int n_hi, int* m_out);
 /* The batch kernel variant later perm_batch_create calls use (0 = the
  * general one, orders up to 40): its largest order, threads per block, CTAs

@@ -25,9 +25,9 @@
 // its transpose) whose rows fit the cheapest of the compiled shapes
 // (cube_shapes.h).  At density
 // 1/2 that leaves about 0.2 x 16 n row values per 16 terms: for an order-32
-// matrix 284 FP64 operations instead of 1024 for the plain walk, and 640 for
-// the three-level row layout this replaced (n = 32, density 1/2: 6.38 ms
-// then, 2.3..2.7 ms by shape now).
+// matrix some 300 FP64 operations instead of 1024 for the plain walk, and 640
+// for the three-level row layout this replaced (n = 32, density 1/2: 5.8..6.4 ms
+// then, 2.3..3.6 ms by shape now).
 //
 // Bound: the FP64 pipe, 80..85% of it on order-32 shapes up to 130 row values
 // (the rest are fixed latencies between dependent products: 2.4 warps' worth
