@@ -78,7 +78,9 @@ typedef struct {
   double kernel_ms;   /* device time of the compute kernel (CUDA events)    */
   int kernel;         /* PERM_KERNEL_*                                      */
   int n;
-  double abs_term_sum;       /* estimate of sum_i |term(i)| (cancellation scale) */
+  double abs_term_sum;       /* estimate of sum_i |term(i)| (cancellation scale); of the
+                                terms that were walked: certified walks from order 25
+                                may take the transpose's */
   double rel_error_estimate; /* estimated relative error of (hi, lo) (0: not estimated);
                                 value, their sum rounded once, adds at most 2^-53 */
 } perm_result;

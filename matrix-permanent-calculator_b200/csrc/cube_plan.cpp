@@ -2,6 +2,7 @@
 #include "cube_plan.h"
 
 #include <algorithm>
+#include <cmath>
 #include <cstdint>
 #include <cstring>
 #include <initializer_list>
@@ -113,7 +114,41 @@ void collect_quads(const std::vector<uint64_t>& sup, int n, int candidates, bool
     }
 }
 
+// Scale of the terms of a walk of the matrix, or of its transpose: log2 of the
+// products over its rows of their absolute sums and of their Euclidean norms.
+struct TermScale {
+  double sum = 0.0, norm = 0.0;
+};
+TermScale term_scale(const std::vector<double>& a, int n, bool transpose) {
+  TermScale t;
+  for (int i = 0; i < n; i++) {
+    const double* row = a.data() + (transpose ? i : (size_t)i * n);
+    const size_t step = transpose ? n : 1;
+    double sum = 0.0, squares = 0.0;
+    for (int k = 0; k < n; k++) sum += std::fabs(row[k * step]);
+    for (int k = 0; k < n; k++) {
+      const double v = row[k * step] / sum;
+      squares += v * v;
+    }
+    const double l = std::log2(sum);
+    t.sum += l;
+    t.norm += l + 0.5 * std::log2(squares);
+  }
+  return t;
+}
+
 }  // namespace
+
+// One bit is allowed, in which 75% (order 36, density 0.2, values (0,1]) to 100%
+// (order 30, 0/1) of matrices whose rows and columns have no sizes of their own
+// pass.  Of 60000 matrices of order 13 with rows, columns or blocks scaled by up
+// to 10^4, the transposes that passed had sums of |term| at most 17 times the
+// matrix's, 2.7 times in 99 of 100.
+WalkSide walk_side(const std::vector<double>& a, int n) {
+  const TermScale own = term_scale(a, n, false), other = term_scale(a, n, true);
+  if (!(other.sum <= own.sum + 1.0 && other.norm <= own.norm + 1.0)) return WalkSide::kMatrix;
+  return other.sum < own.sum - 8.0 && other.norm < own.norm - 8.0 ? WalkSide::kTranspose : WalkSide::kEither;
+}
 
 double cube_shape_ops(int shape) {
   const CubeShape& s = kCubeShapes[shape];

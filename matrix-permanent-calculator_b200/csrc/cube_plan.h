@@ -16,12 +16,21 @@ struct CubeLayout {
   std::vector<int> slot_row;  // row of `mat` in each slot, -1: a row of the constant 1
 };
 
+// Which of a matrix and its transpose (same permanent, other terms) a walk may
+// take.  Every error is a fraction of the terms' absolute sum.  The size of a
+// row is a factor of every term and costs nothing, but columns of different
+// sizes make that sum larger without limit, so the transpose of a matrix whose
+// rows differ in size must not be walked, and that of a matrix whose columns do
+// (by 8 bits in all, in sums and in norms) is the one to walk.
+enum class WalkSide { kMatrix, kEither, kTranspose };
+WalkSide walk_side(const std::vector<double>& a, int n);
+
 // The cheapest compiled shape, of at most max_cost, that holds the rows of some
 // four columns of the n x n row-major matrix or, with `transpose`, of its
 // transpose; false when there is none (orders outside 9..40 among them).  The
-// transpose has the same permanent and saves another 3..6% of the operations,
-// but other terms, whose absolute sum (the scale of every error) was 1.7 times
-// larger in a test: only for walks that certify their error.
+// transpose saves another 3..6% of the operations; even where walk_side allows
+// either, its terms' absolute sum may be a few times larger, so it is only for
+// double-double walks.
 bool cube_layout(const std::vector<double>& a, int n, double max_cost, bool transpose, CubeLayout* layout);
 
 // FP64 operations per 16 terms of a shape's FP64 walk, and the same weighted

@@ -1560,7 +1560,9 @@ struct IntRows {
 // instructions per 8 terms; certified, 90 + 0.65 against 105 + 0.74.  The
 // several-level row layouts need no less than about 0.55 (certified) and 0.6
 // of the one-level instructions; only above that are they searched for.
-static bool cube_operand_int(const std::vector<double>& a, int n, int G, IntRows* rows, DenseOperand* op) {
+// `transpose`: the transpose may be walked instead (certified walk).
+static bool cube_operand_int(const std::vector<double>& a, int n, int G, bool transpose, IntRows* rows,
+                             DenseOperand* op) {
   const bool certified = op->variant == PERM_KERNEL_DENSE_INT_DD;
   const double base = certified ? 90.0 : 40.0, per = certified ? 0.65 : 0.39;
   const double row_base = certified ? 105.0 : 0.0, row_per = certified ? 0.74 : 0.77;
@@ -1568,7 +1570,7 @@ static bool cube_operand_int(const std::vector<double>& a, int n, int G, IntRows
   if (certified) intc_layout(a, n, &pair, &cost1);
   const double one_level = certified ? 8.0 * (n + cost1) : 8.0 * (2 * n + (n + G - 1) / G);
   CubeLayout cube;
-  if (!cube_layout(a, n, (row_base + row_per * one_level - base) / per, certified && n >= 28, &cube)) return false;
+  if (!cube_layout(a, n, (row_base + row_per * one_level - base) / per, transpose, &cube)) return false;
   const double mine = base + per * cube.cost;
   if (mine > row_base + row_per * (certified ? 0.55 : 0.6) * one_level) {
     rows->choose(a, n, G, certified);
@@ -1578,8 +1580,17 @@ static bool cube_operand_int(const std::vector<double>& a, int n, int G, IntRows
   return build_cube_int_operand(cube, op);
 }
 
-static int build_sdd_operand(perm_ctx* ctx, const std::vector<double>& a, int n, DenseOperand* op) {
+static std::vector<double> transposed(const std::vector<double>& a, int n) {
+  std::vector<double> t(a.size());
+  for (int j = 0; j < n; j++)
+    for (int k = 0; k < n; k++) t[(size_t)k * n + j] = a[(size_t)j * n + k];
+  return t;
+}
+
+static int build_sdd_operand(perm_ctx* ctx, std::vector<double> a, int n, DenseOperand* op) {
   if (n < 4 || n > 40) return fail(ctx, PERM_EUNSUPPORTED, "split-dd kernel covers orders 4..40 (got %d)", n);
+  const WalkSide side = n >= kCubeMinN ? walk_side(a, n) : WalkSide::kMatrix;
+  if (side == WalkSide::kTranspose) a = transposed(a, n);
   // The column-cube walk (6 operations per row value, 2 per row and about 280
   // for the class arrays and the sum, per 16 terms; 0.63 of the FP64 pipe)
   // unless a row layout is cheaper (per 8 terms, 0.69 dense, 0.56..0.62 the
@@ -1590,7 +1601,7 @@ static int build_sdd_operand(perm_ctx* ctx, const std::vector<double>& a, int n,
   CubeLayout l;
   int inner = 0, inner1 = 0;
   std::vector<double> perm;
-  bool cube = n >= kCubeMinN && cube_layout(a, n, 1e9, true, &l);
+  bool cube = n >= kCubeMinN && cube_layout(a, n, 1e9, side == WalkSide::kEither, &l);
   bool searched = false;
   if (cube) {
     const double mine = (6.0 * cube_values(kCubeShapes[l.shape]) + 2.0 * n + 280.0) / 0.63;
@@ -1654,7 +1665,16 @@ static int build_operand(perm_ctx* ctx, const void* mat, int n, int dtype, int v
     op->ng1 = op->ng2 = 0;
     if (op->variant != PERM_KERNEL_DENSE_TC) {
       IntRows rows;
-      if (n >= kCubeMinN && cube_operand_int(a, n, G, &rows, op)) return PERM_OK;
+      // the transpose's search costs more than it saves below order 28
+      const WalkSide side = op->variant == PERM_KERNEL_DENSE_INT_DD && n >= 28 ? walk_side(a, n) : WalkSide::kMatrix;
+      if (side == WalkSide::kTranspose) {
+        std::vector<double> t = transposed(a, n);
+        if (const int g = int_group_size(t, n)) {
+          G = g;
+          a.swap(t);
+        }
+      }
+      if (n >= kCubeMinN && cube_operand_int(a, n, G, side == WalkSide::kEither, &rows, op)) return PERM_OK;
       rows.choose(a, n, G, op->variant == PERM_KERNEL_DENSE_INT_DD);
       op->group = rows.group;
       op->pair = rows.pair;
@@ -3285,7 +3305,7 @@ static void batch_cubes(int count, const int* orders, const double* values, std:
       op.variant = G ? PERM_KERNEL_DENSE_INT : PERM_KERNEL_DENSE;
       IntRows int_rows;
       Fp64Rows rows;
-      if (!(G ? cube_operand_int(a, n, G, &int_rows, &op) : cube_operand_f64(a, n, &rows, &op))) op.shape = -1;
+      if (!(G ? cube_operand_int(a, n, G, false, &int_rows, &op) : cube_operand_f64(a, n, &rows, &op))) op.shape = -1;
     }
   };
   std::vector<std::thread> threads;
