@@ -1589,8 +1589,15 @@ static std::vector<double> transposed(const std::vector<double>& a, int n) {
 
 static int build_sdd_operand(perm_ctx* ctx, std::vector<double> a, int n, DenseOperand* op) {
   if (n < 4 || n > 40) return fail(ctx, PERM_EUNSUPPORTED, "split-dd kernel covers orders 4..40 (got %d)", n);
-  const WalkSide side = n >= kCubeMinN ? walk_side(a, n) : WalkSide::kMatrix;
-  if (side == WalkSide::kTranspose) a = transposed(a, n);
+  WalkSide side = n >= kCubeMinN ? walk_side(a, n) : WalkSide::kMatrix;
+  if (side != WalkSide::kMatrix) {
+    // the callers checked the matrix's rows, not the transpose's
+    std::vector<double> t = transposed(a, n);
+    if (!split_rows_ok(t, n))
+      side = WalkSide::kMatrix;
+    else if (side == WalkSide::kTranspose)
+      a.swap(t);
+  }
   // The column-cube walk (6 operations per row value, 2 per row and about 280
   // for the class arrays and the sum, per 16 terms; 0.63 of the FP64 pipe)
   // unless a row layout is cheaper (per 8 terms, 0.69 dense, 0.56..0.62 the

@@ -54,3 +54,16 @@ def test_scaled_integer_matrices(engine, pb, n, axis):
         assert r.rel_error_estimate < 1e-10
         tol = 2 * U + r.rel_error_estimate + want.rel_error_estimate
         assert abs(r.value / np.prod(s) / want.value - 1.0) <= tol
+
+
+@pytest.mark.parametrize("n", [25, 30])
+def test_column_beyond_the_split_is_accepted(engine, pb, n):
+    """Split-dd takes rows with absolute sums below 2^1020.  A column may add
+    up to more: then the transpose is no choice, but the call is not refused
+    (its terms overflow; the status is what is asked here)."""
+    A = _matrix(n, 0.5, 1)
+    A[:8, 0] = 2.0 ** 1018
+    assert A.sum(axis=0).max() >= 2.0 ** 1020 > A.sum(axis=1).max()
+    for variant in (pb.PERM_KERNEL_DENSE_SDD, 0):
+        r = engine.exact_dense(A, variant=variant)
+        assert r.kernel in (pb.PERM_KERNEL_DENSE, pb.PERM_KERNEL_DENSE_DD, pb.PERM_KERNEL_DENSE_SDD)
