@@ -137,6 +137,39 @@ TermScale term_scale(const std::vector<double>& a, int n, bool transpose) {
   return t;
 }
 
+// Rows of very different sizes: sorted into the classes of a cube their products
+// could leave the range of FP64, which in the caller's order they may not.  So
+// where the absolute sums above 1 multiply to more than 2^900 or those below 1
+// to less than 2^-700 (low parts of double-double products are 2^-106 of the
+// high ones, and cancelling rows smaller than their sums), every row is divided
+// by the power of two of its sum; *exp2 is the exponent the permanent lost.
+// False for rows this cannot be done to exactly (not finite, or with entries
+// that would become subnormal).
+bool bring_into_range(std::vector<double>* mat, int n, int* exp2) {
+  *exp2 = 0;
+  int up = 0, down = 0;
+  std::vector<int> e(n, 0);
+  for (int i = 0; i < n; i++) {
+    double sum = 0.0;
+    for (int k = 0; k < n; k++) sum += std::fabs((*mat)[(size_t)i * n + k]);
+    if (!std::isfinite(sum)) return false;
+    if (sum == 0.0) continue;
+    e[i] = std::ilogb(sum);
+    up += std::max(e[i] + 1, 0);
+    down += std::min(e[i], 0);
+  }
+  if (up <= 900 && down >= -700) return true;
+  for (int i = 0; i < n; i++) {
+    for (int k = 0; k < n; k++) {
+      double& v = (*mat)[(size_t)i * n + k];
+      if (v != 0.0 && std::ilogb(v) - e[i] < -1000) return false;
+      v = std::ldexp(v, -e[i]);
+    }
+    *exp2 += e[i];
+  }
+  return true;
+}
+
 }  // namespace
 
 // One bit is allowed, in which 75% (order 36, density 0.2, values (0,1]) to 100%
@@ -365,7 +398,9 @@ bool cube_layout(const std::vector<double>& a, int n, double max_cost, bool tran
   layout->mat.resize((size_t)n * n);
   for (int i = 0; i < n; i++)
     for (int k = 0; k < n; k++) layout->mat[(size_t)i * n + k] = at(row_order[i], col_order[k]);
-  return true;
+  if (bring_into_range(&layout->mat, n, &layout->exp2)) return true;
+  layout->shape = -1;
+  return false;
 }
 
 }  // namespace perm

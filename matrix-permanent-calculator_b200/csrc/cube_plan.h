@@ -13,6 +13,7 @@ struct CubeLayout {
   double cost = 0;            // cube_shape_cost of the shape
   std::vector<double> mat;    // row-major n x n: the fast columns first, rows in slot order
                               // (the matrix or its transpose; same permanent)
+  int exp2 = 0;               // the permanent is mat's times 2^exp2 (rows of extreme sizes are scaled)
   std::vector<int> slot_row;  // row of `mat` in each slot, -1: a row of the constant 1
 };
 
@@ -27,10 +28,10 @@ WalkSide walk_side(const std::vector<double>& a, int n);
 
 // The cheapest compiled shape, of at most max_cost, that holds the rows of some
 // four columns of the n x n row-major matrix or, with `transpose`, of its
-// transpose; false when there is none (orders outside 9..40 among them).  The
-// transpose saves another 3..6% of the operations; even where walk_side allows
-// either, its terms' absolute sum may be a few times larger, so it is only for
-// double-double walks.
+// transpose; false when there is none (orders outside 9..40 and matrices with
+// infinities or NaNs among them).  The transpose saves another 3..6% of the
+// operations; even where walk_side allows either, its terms' absolute sum may be
+// a few times larger, so it is only for double-double walks.
 bool cube_layout(const std::vector<double>& a, int n, double max_cost, bool transpose, CubeLayout* layout);
 
 // FP64 operations per 16 terms of a shape's FP64 walk, and the same weighted

@@ -765,6 +765,7 @@ struct DenseOperand {
   int inner1 = 0;  // split-dd three-level layout: rows 0..inner1-1 hold column 0's support (0: not)
   int shape = -1;  // column-cube walk (ryser_cube.cuh): its shape, -1: one of the row layouts above
   bool abs_sum = false;  // ... which sums |term| too (FP64 walk; the certified ones always do)
+  int exp2 = 0;  // ... whose results are multiplied by 2^exp2
   std::vector<double> sums;  // ... and the fast columns' sums, then (split-dd) those of their remainders
   std::vector<unsigned char> image;
 };
@@ -1399,6 +1400,7 @@ static void build_cube_operand(const CubeLayout& l, int parts, DenseOperand* op)
   const std::vector<unsigned char> columns = std::move(op->image);
   const double* col = reinterpret_cast<const double*>(columns.data());
   op->shape = l.shape;
+  op->exp2 = l.exp2;
   op->image.assign(sizeof(double) * parts * nc * N, 0);
   op->sums.assign((size_t)parts * kCubeMaxSums, 0.0);
   double* img = reinterpret_cast<double*>(op->image.data());
@@ -1436,7 +1438,7 @@ static bool build_cube_int_operand(const CubeLayout& l, DenseOperand* op) {
   const CubeShape& shape = kCubeShapes[l.shape];
   const int N = cube_rows(shape);
   std::vector<double> rowabs;
-  if (!int_row_abs(l.mat, n, rowabs)) return false;
+  if (l.exp2 || !int_row_abs(l.mat, n, rowabs)) return false;
   for (int i = 0; i < 16; i++) {
     const int rows = shape.rows[cube_class(i)], runs = rows - cube_left(rows);
     for (int r = 0; r < runs; r += 4) {
@@ -2129,14 +2131,14 @@ static int dense_collect(perm_ctx* ctx, const DenseOperand& op, const DensePlan&
     ctx->split_m2 = ctx->h_out[13] * 4.0;
   } else if (sums) {
     // the int32-X walk's terms are prod y = 2^n prod x (|factor| 2^(1-n))
-    ctx->walk_m1 = ctx->h_out[12] * (op.variant == PERM_KERNEL_DENSE_INT_DD ? std::ldexp(1.0, 1 - op.n) : 2.0);
+    ctx->walk_m1 = std::ldexp(ctx->h_out[12], op.variant == PERM_KERNEL_DENSE_INT_DD ? 1 - op.n : 1 + op.exp2);
     const uint64_t threads = (uint64_t)p.grid * operand_threads(op);
     ctx->walk_terms_per_thread = ((p.nblocks + threads - 1) / threads) << p.m;
   }
   float ms = 0;
   CU(ctx, cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));
   const int n = op.n;
-  const double hi = ctx->h_out[0], lo = ctx->h_out[1];
+  const double hi = std::ldexp(ctx->h_out[0], op.exp2), lo = std::ldexp(ctx->h_out[1], op.exp2);
   out->hi = hi;
   out->lo = lo;
   out->value = hi + lo;
@@ -3248,6 +3250,7 @@ struct perm_batch {
   unsigned* d_cube_tickets = nullptr;
   std::vector<double> roundings;  // per matrix: roundings per term
   std::vector<double> abs_scale;  // per matrix: factor of its sum |term|
+  std::vector<std::pair<int, int>> exp2;  // matrices whose three results are multiplied by 2^second
   std::vector<int> groups;       // per matrix: 0 = FP64 X, else the int32-X group size
   std::vector<int> orders;       // host copies for double-double reruns
   std::vector<uint64_t> offsets;
@@ -3482,6 +3485,7 @@ static int batch_create_locked(perm_ctx* ctx, int count, const int* orders, cons
   for (const BatchCube& c : cube) {
     // |factor| = 2, of prod y = 2^n prod x in the int32 walk
     b->abs_scale[c.index] = c.op.variant == PERM_KERNEL_DENSE_INT ? std::ldexp(1.0, 1 - c.op.n) : 2.0;
+    if (c.op.exp2) b->exp2.push_back({c.index, c.op.exp2});
     if (c.op.variant == PERM_KERNEL_DENSE_INT) b->roundings[c.index] = cube_factors(kCubeShapes[c.op.shape]) + 1.0;
   }
   b->offsets = src_off;
@@ -3626,6 +3630,8 @@ static int batch_run_locked(perm_ctx* ctx, perm_batch* b, double* results, doubl
   memcpy(&errflag, b->h_results + 3 * (size_t)b->count, sizeof errflag);
   if (errflag) return fail(ctx, PERM_ETIMEOUT, "shared-memory staging wait timed out on device %d", ctx->device);
   if (kernel_ms) *kernel_ms = ms;
+  for (const auto& [i, exp2] : b->exp2)
+    for (int k = 0; k < 3; k++) b->h_results[3 * i + k] = std::ldexp(b->h_results[3 * i + k], exp2);
   if (results)
     for (int i = 0; i < b->count; i++) {
       results[2 * i] = b->h_results[3 * i];

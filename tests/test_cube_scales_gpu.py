@@ -67,3 +67,34 @@ def test_column_beyond_the_split_is_accepted(engine, pb, n):
     for variant in (pb.PERM_KERNEL_DENSE_SDD, 0):
         r = engine.exact_dense(A, variant=variant)
         assert r.kernel in (pb.PERM_KERNEL_DENSE, pb.PERM_KERNEL_DENSE_DD, pb.PERM_KERNEL_DENSE_SDD)
+
+
+@pytest.mark.parametrize("n", [21, 25, 29, 32])
+def test_rows_of_extreme_sizes(engine, pb, n):
+    """Rows times 2^200 and 2^-200 in turn: their products stay in range when
+    rows are multiplied as they come, and would not when they are sorted into
+    the classes of a cube.  Scaling is exact, so the permanent is too."""
+    s = np.where(np.arange(n) % 2, 2.0 ** -200, 2.0 ** 200)
+    factor = 2.0 ** (200 * (n % 2))
+    for seed in range(3):
+        A = _matrix(n, 0.5, seed)
+        want = engine.exact_dense(A, variant=pb.PERM_KERNEL_DENSE_SDD)
+        for variant in (0, pb.PERM_KERNEL_DENSE, pb.PERM_KERNEL_DENSE_SDD):
+            r = engine.exact_dense(A * s[:, None], variant=variant)
+            tol = 2 * U + r.rel_error_estimate + want.rel_error_estimate
+            assert tol < 1e-8 and abs(r.value / factor / want.value - 1.0) <= tol, (seed, variant, r)
+
+
+def test_rows_of_extreme_sizes_in_a_batch(engine):
+    n = 26
+    s = np.where(np.arange(n) % 2, 2.0 ** -200, 2.0 ** 200)
+    mats = [_matrix(n, 0.5, seed) for seed in range(3)]
+    b = engine.batch(mats + [A * s[:, None] for A in mats])
+    try:
+        for _ in range(2):
+            values, estimates, _, _ = b.run_ex()
+            for k in range(3):
+                tol = 2 * U + estimates[k] + estimates[k + 3]
+                assert tol < 1e-8 and abs(values[k + 3] / values[k] - 1.0) <= tol, k
+    finally:
+        b.free()
