@@ -167,6 +167,13 @@ int perm_exact_sparse_ex(perm_ctx* ctx, int n, const int* rptrs, const int* cols
  * the int32-X kernel. */
 int perm_exact_dense_ex(perm_ctx* ctx, const void* mat, int n, int dtype, int variant, int shard, int nshards,
                         perm_result* out);
+/* perm_exact_dense_ex, walked in a row layout of the matrix itself and once
+ * (no accuracy policy), where perm_exact_dense_ex may walk column cubes or, for
+ * the certified kernels, the transpose.  Its shards complete a walk that was
+ * begun in rows, and its whole walks are a second evaluation by other kernels
+ * in another order of the terms. */
+int perm_exact_dense_rows(perm_ctx* ctx, const void* mat, int n, int dtype, int variant, int shard, int nshards,
+                          perm_result* out);
 /* Whole-walk dense results carry rel_error_estimate, a worst-case bound
  * formed from sum |term|, estimated by a sample of Ryser terms stratified by
  * subset size (exact for the split-X and the certified kernels, whose walks

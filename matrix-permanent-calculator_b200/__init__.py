@@ -43,7 +43,7 @@ MAX_MC_SPARSE_N = 2047
 EXPORTED_SYMBOLS = (
     "perm_version", "perm_device_count", "perm_ctx_create", "perm_ctx_destroy", "perm_ctx_last_error",
     "perm_status_string", "perm_exact_dense", "perm_exact_dense_shard", "perm_shard_range", "perm_exact_dense_multi",
-    "perm_exact_dense_ex",
+    "perm_exact_dense_ex", "perm_exact_dense_rows",
     "perm_exact_sparse", "perm_exact_sparse_ex", "perm_matrix_create_dense", "perm_matrix_create_dense_ex", "perm_matrix_destroy",
     "perm_exact_dense_resident", "perm_exact_dense_resident_shard", "perm_exact_dense_refine", "perm_sdd_layout", "perm_sdd_levels", "perm_fp64_layout", "perm_fp64_levels", "perm_int_layout", "perm_intc_layout", "perm_exact_dense_plan", "perm_exact_dense_tc_rounds", "perm_exact_dense_noalloc", "perm_dense_autotune", "perm_ctx_set_rel_target", "perm_ctx_inject_wait_timeout",
     "perm_batch_create", "perm_batch_run", "perm_batch_run_ex", "perm_batch_destroy", "perm_batch_exact", "perm_batch_autotune", "perm_batch_variant", "perm_batch_use_variant",
@@ -122,6 +122,7 @@ def load_library(path: str | os.PathLike | None = None) -> ctypes.CDLL:
         "perm_exact_dense": (i, [_P, _P, i, i, ctypes.POINTER(PermResult)]),
         "perm_exact_dense_shard": (i, [_P, _P, i, i, i, i, ctypes.POINTER(PermResult)]),
         "perm_exact_dense_ex": (i, [_P, _P, i, i, i, i, i, ctypes.POINTER(PermResult)]),
+        "perm_exact_dense_rows": (i, [_P, _P, i, i, i, i, i, ctypes.POINTER(PermResult)]),
         "perm_shard_range": (i, [i, i, i, ctypes.POINTER(u64), ctypes.POINTER(u64)]),
         "perm_exact_dense_multi": (i, [_P, i, i, i, i, _P, ctypes.POINTER(PermResult)]),
         "perm_sdd_layout": (i, [_P, i]),
@@ -305,6 +306,15 @@ class Engine:
         r = PermResult()
         self._check(self.lib.perm_exact_dense_ex(self.ctx, _ptr(a), a.shape[0], dt, variant, shard, nshards,
                                                  ctypes.byref(r)))
+        return _exact(r)
+
+    def exact_dense_rows(self, mat, shard: int = 0, nshards: int = 1, variant: int = 0) -> ExactResult:
+        """exact_dense_shard walked in a row layout, never in column cubes
+        (perm_exact_dense_rows); no accuracy policy."""
+        a, dt = _as_matrix(mat)
+        r = PermResult()
+        self._check(self.lib.perm_exact_dense_rows(self.ctx, _ptr(a), a.shape[0], dt, variant, shard, nshards,
+                                                   ctypes.byref(r)))
         return _exact(r)
 
     def exact_sparse(self, n: int, rptrs, cols, rvals, cptrs, rows, cvals, variant: int = 0) -> ExactResult:
@@ -807,14 +817,20 @@ def distributed_exact_dense_dynamic(mat, chunks: int | None = None, group=None, 
     return dd_sum((float(table[c, 1]), float(table[c, 2])) for c in range(chunks))
 
 
+# The sums of shards add up only if all were walked in one layout, so a file
+# names the walk it belongs to: row layouts; from order 25 column cubes; and
+# those with the transpose taken by the sizes of rows and columns (certified
+# variants; in files of the format before, only by cost).
 CHECKPOINT_FORMAT = "perm_b200_checkpoint_v1"
-# from order 25 a shard's terms are those of the column-cube layout, so sums of
-# an earlier library's shards cannot be completed by this one's
 CHECKPOINT_FORMAT_CUBE = "perm_b200_checkpoint_v2"
+CHECKPOINT_FORMAT_SIDE = "perm_b200_checkpoint_v3"
 
 
-def _checkpoint_format(n: int) -> str:
-    return CHECKPOINT_FORMAT_CUBE if n >= 25 else CHECKPOINT_FORMAT
+def _checkpoint_format(n: int, variant: int) -> str:
+    if n < 25:
+        return CHECKPOINT_FORMAT
+    return CHECKPOINT_FORMAT_SIDE if variant in (PERM_KERNEL_DENSE_INT_DD, PERM_KERNEL_DENSE_SDD) else \
+        CHECKPOINT_FORMAT_CUBE
 
 
 def _fingerprint(a: np.ndarray) -> str:
@@ -826,17 +842,21 @@ def _fingerprint(a: np.ndarray) -> str:
     return h.hexdigest()
 
 
-def _read_checkpoint(path, fingerprint: str, n: int, chunks: int, variant: int) -> dict[int, tuple[float, float]]:
+def _read_checkpoint(path, fingerprint: str, n: int, chunks: int, variant: int,
+                     rows_too: bool = False) -> tuple[str, dict[int, tuple[float, float]]]:
+    """Format and finished shards of the file; `rows_too`: a walk in rows can
+    be completed whatever the order."""
     import json
 
     try:
         with open(path) as f:
             state = json.load(f)
     except FileNotFoundError:
-        return {}
+        return _checkpoint_format(n, variant), {}
     except (OSError, ValueError) as e:
         raise PermError(PERM_EIO, f"checkpoint {path} is unreadable ({e}); remove it to start over") from e
-    want = {"format": _checkpoint_format(n), "matrix_sha256": fingerprint, "n": n, "chunks": chunks,
+    fmt = CHECKPOINT_FORMAT if rows_too and state.get("format") == CHECKPOINT_FORMAT else _checkpoint_format(n, variant)
+    want = {"format": fmt, "matrix_sha256": fingerprint, "n": n, "chunks": chunks,
             "variant": variant}
     for k, v in want.items():
         if state.get(k) != v:
@@ -851,14 +871,14 @@ def _read_checkpoint(path, fingerprint: str, n: int, chunks: int, variant: int) 
             done[c] = (float.fromhex(h), float.fromhex(l))
     except (AttributeError, TypeError, ValueError) as e:
         raise PermError(PERM_EIO, f"checkpoint {path} is unreadable ({e}); remove it to start over") from e
-    return done
+    return fmt, done
 
 
-def _write_checkpoint(path, fingerprint: str, n: int, chunks: int, variant: int,
+def _write_checkpoint(path, fmt: str, fingerprint: str, n: int, chunks: int, variant: int,
                       done: dict[int, tuple[float, float]]) -> None:
     import json
 
-    state = {"format": _checkpoint_format(n), "matrix_sha256": fingerprint, "n": n, "chunks": chunks,
+    state = {"format": fmt, "matrix_sha256": fingerprint, "n": n, "chunks": chunks,
              "variant": variant,
              "done": {str(c): [h.hex(), l.hex()] for c, (h, l) in sorted(done.items())}}
     tmp = f"{path}.tmp"
@@ -885,7 +905,8 @@ def checkpointed_exact_dense(mat, path, chunks: int = 64, variant: int = 0, engi
     file lacks.  The shards are added in chunk order in double-double, so an
     interrupted and resumed run returns the uninterrupted run's value bit
     for bit.  A file written for another matrix, chunk count or variant is
-    refused (PermError) instead of being mixed in.  The file is removed
+    refused (PermError) instead of being mixed in; one begun in row layouts
+    by a library that had no column cubes is completed in them.  The file is removed
     after success unless `keep`.  One process at a time per file: two runs
     sharing a path would overwrite each other's progress.  One evaluation, like the shard API: pass
     the sum to Engine.refine_dense for the accuracy policy.  `shard_fn(mat,
@@ -898,18 +919,19 @@ def checkpointed_exact_dense(mat, path, chunks: int = 64, variant: int = 0, engi
     if not 1 <= chunks <= (1 << 20):
         raise PermError(PERM_EINVAL, f"chunks must be in [1, 2^20], got {chunks}")
     fp = _fingerprint(a)
-    done = _read_checkpoint(path, fp, n, chunks, variant)
+    fmt, done = _read_checkpoint(path, fp, n, chunks, variant, rows_too=shard_fn is None)
     eng = None if shard_fn is not None else (engine or default_engine())
     for c in range(chunks):
         if c in done:
             continue
         if shard_fn is None:
-            r = eng.exact_dense_shard(a, c, chunks, variant=variant)
+            in_rows = n >= 25 and fmt == CHECKPOINT_FORMAT
+            r = (eng.exact_dense_rows if in_rows else eng.exact_dense_shard)(a, c, chunks, variant=variant)
             done[c] = (r.hi, r.lo)
         else:
             hi, lo = shard_fn(a, c, chunks)
             done[c] = (float(hi), float(lo))
-        _write_checkpoint(path, fp, n, chunks, variant, done)
+        _write_checkpoint(path, fmt, fp, n, chunks, variant, done)
     result = dd_sum(done[c] for c in range(chunks))
     if not keep:
         try:

@@ -1589,9 +1589,10 @@ static std::vector<double> transposed(const std::vector<double>& a, int n) {
   return t;
 }
 
-static int build_sdd_operand(perm_ctx* ctx, std::vector<double> a, int n, DenseOperand* op) {
+static int build_sdd_operand(perm_ctx* ctx, std::vector<double> a, int n, bool rows_only, DenseOperand* op) {
   if (n < 4 || n > 40) return fail(ctx, PERM_EUNSUPPORTED, "split-dd kernel covers orders 4..40 (got %d)", n);
-  WalkSide side = n >= kCubeMinN ? walk_side(a, n) : WalkSide::kMatrix;
+  const bool cubes = n >= kCubeMinN && !rows_only;
+  WalkSide side = cubes ? walk_side(a, n) : WalkSide::kMatrix;
   if (side != WalkSide::kMatrix) {
     // the callers checked the matrix's rows, not the transpose's
     std::vector<double> t = transposed(a, n);
@@ -1610,7 +1611,7 @@ static int build_sdd_operand(perm_ctx* ctx, std::vector<double> a, int n, DenseO
   CubeLayout l;
   int inner = 0, inner1 = 0;
   std::vector<double> perm;
-  bool cube = n >= kCubeMinN && cube_layout(a, n, 1e9, side == WalkSide::kEither, &l);
+  bool cube = cubes && cube_layout(a, n, 1e9, side == WalkSide::kEither, &l);
   bool searched = false;
   if (cube) {
     const double mine = (6.0 * cube_values(kCubeShapes[l.shape]) + 2.0 * n + 280.0) / 0.63;
@@ -1643,16 +1644,17 @@ static bool sparse_enough(const std::vector<double>& a) {
   return nonzeros <= a.size() * 8 / 10;
 }
 
-// `own_sum`: the operand is walked in one piece under the accuracy policy.
+// `own_sum`: the operand is walked in one piece under the accuracy policy;
+// `rows_only`: a row layout of the matrix itself, no cubes and no transpose.
 static int build_operand(perm_ctx* ctx, const void* mat, int n, int dtype, int variant, DenseOperand* op,
-                         bool own_sum = false) {
+                         bool own_sum = false, bool rows_only = false) {
   std::vector<double> a((size_t)n * n);
   for (size_t i = 0; i < a.size(); i++) a[i] = elem(mat, dtype, i);
   op->n = n;
   const int pref = variant == 0 && n <= PERM_MAX_EXACT_N ? ctx->dense_pref[n] : 0;
   const bool prefer_fp64 = pref == PERM_KERNEL_DENSE;
   if (variant == PERM_KERNEL_DENSE_SPLIT) return build_split_operand(ctx, a, n, op);
-  if (variant == PERM_KERNEL_DENSE_SDD) return build_sdd_operand(ctx, a, n, op);
+  if (variant == PERM_KERNEL_DENSE_SDD) return build_sdd_operand(ctx, a, n, rows_only, op);
   int G = (variant == PERM_KERNEL_DENSE || variant == PERM_KERNEL_DENSE_DD || prefer_fp64) ? 0 : int_group_size(a, n);
   if ((variant == PERM_KERNEL_DENSE_INT || variant == PERM_KERNEL_DENSE_INT_DD) && G == 0)
     return fail(ctx, PERM_EUNSUPPORTED,
@@ -1675,7 +1677,8 @@ static int build_operand(perm_ctx* ctx, const void* mat, int n, int dtype, int v
     if (op->variant != PERM_KERNEL_DENSE_TC) {
       IntRows rows;
       // the transpose's search costs more than it saves below order 28
-      const WalkSide side = op->variant == PERM_KERNEL_DENSE_INT_DD && n >= 28 ? walk_side(a, n) : WalkSide::kMatrix;
+      const bool turn = op->variant == PERM_KERNEL_DENSE_INT_DD && n >= 28 && !rows_only;
+      const WalkSide side = turn ? walk_side(a, n) : WalkSide::kMatrix;
       if (side == WalkSide::kTranspose) {
         std::vector<double> t = transposed(a, n);
         if (const int g = int_group_size(t, n)) {
@@ -1683,7 +1686,8 @@ static int build_operand(perm_ctx* ctx, const void* mat, int n, int dtype, int v
           a.swap(t);
         }
       }
-      if (n >= kCubeMinN && cube_operand_int(a, n, G, side == WalkSide::kEither, &rows, op)) return PERM_OK;
+      if (n >= kCubeMinN && !rows_only && cube_operand_int(a, n, G, side == WalkSide::kEither, &rows, op))
+        return PERM_OK;
       rows.choose(a, n, G, op->variant == PERM_KERNEL_DENSE_INT_DD);
       op->group = rows.group;
       op->pair = rows.pair;
@@ -1709,7 +1713,8 @@ static int build_operand(perm_ctx* ctx, const void* mat, int n, int dtype, int v
     op->inner1 = 0;
     if (op->variant == PERM_KERNEL_DENSE) {
       Fp64Rows rows;
-      if (n >= (own_sum && sparse_enough(a) ? kCubeSumMinN : kCubeMinN) && cube_operand_f64(a, n, &rows, op))
+      if (!rows_only && n >= (own_sum && sparse_enough(a) ? kCubeSumMinN : kCubeMinN) &&
+          cube_operand_f64(a, n, &rows, op))
         return PERM_OK;
       rows.choose(a, n);
       op->inner = rows.inner;
@@ -2564,8 +2569,9 @@ extern "C" int perm_exact_dense_plan(perm_ctx* ctx, const void* mat, int n, int 
   return policy_plan(ctx, mat, n, dtype, kernel, fp64_bound);
 }
 
-extern "C" int perm_exact_dense_ex(perm_ctx* ctx, const void* mat, int n, int dtype, int variant, int shard,
-                                   int nshards, perm_result* out) {
+// `rows_only`: walked in a row layout, once (no policy).
+static int exact_dense_call(perm_ctx* ctx, const void* mat, int n, int dtype, int variant, int shard, int nshards,
+                            bool rows_only, perm_result* out) {
   int rc = check_dense_args(ctx, mat, n, dtype, out);
   if (rc) return rc;
   if ((rc = check_variant(ctx, variant))) return rc;
@@ -2573,10 +2579,9 @@ extern "C" int perm_exact_dense_ex(perm_ctx* ctx, const void* mat, int n, int dt
     return fail(ctx, PERM_EINVAL, "shard %d of %d", shard, nshards);
   DenseOperand op;
   int first = 0;
-  if (variant == 0 && nshards == 1 && ctx->rel_target > 0 && (rc = policy_plan(ctx, mat, n, dtype, &first)))
-    return rc;
-  if ((rc = build_operand(ctx, mat, n, dtype, first ? first : variant, &op,
-                          nshards == 1 && variant == 0 && ctx->rel_target > 0))) return rc;
+  const bool policed = variant == 0 && nshards == 1 && ctx->rel_target > 0 && !rows_only;
+  if (policed && (rc = policy_plan(ctx, mat, n, dtype, &first))) return rc;
+  if ((rc = build_operand(ctx, mat, n, dtype, first ? first : variant, &op, policed, rows_only))) return rc;
   // shards are Gray-index ranges of the walking kernels; the tensor-core
   // kernel's operand image is the int32-X one
   if (nshards > 1 && op.variant == PERM_KERNEL_DENSE_TC) op.variant = PERM_KERNEL_DENSE_INT;
@@ -2594,7 +2599,7 @@ extern "C" int perm_exact_dense_ex(perm_ctx* ctx, const void* mat, int n, int dt
   // the same image, and the matching check runs while both do: one wait and
   // one copy back for all of it (n = 12, real: 55 us a call, 77 with a copy, a
   // second image and a wait of its own for the sample).
-  const bool policy = refine && variant == 0 && ctx->rel_target > 0;
+  const bool policy = refine && policed;
   const bool sampled = refine && n >= 2 && plain_columns(op);
   if (sampled && (rc = queue_moments(ctx, ctx->d_stage, n))) return rc;
   int matching = -1;
@@ -2605,6 +2610,16 @@ extern "C" int perm_exact_dense_ex(perm_ctx* ctx, const void* mat, int n, int dt
   out->abs_term_sum = out->rel_error_estimate = 0;
   if (!refine) return PERM_OK;
   return refine_result(ctx, mat, n, dtype, op, policy, out, matching, sampled);
+}
+
+extern "C" int perm_exact_dense_ex(perm_ctx* ctx, const void* mat, int n, int dtype, int variant, int shard,
+                                   int nshards, perm_result* out) {
+  return exact_dense_call(ctx, mat, n, dtype, variant, shard, nshards, false, out);
+}
+
+extern "C" int perm_exact_dense_rows(perm_ctx* ctx, const void* mat, int n, int dtype, int variant, int shard,
+                                     int nshards, perm_result* out) {
+  return exact_dense_call(ctx, mat, n, dtype, variant, shard, nshards, true, out);
 }
 
 extern "C" int perm_exact_dense_refine(perm_ctx* ctx, const void* mat, int n, int dtype, perm_result* io) {
