@@ -70,6 +70,12 @@ struct Acc {
     hi = s.hi;
     lo = __dadd_rn(lo, s.lo);
   }
+  // adds v times sign (+1 or -1) in as many operations
+  __device__ __forceinline__ void add(double v, double sign) {
+    const double s = __fma_rn(sign, v, hi), bb = __dsub_rn(s, hi);
+    lo = __dadd_rn(lo, __dadd_rn(__dsub_rn(hi, __dsub_rn(s, bb)), __fma_rn(sign, v, -bb)));
+    hi = s;
+  }
   __device__ __forceinline__ dd value() const { return fast_two_sum_safe(); }
   __device__ __forceinline__ dd fast_two_sum_safe() const { return two_sum(hi, lo); }
 };

@@ -347,27 +347,38 @@ __device__ __forceinline__ void cube_sum_dd(const CubeArray<15, Num>& top, const
   sum2_add(H, L, odd ? -t[0].hi : t[0].hi, odd ? -t[0].lo : t[0].lo);
 }
 
-// The signed sum of the 16 terms top x third x last: over column 2's sign
-// first, then column 0's, then the other two.  Neighbouring terms mostly
-// cancel, so what is rounded stays small, and the differences of products are
-// fused (one rounding less per term; errors over integer matrices then match
-// those of the row layouts).
-// kAbs: their absolute values are added to m1.
-template <bool kThird, bool kAbs>
-__device__ __forceinline__ double cube_sum_f64(const CubeArray<15, CubeF64>& top, const CubeArray<13, CubeF64>& third,
-                                               const CubeArray<11, CubeF64>& last, double& m1) {
+// Adds the 16 signed terms top x third x last to acc: over column 2's sign
+// first, then column 0's, then the other two, as one sum or (kTwo) as two.
+//
+// What the error comes from are the roundings of the largest terms, which for
+// matrices without negative entries are those of plus signs alone.  So every
+// difference of products is fused on the side of the plus sign, and only the
+// minus side's product is rounded by itself; integer walks, whose row layouts
+// round less than those of FP64 x, add two sums.  Errors then are no larger than
+// the row layouts' (rms in units of 2^-53 sum |term|, orders 25..28: values
+// 1..4, 600 matrices each, 0.074/0.064/0.061/0.058 against
+// 0.082/0.076/0.068/0.070; FP32 values, 360 matrices each,
+// 0.154/0.124/0.125/0.120 against 0.177/0.162/0.144/0.125).  With the minus sides
+// fused and one sum the integers' were above them (0.088/0.084/0.076/0.069), and
+// with one sum now they are 4% larger than with two, in 1% less time; four sums
+// are 5% below two, in 3% more time.  The sign as a factor of fused additions
+// pays for the second sum: selected, one sum takes as long (n = 30..37).
+// kAbs: the terms' absolute values are added to m1.
+template <bool kThird, bool kAbs, bool kTwo>
+__device__ __forceinline__ void cube_add_f64(const CubeArray<15, CubeF64>& top, const CubeArray<13, CubeF64>& third,
+                                             const CubeArray<11, CubeF64>& last, bool odd, Acc& acc, double& m1) {
   double d[8];
 #pragma unroll
   for (int s = 0; s < 8; s++) {
     const int t0 = (s & 3) | ((s & 4) << 1), t1 = t0 | 4;  // column 2 minus, plus
     if constexpr (kThird) {
       const int a0 = (s & 1) | (s & 4), a1 = a0 | 2;
-      const double p = __dmul_rn(top.v[t1].hi, third.v[a1].hi);
-      d[s] = __fma_rn(top.v[t0].hi, third.v[a0].hi, -p);
+      const double p = __dmul_rn(top.v[t0].hi, third.v[a0].hi);
+      d[s] = __fma_rn(top.v[t1].hi, third.v[a1].hi, -p);
       if constexpr (kAbs)
-        m1 = __fma_rn(fabs(last.v[s].hi), __fma_rn(fabs(top.v[t0].hi), fabs(third.v[a0].hi), fabs(p)), m1);
+        m1 = __fma_rn(fabs(last.v[s].hi), __fma_rn(fabs(top.v[t1].hi), fabs(third.v[a1].hi), fabs(p)), m1);
     } else {
-      d[s] = __dsub_rn(top.v[t0].hi, top.v[t1].hi);
+      d[s] = __dsub_rn(top.v[t1].hi, top.v[t0].hi);
       if constexpr (kAbs)
         m1 = __fma_rn(fabs(last.v[s].hi), __dadd_rn(fabs(top.v[t0].hi), fabs(top.v[t1].hi)), m1);
     }
@@ -375,10 +386,17 @@ __device__ __forceinline__ double cube_sum_f64(const CubeArray<15, CubeF64>& top
   double t[4];
 #pragma unroll
   for (int q = 0; q < 4; q++) {
-    const int s = 2 * q + (__popc(q) & 1), r = s ^ 1;  // plus term, minus term
-    t[q] = __fma_rn(last.v[s].hi, d[s], -__dmul_rn(last.v[r].hi, d[r]));
+    const int s = 2 * q;
+    t[q] = __fma_rn(last.v[s + 1].hi, d[s + 1], -__dmul_rn(last.v[s].hi, d[s]));
   }
-  return __dadd_rn(__dadd_rn(t[0], t[1]), __dadd_rn(t[2], t[3]));
+  // terms with an even number of minus signs among the four columns count plus
+  const double sign = odd ? -1.0 : 1.0, large = __dsub_rn(t[3], t[2]), small = __dsub_rn(t[0], t[1]);
+  if constexpr (kTwo) {
+    acc.add(large, sign);
+    acc.add(small, sign);
+  } else {
+    acc.add(__dadd_rn(large, small), sign);
+  }
 }
 
 // Range of outer Gray indices of this thread, and the loop over it:
@@ -461,8 +479,7 @@ __global__ void __launch_bounds__(kCubeThreads, 1) ryser_cube_kernel(const __gri
           CubeArray<13, CubeF64> third;
           CubeArray<11, CubeF64> last;
           cube.products(top, third, last);
-          const double t = cube_sum_f64<(decltype(cube)::kThird > 0), kAbs>(top, third, last, m1);
-          acc.add((h & 1) ? -t : t);
+          cube_add_f64<(decltype(cube)::kThird > 0), kAbs, false>(top, third, last, (h & 1) != 0, acc, m1);
         });
   }
   cube_finish(a, acc.value(), kAbs, m1, (a.n & 1) ? 2.0 : -2.0, red);
@@ -595,8 +612,7 @@ __global__ void __launch_bounds__(kCubeThreads, 1) ryser_cube_int_kernel(const _
             cube_sum_dd<C::kFirst + C::kSecond + C::kThird <= kCubeExactRows, C::kLast <= kCubeExactRows>(
                 top, last, (h & 1) != 0, H, L, m1);
           } else {
-            const double t = cube_sum_f64<(C::kThird > 0), kAbs>(top, third, last, m1);
-            acc.add((h & 1) ? -t : t);
+            cube_add_f64<(C::kThird > 0), kAbs, true>(top, third, last, (h & 1) != 0, acc, m1);
           }
         });
   }

@@ -130,3 +130,30 @@ def test_checkpoint_begun_in_rows_on_the_gpu(pb, engine, tmp_path):
         want = engine.exact_dense(A)
         bound = engine.exact_dense_rows(A, variant=variant or pb.PERM_KERNEL_DENSE).rel_error_estimate
         assert abs(hi + lo - want.value) <= (bound + want.rel_error_estimate + 2 * U) * abs(want.value)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,top,variant", [(25, 4, "PERM_KERNEL_DENSE_INT"), (27, 4, "PERM_KERNEL_DENSE_INT"),
+                                           (28, 4, "PERM_KERNEL_DENSE_INT"), (25, 0, "PERM_KERNEL_DENSE")])
+def test_cubes_are_as_exact_as_rows(engine, pb, n, top, variant):
+    """Errors of one plain walk against the certified value, in units of
+    sum |term|: over 300 matrices the cubes' rms is no larger than the row
+    layouts' (top 0: FP32 values, whose x are exact too)."""
+    variant = getattr(pb, variant)
+    certified = pb.PERM_KERNEL_DENSE_INT_DD if top else pb.PERM_KERNEL_DENSE_SDD
+    square = np.zeros(2)
+    engine.set_rel_target(0.0)
+    try:
+        for d in (0.35, 0.5, 0.7):
+            for seed in range(100):
+                rng = np.random.default_rng([n, seed, 77])
+                mask = (rng.random((n, n)) < d) | (np.eye(n)[rng.permutation(n)] > 0)
+                A = mask * (rng.integers(1, top + 1, (n, n)) if top else np.float32(1.0 - rng.random((n, n))))
+                A = A.astype(np.float64)
+                c = engine.exact_dense(A, variant=certified)
+                for k, r in enumerate((engine.exact_dense_shard(A, 0, 1, variant=variant),
+                                       engine.exact_dense_rows(A, variant=variant))):
+                    square[k] += (((r.hi - c.hi) + (r.lo - c.lo)) / (U * c.abs_term_sum)) ** 2
+    finally:
+        engine.set_rel_target(1e-10)
+    assert square[0] <= square[1], np.sqrt(square / 300)
