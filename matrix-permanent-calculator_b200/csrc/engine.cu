@@ -2355,9 +2355,10 @@ static bool has_perfect_matching(const void* mat, int n, int dtype) {
 // its bound uses the exact sum |term| the walk accumulated.
 // Context lock held.
 // `matching`: whether the pattern has a perfect matching (-1: not known yet);
-// `sampled`: the term moments of `op`'s matrix are in the result block already.
+// `sampled`: the term moments of `op`'s matrix are in the result block already;
+// `term_sum`: the walk's own sum |term|, where the caller has it (0: not).
 static int refine_result(perm_ctx* ctx, const void* mat, int n, int dtype, const DenseOperand& op, bool policy,
-                         perm_result* out, int matching = -1, bool sampled = false) {
+                         perm_result* out, int matching = -1, bool sampled = false, double term_sum = 0.0) {
   int rc;
   if (policy && (matching < 0 ? !has_perfect_matching(mat, n, dtype) : !matching)) {
     out->value = out->hi = out->lo = 0.0;
@@ -2382,7 +2383,7 @@ static int refine_result(perm_ctx* ctx, const void* mat, int n, int dtype, const
     out->rel_error_estimate = e.worst;
     if (!policy || e.worst <= ctx->rel_target) return PERM_OK;
   }
-  const double walked = e.s1;
+  const double walked = term_sum > 0.0 ? term_sum : e.s1;
   if (sampled) {
     estimate_from_moments(ctx, n, op, out->value, &e);
   } else {
@@ -3267,6 +3268,7 @@ struct perm_batch {
   std::vector<double> abs_scale;  // per matrix: factor of its sum |term|
   std::vector<std::pair<int, int>> exp2;  // matrices whose three results are multiplied by 2^second
   std::vector<int> groups;       // per matrix: 0 = FP64 X, else the int32-X group size
+  std::vector<int> shapes;       // per matrix: of its column-cube walk, -1: row layout
   std::vector<int> orders;       // host copies for double-double reruns
   std::vector<uint64_t> offsets;
   std::vector<double> values;
@@ -3491,6 +3493,7 @@ static int batch_create_locked(perm_ctx* ctx, int count, const int* orders, cons
   const BatchVariant& V = kBatchVariants[vi];
   b->orders.assign(orders, orders + count);
   b->groups.resize(count);
+  b->shapes.assign(count, -1);
   b->roundings.resize(count);
   b->abs_scale.assign(count, 1.0);
   for (int i = 0; i < count; i++) {
@@ -3500,6 +3503,7 @@ static int batch_create_locked(perm_ctx* ctx, int count, const int* orders, cons
   for (const BatchCube& c : cube) {
     // |factor| = 2, of prod y = 2^n prod x in the int32 walk
     b->abs_scale[c.index] = c.op.variant == PERM_KERNEL_DENSE_INT ? std::ldexp(1.0, 1 - c.op.n) : 2.0;
+    b->shapes[c.index] = c.op.shape;
     if (c.op.exp2) b->exp2.push_back({c.index, c.op.exp2});
     if (c.op.variant == PERM_KERNEL_DENSE_INT) b->roundings[c.index] = cube_factors(kCubeShapes[c.op.shape]) + 1.0;
   }
@@ -3677,15 +3681,21 @@ extern "C" int perm_batch_run_ex(perm_ctx* ctx, perm_batch* b, double* results, 
     if (ctx->rel_target > 0 && est > ctx->rel_target && n >= 2) {
       const double* mat = b->values.data() + b->offsets[i];
       const int kernel = G ? PERM_KERNEL_DENSE_INT : PERM_KERNEL_DENSE;
+      // the walk that made the value, whose bound this is; its columns as they
+      // are, for the sample of the term moments
       DenseOperand op;
-      if ((rc = build_operand(ctx, mat, n, PERM_F64, kernel, &op))) return rc;
+      op.n = n;
+      op.variant = kernel;
+      op.group = G;
+      op.shape = b->shapes[i];
+      if (plain_columns(op)) build_fp64_image(std::vector<double>(mat, mat + (size_t)n * n), n, &op);
       perm_result r{};
       r.hi = b->h_results[3 * i];
       r.lo = b->h_results[3 * i + 1];
       r.value = v;
       r.n = n;
       r.kernel = kernel;
-      if ((rc = refine_result(ctx, mat, n, PERM_F64, op, true, &r))) return rc;
+      if ((rc = refine_result(ctx, mat, n, PERM_F64, op, true, &r, -1, false, sa))) return rc;
       if (results) {
         results[2 * i] = r.hi;
         results[2 * i + 1] = r.lo;
