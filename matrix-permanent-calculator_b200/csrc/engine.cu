@@ -313,7 +313,8 @@ __device__ __forceinline__ uint64_t splitmix64(uint64_t& state) {
 }
 
 __global__ void __launch_bounds__(256) ryser_abs_sample_kernel(const double* colA, int n, int np, int per_class,
-                                                                uint64_t seed, double* out) {
+                                                                uint64_t seed, dd* partials, unsigned* ticket,
+                                                                double* out) {
   __shared__ double sA[64 * 64];
   __shared__ double x0[64];
   __shared__ double red[8], red2[8];
@@ -384,14 +385,35 @@ __global__ void __launch_bounds__(256) ryser_abs_sample_kernel(const double* col
     red2[threadIdx.x >> 5] = local2;
   }
   __syncthreads();
+  // block sums in block order by the block that finishes last: the same every
+  // time, and the ticket ends at 0
+  __shared__ bool is_last;
   if (threadIdx.x == 0) {
     double t = 0.0, t2 = 0.0;
     for (int w = 0; w < (int)(blockDim.x >> 5); w++) {
       t += red[w];
       t2 += red2[w];
     }
-    atomicAdd(out, t);
-    atomicAdd(out + 1, t2);
+    partials[blockIdx.x] = {t, t2};
+    __threadfence();
+    is_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!is_last || threadIdx.x >= 32) return;
+  __threadfence();
+  local = local2 = 0.0;
+  for (unsigned b = threadIdx.x; b < gridDim.x; b += 32) {
+    local += __ldcg(&partials[b].hi);
+    local2 += __ldcg(&partials[b].lo);
+  }
+  for (int d = 16; d >= 1; d >>= 1) {
+    local += __shfl_down_sync(0xffffffffu, local, d);
+    local2 += __shfl_down_sync(0xffffffffu, local2, d);
+  }
+  if (threadIdx.x == 0) {
+    out[0] = local;
+    out[1] = local2;
+    *ticket = 0u;
   }
 }
 
@@ -2022,8 +2044,6 @@ static int dense_launch(perm_ctx* ctx, const DenseOperand& op, const void* d_ima
       ctx->inject_timeouts--;
     }
     void* kargs[] = {&u};
-    if (kind == kCubeSdd || kind == kCubeIntc || kind == kCubeF64Abs)
-      CU(ctx, cudaMemsetAsync(ctx->d_est, 0, 2 * sizeof(double), ctx->stream));
     CU(ctx, cudaLaunchKernel(operand_kernel(op), dim3(p.grid), dim3(operand_threads(op)), kargs, operand_smem(op),
                              ctx->stream));
   } else if (op.variant == PERM_KERNEL_DENSE_TC) {
@@ -2256,9 +2276,9 @@ static int queue_moments(perm_ctx* ctx, const void* d_col_fp64, int n) {
   const int np = (n + 1) & ~1;
   const int per_class = kSamplesPerClass;
   const uint64_t threads = (uint64_t)n * per_class;  // classes |S| = 0 .. n-1
-  CU(ctx, cudaMemsetAsync(ctx->d_est, 0, 2 * sizeof(double), ctx->stream));
   ryser_abs_sample_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, ctx->stream>>>(
-      static_cast<const double*>(d_col_fp64), n, np, per_class, 0x243F6A8885A308D3ull, ctx->d_est);
+      static_cast<const double*>(d_col_fp64), n, np, per_class, 0x243F6A8885A308D3ull, ctx->partials, ctx->ticket,
+      ctx->d_est);
   CU(ctx, cudaGetLastError());
   return PERM_OK;
 }
@@ -2523,9 +2543,10 @@ static int policy_predicts_sdd(perm_ctx* ctx, const void* mat, int n, int dtype,
   if ((rc = stage_operand(ctx, f))) return rc;
   const int np = (n + 1) & ~1;
   const uint64_t threads = (uint64_t)n * kSamplesPerClass;
-  CU(ctx, cudaMemsetAsync(ctx->d_est, 0, 4 * sizeof(double), ctx->stream));
+  CU(ctx, cudaMemsetAsync(ctx->d_est + 2, 0, 2 * sizeof(double), ctx->stream));
   ryser_abs_sample_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, ctx->stream>>>(
-      reinterpret_cast<const double*>(ctx->d_stage), n, np, kSamplesPerClass, 0x243F6A8885A308D3ull, ctx->d_est);
+      reinterpret_cast<const double*>(ctx->d_stage), n, np, kSamplesPerClass, 0x243F6A8885A308D3ull, ctx->partials,
+      ctx->ticket, ctx->d_est);
   CU(ctx, cudaGetLastError());
   weighted_rasmussen_kernel<<<(kPredictTrials + 255) / 256, 256, 0, ctx->stream>>>(
       reinterpret_cast<const double*>(ctx->d_stage), n, np, kPredictTrials, 0x13198A2E03707344ull, log2_ub,
@@ -3558,7 +3579,7 @@ static int batch_create_locked(perm_ctx* ctx, int count, const int* orders, cons
   const uint64_t warps = (uint64_t)ctx->num_sms * ctx->batch_occ[vi] * wpb;
   const uint64_t want = std::min<uint64_t>(warps, tiles);
   b->grid = (int)std::max<uint64_t>(1, (want + wpb - 1) / wpb);
-  // capture: reset the queue head and the results, run, read the results back.
+  // capture: reset the queue head and the error flag, run, read the results back.
   // The column-cube walks are dealt to parallel branches beside the persistent
   // kernel's: the next walk's CTAs fill the SMs that one leaves.
   BatchArgs args;
@@ -3591,10 +3612,10 @@ static int batch_create_locked(perm_ctx* ctx, int count, const int* orders, cons
   }
   BT(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
   cudaMemsetAsync(b->d_next, 0, sizeof(unsigned long long), ctx->stream);
-  // only the column-cube walks add to their results (a node of the graph takes
-  // 10 us: 350 us for 130 matrices of orders 15..21)
+  // only the column-cube walks set the error flag (a node of the graph takes 10
+  // us: 350 us for 130 matrices of orders 15..21)
   if (branches) {
-    cudaMemsetAsync(b->d_results, 0, result_bytes, ctx->stream);
+    cudaMemsetAsync(b->d_results + 3 * (size_t)count, 0, sizeof(double), ctx->stream);
     cudaEventRecord(br.fork, ctx->stream);
   }
   for (int i = 0; i < branches; i++) cudaStreamWaitEvent(br.stream[i], br.fork, 0);

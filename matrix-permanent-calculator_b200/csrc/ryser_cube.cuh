@@ -423,18 +423,34 @@ __device__ __forceinline__ void cube_walk(const CubeWalk& a, Start start, Flip f
   }
 }
 
-// Sum of m1 over the grid to *sums, and the thread totals to *out.
+// The thread totals' sum to *out and, with abs_sum, that of m1 to *sums; both in
+// a fixed order, so that a walk's error estimate is the same every time.  A
+// block's m1 stands behind the blocks' totals in `partials`.
 __device__ __forceinline__ void cube_finish(const CubeWalk& a, dd total, bool abs_sum, double m1, double factor, dd* red) {
+  constexpr int kWarps = kCubeThreads / 32;
+  static_assert(2 * kWarps <= 32, "red holds the warps' totals and their m1");
+  const int lane = threadIdx.x & 31;
   if (abs_sum) {
 #pragma unroll
     for (int d = 16; d >= 1; d >>= 1) m1 += __shfl_down_sync(0xffffffffu, m1, d);
-    if ((threadIdx.x & 31) == 0 && m1 > 0.0) atomicAdd(a.sums, m1);
+    if (lane == 0) red[kWarps + (threadIdx.x >> 5)].hi = m1;
   }
-  const dd bt = block_reduce_dd(total, red);
-  grid_finish_dd(bt, a.partials, a.ticket, a.out, factor, red);
+  const dd bt = block_reduce_dd(total, red);  // red is written before its barrier
+  if (abs_sum && threadIdx.x == 0) {
+    double s = 0.0;
+    for (int w = 0; w < kWarps; w++) s += red[kWarps + w].hi;
+    a.partials[gridDim.x + blockIdx.x].hi = s;
+  }
+  const bool last = grid_finish_dd(bt, a.partials, a.ticket, a.out, factor, red);
+  if (!abs_sum || !last || threadIdx.x >= 32) return;
+  double s = 0.0;
+  for (unsigned b = lane; b < gridDim.x; b += 32) s += __ldcg(&a.partials[gridDim.x + b].hi);
+#pragma unroll
+  for (int d = 16; d >= 1; d >>= 1) s += __shfl_down_sync(0xffffffffu, s, d);
+  if (lane == 0) *a.sums = s;
 }
 
-// FP64 walk; kAbs: sums[0] += sum |term| as well (16 of some 250 operations).
+// FP64 walk; kAbs: *sums = sum |term| as well (16 of some 250 operations).
 template <int kShape, bool kAbs>
 __global__ void __launch_bounds__(kCubeThreads, 1) ryser_cube_kernel(const __grid_constant__ CubeArgs a) {
   constexpr int N = cube_rows(kCubeShapes[kShape]);

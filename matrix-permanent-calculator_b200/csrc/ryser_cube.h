@@ -20,10 +20,10 @@ struct CubeWalk {
   int m;                     // log2 of the range alignment, in outer Gray indices
   uint64_t block0, nblocks;  // aligned blocks of 2^m outer indices of this launch
   uint64_t seg;              // cubes between two recomputations of b
-  dd* partials;
+  dd* partials;  // two per block of the grid
   unsigned* ticket;
   double* out;
-  double* sums;  // sums[0] += sum |term| (zeroed by the host; walks that sum it)
+  double* sums;  // sum |term| (walks that sum it)
   int* err;
   uint32_t inject;  // failure injection (tests): staging expects this many extra bytes
 };

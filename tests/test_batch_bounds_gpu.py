@@ -41,3 +41,24 @@ def test_target_just_below_the_own_bound(pb, n, d, integers):
                     assert np.all(est < 1e-14), est
         finally:
             b.free()
+
+
+def test_estimates_repeat_to_the_bit(pb):
+    """Sums of |term| are added in a fixed order: the bound of a value, and
+    with it whether it is evaluated again, does not change between runs."""
+    mats = [_matrix(n, d, 5, integers) for n in (18, 22, 24, 25, 27) for d in (0.3, 0.5) for integers in (True, False)]
+    with pb.Engine(0) as eng:
+        eng.set_rel_target(0.0)
+        b = eng.batch(mats)
+        try:
+            first = b.run_ex()
+            for _ in range(20):
+                values, est, _, _ = b.run_ex()
+                assert np.array_equal(values, first[0]) and np.array_equal(est, first[1])
+        finally:
+            b.free()
+        for A in mats:
+            for variant in (0, pb.PERM_KERNEL_DENSE_SDD):
+                got = {(r.hi, r.lo, r.abs_term_sum) for r in (eng.exact_dense(A, variant=variant) for _ in range(10))
+                       if len(A) >= 25}
+                assert len(got) <= 1, (A.shape, variant, got)
