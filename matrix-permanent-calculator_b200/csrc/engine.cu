@@ -24,14 +24,15 @@
 #include <cstring>
 #include <functional>
 #include <mutex>
+#include <new>
 #include <string>
-#include <system_error>
 #include <thread>
 #include <vector>
 
 #include "../../include/perman_b200.h"
 #include "batch.h"
 #include "cube_plan.h"
+#include "host_pool.h"
 #include "matrix_io.h"
 #include "mc.h"
 #include "mc_sparse.h"
@@ -3343,27 +3344,17 @@ static void batch_cubes(int count, const int* orders, const double* values, std:
     }
     found.resize(kept);
   }
-  std::atomic<size_t> next{0};
-  auto work = [&]() {
-    for (size_t k; (k = next.fetch_add(1)) < found.size();) {
-      const int n = orders[found[k].index];
-      const std::vector<double> a(values + offset[k], values + offset[k] + (size_t)n * n);
-      const int G = int_group_size(a, n);
-      DenseOperand& op = found[k].op;
-      op.variant = G ? PERM_KERNEL_DENSE_INT : PERM_KERNEL_DENSE;
-      IntRows int_rows;
-      Fp64Rows rows;
-      if (!(G ? cube_operand_int(a, n, G, false, &int_rows, &op) : cube_operand_f64(a, n, &rows, &op))) op.shape = -1;
-    }
-  };
-  std::vector<std::thread> threads;
-  const size_t want = std::min<size_t>({found.size() / 8, std::thread::hardware_concurrency(), 8});
-  try {
-    while (threads.size() + 1 < want) threads.emplace_back(work);
-  } catch (const std::system_error&) {  // no more threads: the ones there do the work
-  }
-  work();
-  for (std::thread& t : threads) t.join();
+  const size_t threads = std::min<size_t>({found.size() / 8, std::thread::hardware_concurrency(), 8});
+  for_each_shared(found.size(), threads ? threads - 1 : 0, [&](size_t k) {
+    const int n = orders[found[k].index];
+    const std::vector<double> a(values + offset[k], values + offset[k] + (size_t)n * n);
+    const int G = int_group_size(a, n);
+    DenseOperand& op = found[k].op;
+    op.variant = G ? PERM_KERNEL_DENSE_INT : PERM_KERNEL_DENSE;
+    IntRows int_rows;
+    Fp64Rows rows;
+    if (!(G ? cube_operand_int(a, n, G, false, &int_rows, &op) : cube_operand_f64(a, n, &rows, &op))) op.shape = -1;
+  });
   for (BatchCube& c : found)
     if (c.op.shape >= 0) out->push_back(std::move(c));
 }
@@ -3378,7 +3369,11 @@ static int batch_create_locked(perm_ctx* ctx, int count, const int* orders, cons
   // Larger matrices walk in column cubes where that is cheaper.
   std::vector<BatchCube> cube;
   std::vector<int> cube_of(count, -1);
-  if (cubes) batch_cubes(count, orders, values, &cube);
+  try {
+    if (cubes) batch_cubes(count, orders, values, &cube);
+  } catch (const std::bad_alloc&) {
+    return fail(ctx, PERM_ENOMEM, "no host memory for the layouts of %d matrices", count);
+  }
   for (size_t k = 0; k < cube.size(); k++) cube_of[cube[k].index] = (int)k;
   uint64_t cube_bytes = 0;
   uint64_t off = 0, img = 0;
