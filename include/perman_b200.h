@@ -220,7 +220,8 @@ int perm_ctx_set_rel_target(perm_ctx* ctx, double rel_target);
 int perm_exact_dense_plan(perm_ctx* ctx, const void* mat, int n, int dtype, int* kernel, double* fp64_bound);
 
 /* Failure-injection hook for tests of the bounded device waits.  The next
- * `launches` launches of the FP64-X dense kernel (PERM_KERNEL_DENSE) or of
+ * `launches` launches of the FP64-X dense kernel (PERM_KERNEL_DENSE, in rows
+ * or column cubes; in a batch, launches are those it is created with) or of
  * the tensor-core kernel (PERM_KERNEL_DENSE_TC) on this context wait on a
  * barrier that never completes: the FP64-X kernel's operand staging expects
  * 16 bytes more than it copies (every copy still lands), the tensor-core

@@ -3627,6 +3627,10 @@ static int batch_create_locked(perm_ctx* ctx, int count, const int* orders, cons
     u.walk.out = b->d_results + 3 * c.index;
     u.walk.sums = b->d_results + 3 * c.index + 2;
     u.walk.err = reinterpret_cast<int*>(b->d_results + 3 * (size_t)count);
+    if (ctx->inject_timeouts > 0 && cube_kind(c.op) == kCubeF64) {
+      u.walk.inject = 16u;
+      ctx->inject_timeouts--;
+    }
     void* cargs[] = {&u};
     cudaLaunchKernel(cube_kernel(c.op.shape, cube_kind(c.op) + 1), dim3(grid), dim3(kCubeThreads), cargs,
                      operand_smem(c.op), br.stream[branch]);
