@@ -185,10 +185,9 @@ def run_reference_arm(args):
 # a recorded ncu count is only valid for the same template instance compiled
 # from the same text.
 KERNEL_SOURCES = {
-    "int32x": ["ryser_cube.cuh", "cube_shapes.h", "cube_plan.cpp", "ryser_dense_int.cuh", "ryser_dense.cuh",
-               "perman_common.cuh"],
-    "int32x_dd": ["ryser_cube.cuh", "cube_shapes.h", "cube_plan.cpp", "ryser_dense_sdd.cuh", "ryser_dense_int.cuh",
-                  "ryser_dense.cuh", "perman_common.cuh"],
+    "int32x": ["ryser_cube.cuh", "cube_shapes.h", "ryser_dense_int.cuh", "ryser_dense.cuh", "perman_common.cuh"],
+    "int32x_dd": ["ryser_cube.cuh", "cube_shapes.h", "ryser_dense_sdd.cuh", "ryser_dense_int.cuh", "ryser_dense.cuh",
+                  "perman_common.cuh"],
 }
 
 
@@ -204,19 +203,22 @@ def source_sha16(kname: str) -> str | None:
 
 def kernel_template(kname: str, A: np.ndarray) -> str:
     n = A.shape[0]
-    if n >= 25 and kname in ("int32x", "int32x_dd"):
-        # column-cube walk: the shape depends on the pattern of zeros
-        sha = hashlib.sha256(np.ascontiguousarray(A, dtype=np.float64).tobytes()).hexdigest()[:8]
-        return f"ryser_cube_int_kernel<shape, {'true' if kname == 'int32x_dd' else 'false'}, false>, matrix {sha}"
+    pb = sys.modules.get("perman_b200") or load_pkg()
+    variant = {"int32x": pb.PERM_KERNEL_DENSE_INT, "int32x_dd": pb.PERM_KERNEL_DENSE_INT_DD,
+               "fp64x": pb.PERM_KERNEL_DENSE}.get(kname)
+    shape = pb.cube_layout(A, variant)[0] if variant else -1
+    if shape >= 0:
+        return (f"ryser_cube_kernel<{shape}, false>" if kname == "fp64x" else
+                f"ryser_cube_int_kernel<{shape}, {'true' if kname == 'int32x_dd' else 'false'}, false>")
     if kname == "int32x":
-        g, ngo, ng1, ng2 = (sys.modules.get("perman_b200") or load_pkg()).int_layout(A)
+        g, ngo, ng1, ng2 = pb.int_layout(A)
         if ng1:
             return f"ryser_dense_int_3l_kernel<{n}, {g}, {ng1}, {ng2}>"
         return f"ryser_dense_int_sparse_kernel<{n}, {g}, {ngo}>" if ngo else f"ryser_dense_int_kernel<{n}, {g}>"
     if kname == "int32x_dd":
         # product groups and pairing as the engine lays them out; last template
         # argument: CTAs per SM compiled for (3 up to order 36, 2 above)
-        g, pair, ngo, ng1, ng2 = (sys.modules.get("perman_b200") or load_pkg()).intc_layout(A)
+        g, pair, ngo, ng1, ng2 = pb.intc_layout(A)
         pb_ = "true" if pair else "false"
         if ng1:
             return f"ryser_dense_intc_3l_kernel<{n}, {g}, {pb_}, {ng1}, {ng2}, {3 if n <= 40 else 2}>"
@@ -224,7 +226,7 @@ def kernel_template(kname: str, A: np.ndarray) -> str:
             return f"ryser_dense_intc_sparse_kernel<{n}, {g}, {pb_}, {ngo}, {3 if n <= 36 else 2}>"
         return f"ryser_dense_intc_kernel<{n}, {g}, {pb_}, {3 if n <= 36 else 2}>"
     if kname == "fp64x":
-        r1, r = (sys.modules.get("perman_b200") or load_pkg()).fp64_levels(A)
+        r1, r = pb.fp64_levels(A)
         if r1:
             return f"ryser_dense_3l_kernel<{n}, {r1}, {r}>"
         return f"ryser_dense_2l_kernel<{n}, {r}>" if r else f"ryser_dense_kernel<{n}>"
@@ -499,9 +501,10 @@ def main():
         if prof_stale:
             line["roofline"]["frac_stale"] = True
             line["roofline"]["stale_reason"] = prof_stale
-    line["config"]["kernel"] = {1: "FP64-X column-cube kernel", 3: "int32-X column-cube kernel",
+    walk = "column-cube" if pb.cube_layout(A, r.kernel)[0] >= 0 else "register"
+    line["config"]["kernel"] = {1: f"FP64-X {walk} kernel", 3: f"int32-X {walk} kernel",
                                 5: "tensor-core row sums (tcgen05 kind::i8) + int32 products",
-                                7: "int32-X column-cube kernel, double-double products and sum"}.get(r.kernel, r.kernel)
+                                7: f"int32-X {walk} kernel, double-double products and sum"}.get(r.kernel, r.kernel)
     if r.kernel == pb.PERM_KERNEL_DENSE_INT:
         line["config"]["kernel_instance"] = kernel_template("int32x", A)
     if rank == 0 and not args.no_secondary:
@@ -520,9 +523,19 @@ def main():
         f64.run()
         fr = f64.run()
         f64.free()
+        # FP64 operations the walk executes per Gray step: column cubes a 16th of
+        # their shape's; in rows n updates and n - 1 multiplies (one level), R
+        # inner rows at seven of eight steps (two), 2 R1 at four steps in eight
+        # and 2 R2 at three (three levels)
+        executed = pb.cube_layout(A, pb.PERM_KERNEL_DENSE)[1] / 16
+        if not executed:
+            r1, r2l = pb.fp64_levels(A)
+            executed = ((4 * 2 * r1 + 3 * 2 * r2l + 2 * n - 1) / 8 if r1 else
+                        (7 * 2 * r2l + 2 * n - 1) / 8 if r2l else 2 * n - 1)
         line["secondary"]["dense_n40_fp64x_same_matrix"] = {
             "kernel_ms": fr.kernel_ms, "steps_per_s": total_steps / (fr.kernel_ms * 1e-3),
-            "layout": "column cubes",
+            "kernel_instance": kernel_template("fp64x", A),
+            "fp64_pipe_frac_of_measured_peak": total_steps * executed / (fr.kernel_ms * 1e-3) / peak_ops,
             "fp64_equivalent_frac_of_measured_peak": total_steps * ops_per_step / (fr.kernel_ms * 1e-3) / peak_ops,
             "rel_diff_vs_headline": abs(fr.value - perm_value) / abs(perm_value)}
         line["secondary"]["reference_gpu_same_box"] = reference_gpu(

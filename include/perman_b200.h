@@ -187,8 +187,9 @@ int perm_exact_dense_rows(perm_ctx* ctx, const void* mat, int n, int dtype, int 
  *    PERM_KERNEL_DENSE_INT_DD at once (1.4 int32-X walks in rows, 1.9 in cubes), and real
  *    matrices of order 12..40 whose three sparsest columns touch so few rows
  *    R that the sparse layout's (7 (6R + 9) + 6n + 5) / 8 FP64 operations
- *    per Gray step are at most FP64 X's 2n run PERM_KERNEL_DENSE_SDD in
- *    that layout: their bound is the estimate, no other step runs;
+ *    per Gray step are at most one-level FP64 X's 2n run
+ *    PERM_KERNEL_DENSE_SDD (below order 25 in that layout, from there on in
+ *    column cubes): their bound is the estimate, no other step runs;
  *  - for other nonnegative real matrices of order 28..40 the FP64-X walk's
  *    bound is predicted on the device before any walk (stratified sample of
  *    sum |term| and a weighted-Rasmussen estimate of perm, 4096 trials); when
@@ -233,10 +234,17 @@ int perm_exact_dense_plan(perm_ctx* ctx, const void* mat, int n, int dtype, int*
  * counterpart in the reference (which has no device waits to bound). */
 int perm_ctx_inject_wait_timeout(perm_ctx* ctx, int launches);
 
-/* The layout queries below describe the row layouts: what the walks use below
- * order 25 (the accuracy policy's whole FP64 walks: below order 20), and from
- * there on for matrices too dense for the column-cube walk, which sums the 16
- * sign choices of four columns at once. */
+/* Host only (no device): the walk perm_exact_dense_ex(variant, whole) takes for
+ * the row-major n x n matrix `mat` (variant PERM_KERNEL_DENSE, _INT, _INT_DD or
+ * _SDD): the compiled shape (0 or more) of its column cubes, which sum the 16
+ * sign choices of four columns at once, or -1 for a row layout (and for what
+ * that kernel does not take).  *fp64_ops (may be NULL) receives the FP64
+ * operations of a plain FP64 walk of that shape per 16 terms, 0 without one. */
+int perm_cube_layout(const double* mat, int n, int variant, double* fp64_ops);
+/* The layout queries below describe the row layouts: what perm_exact_dense_rows
+ * walks, and the other calls below order 25 (the accuracy policy's whole FP64
+ * walks: below order 20) and wherever perm_cube_layout is -1 (density 0.8 or so
+ * and more; integer matrices of density 0.7, orders 28 and more, in part). */
 
 /* Host only (no device): the layout PERM_KERNEL_DENSE_SDD uses for the
  * row-major n x n matrix `mat`: the number of inner rows R of the sparse

@@ -45,7 +45,7 @@ EXPORTED_SYMBOLS = (
     "perm_status_string", "perm_exact_dense", "perm_exact_dense_shard", "perm_shard_range", "perm_exact_dense_multi",
     "perm_exact_dense_ex", "perm_exact_dense_rows",
     "perm_exact_sparse", "perm_exact_sparse_ex", "perm_matrix_create_dense", "perm_matrix_create_dense_ex", "perm_matrix_destroy",
-    "perm_exact_dense_resident", "perm_exact_dense_resident_shard", "perm_exact_dense_refine", "perm_sdd_layout", "perm_sdd_levels", "perm_fp64_layout", "perm_fp64_levels", "perm_int_layout", "perm_intc_layout", "perm_exact_dense_plan", "perm_exact_dense_tc_rounds", "perm_exact_dense_noalloc", "perm_dense_autotune", "perm_ctx_set_rel_target", "perm_ctx_inject_wait_timeout",
+    "perm_exact_dense_resident", "perm_exact_dense_resident_shard", "perm_exact_dense_refine", "perm_cube_layout", "perm_sdd_layout", "perm_sdd_levels", "perm_fp64_layout", "perm_fp64_levels", "perm_int_layout", "perm_intc_layout", "perm_exact_dense_plan", "perm_exact_dense_tc_rounds", "perm_exact_dense_noalloc", "perm_dense_autotune", "perm_ctx_set_rel_target", "perm_ctx_inject_wait_timeout",
     "perm_batch_create", "perm_batch_run", "perm_batch_run_ex", "perm_batch_destroy", "perm_batch_exact", "perm_batch_autotune", "perm_batch_variant", "perm_batch_use_variant",
     "perm_server_create", "perm_server_submit", "perm_server_wait", "perm_server_stats", "perm_server_destroy",
     "perm_approx_rasmussen", "perm_approx_scaling", "perm_approx_rasmussen_range", "perm_approx_scaling_range",
@@ -125,6 +125,7 @@ def load_library(path: str | os.PathLike | None = None) -> ctypes.CDLL:
         "perm_exact_dense_rows": (i, [_P, _P, i, i, i, i, i, ctypes.POINTER(PermResult)]),
         "perm_shard_range": (i, [i, i, i, ctypes.POINTER(u64), ctypes.POINTER(u64)]),
         "perm_exact_dense_multi": (i, [_P, i, i, i, i, _P, ctypes.POINTER(PermResult)]),
+        "perm_cube_layout": (i, [_P, i, i, ctypes.POINTER(d)]),
         "perm_sdd_layout": (i, [_P, i]),
         "perm_sdd_levels": (i, [_P, i, _P]),
         "perm_intc_layout": (i, [_P, i, ctypes.POINTER(ctypes.c_int), _P]),
@@ -623,6 +624,14 @@ def compress(mode: int, mat) -> dict:
         raise PermError(nnz, "perm_compress failed")
     return {"n": n, "nnz": nnz, "mat": a, "cptrs": cptrs, "rows": rows[:nnz], "cvals": cvals[:nnz],
             "rptrs": rptrs, "cols": cols[:nnz], "rvals": rvals[:nnz]}
+
+
+def cube_layout(mat, variant: int) -> tuple[int, float]:
+    """(shape, FP64 operations per 16 terms) of the column cubes that
+    exact_dense(variant) walks; (-1, 0.0): a row layout.  Host only."""
+    a = np.ascontiguousarray(np.asarray(mat, dtype=np.float64))
+    ops = ctypes.c_double(0.0)
+    return load_library().perm_cube_layout(_ptr(a), a.shape[0], variant, ctypes.byref(ops)), ops.value
 
 
 def sdd_layout(mat) -> int:

@@ -35,9 +35,9 @@ WalkSide walk_side(const std::vector<double>& a, int n);
 bool cube_layout(const std::vector<double>& a, int n, double max_cost, bool transpose, CubeLayout* layout);
 
 // FP64 operations per 16 terms of a shape's FP64 walk, and the same weighted
-// by the rate its size reaches: measured 0.80..0.85 of the FP64 pipe up to 130
-// row values, 0.73 at 198, 0.65 at 257, 0.62 at 364, as operations at a rate
-// of 0.82.
+// by the rate its size reaches, as operations at a rate of 0.82: fitted to
+// 0.80..0.85 up to 130 row values, 0.73 at 198, 0.65 at 257, 0.62 at 364, all of
+// the FP64 peak that dependent chains of FMAs measure (0.92 of the pipe's).
 double cube_shape_ops(int shape);
 double cube_shape_cost(int shape);
 

@@ -573,8 +573,8 @@ struct perm_ctx {
 };
 
 static const int kMaxBlocks = 8192;
-// Column-cube walks recompute b after this many cubes: its updates' roundings
-// add up over no more steps than in the row layouts (2^11 terms a segment),
+// Column-cube walks recompute b after this many cubes (2^12 terms): its
+// updates' roundings add up over 256 steps, in the row layouts over up to 2^12,
 // and the n (n - 5) additions are below 2% of the segment.
 constexpr uint64_t kCubeSegment = 256;
 
@@ -1890,6 +1890,19 @@ extern "C" int perm_sdd_levels(const double* mat, int n, int* levels) {
   return PERM_OK;
 }
 
+extern "C" int perm_cube_layout(const double* mat, int n, int variant, double* fp64_ops) {
+  if (fp64_ops) *fp64_ops = 0.0;
+  if (!mat || n < 1 || n > PERM_MAX_EXACT_N) return -1;
+  if (variant != PERM_KERNEL_DENSE && variant != PERM_KERNEL_DENSE_INT && variant != PERM_KERNEL_DENSE_INT_DD &&
+      variant != PERM_KERNEL_DENSE_SDD)
+    return -1;
+  perm_ctx host;  // keeps the message of a refusal
+  DenseOperand op;
+  if (build_operand(&host, mat, n, PERM_F64, variant, &op) != PERM_OK) return -1;
+  if (op.shape >= 0 && fp64_ops) *fp64_ops = cube_shape_ops(op.shape);
+  return op.shape;
+}
+
 extern "C" int perm_shard_range(int n, int shard, int nshards, uint64_t* first, uint64_t* last) {
   if (n < 1 || n > PERM_MAX_EXACT_N || nshards < 1 || shard < 0 || shard >= nshards || !first || !last)
     return PERM_EINVAL;
@@ -2004,6 +2017,7 @@ static int dense_plan(perm_ctx* ctx, const DenseOperand& op, int shard, int nsha
   }
   int grid = std::min(kMaxBlocks, ctx->num_sms * occ_slot);
   if (op.shape >= 0) {
+    grid = std::min(grid, kMaxBlocks / kCubePartials);
     p->m = 4 + cube_align((last - first) >> 4, (uint64_t)grid * operand_threads(op), nshards == 1 ? n - 5 : ms - 4);
     p->block0 = first >> p->m;
     p->nblocks = (last - first) >> p->m;
@@ -2491,10 +2505,12 @@ static int refine_result(perm_ctx* ctx, const void* mat, int n, int dtype, const
 // With the accuracy policy on, the kernel a whole-walk call starts with
 // when a certified walk is cheap enough to go first: int32 X with
 // double-double products for integer matrices (about 1.4 int32-X walks, its
-// bound needs no sample), split-dd in the sparse layout for real matrices
-// whose three sparsest columns touch so few rows R that its
-// (7 (6R + 9) + 6n + 5) / 8 FP64 operations per Gray step are no more than
-// the FP64-X walk's 2n (cfg-2-like matrices: n = 36, R = 6, 67 against 72).
+// bound needs no sample), split-dd for real matrices whose three sparsest
+// columns touch so few rows R that the (7 (6R + 9) + 6n + 5) / 8 FP64 operations
+// per Gray step of its sparse layout are no more than the one-level FP64-X
+// walk's 2n (sparse real matrices of order 36: R = 6, 67 against 72).  From
+// order 25 both walk column cubes instead; the line between them was drawn for
+// the row layouts and not moved.
 // 0: the FP64-X / int32-X walk goes first (host checks only;
 // policy_predicts_sdd may still choose split-dd for a real matrix).
 static int policy_first_kernel(const void* mat, int n, int dtype) {
@@ -2903,7 +2919,10 @@ static int run_skipper(perm_ctx* ctx, int n, const int* rptrs, const int* cols, 
 // pseudo-random sample (deterministic) have an x vector with a zero entry.
 // SkipPer only pays off when most terms vanish: a visited index costs it
 // several times a dense-kernel step, so below kSkipperZeroFraction the register
-// kernel runs instead (same matrix, same permanent).  Row by row up to the
+// kernel runs instead (same matrix, same permanent).  The line was drawn against
+// the row layouts; column cubes win somewhat above it too (0/1 matrices, n = 36:
+// 1e7..7e7 visited indices 1.5..3.5 ms and 33 in cubes, 1.1e9 of them 43 ms and
+// 33; n = 30: 5e6 0.4..0.5 ms, 1.8e7 1.3, cubes 0.51).  Row by row up to the
 // first zero, and until the answer is settled (the call beyond the kernel, n =
 // 36, three nonzeros a row: 0.55 ms with every x vector built whole, 0.1 so).
 static const double kSkipperZeroFraction = 0.75;
@@ -3618,7 +3637,8 @@ static int batch_create_locked(perm_ctx* ctx, int count, const int* orders, cons
     const BatchCube& c = cube[i];
     const int branch = (int)(i % branches);
     const uint64_t cubes_n = 1ull << (c.op.n - 5);
-    const int grid = (int)std::min<uint64_t>((uint64_t)ctx->num_sms, std::max<uint64_t>(1, cubes_n / (64 * kCubeThreads)));
+    const int sms = std::min(ctx->num_sms, kMaxBlocks / kCubePartials);
+    const int grid = (int)std::min<uint64_t>((uint64_t)sms, std::max<uint64_t>(1, cubes_n / (64 * kCubeThreads)));
     const int m = cube_align(cubes_n, (uint64_t)grid * kCubeThreads, c.op.n - 5);
     CubeLaunch u;
     cube_args(c.op, b->d_cubes + c.offset, m, 0, cubes_n >> m, &u);

@@ -29,9 +29,9 @@
 // for the three-level row layout this replaced (n = 32, density 1/2: 5.8..6.4 ms
 // then, 2.3..3.6 ms by shape now).
 //
-// Bound: the FP64 pipe, 80..85% of it on order-32 shapes up to 130 row values
-// (the rest are fixed latencies between dependent products: 2.4 warps' worth
-// of independent work per scheduler), falling to 62% at 360 values.  The sums
+// Bound: the FP64 pipe, 74..83% of it at orders 32..34 up to 130 row values,
+// 72% at 142, 60..65% at 200..290 (the rest are fixed latencies between dependent
+// products: 2.4 warps' worth of independent work per scheduler).  The sums
 // c are kernel parameters, read as constant operands of the additions: from
 // shared memory they would take more cycles than the arithmetic (a 64-bit
 // broadcast load takes two, an addition and a multiply one; 3.5..3.9 ms at
@@ -424,30 +424,27 @@ __device__ __forceinline__ void cube_walk(const CubeWalk& a, Start start, Flip f
 }
 
 // The thread totals' sum to *out and, with abs_sum, that of m1 to *sums; both in
-// a fixed order, so that a walk's error estimate is the same every time.  A
-// block's m1 stands behind the blocks' totals in `partials`.
+// a fixed order, so that a walk's error estimate is the same every time.  The
+// warps' m1 stand behind the blocks' totals in `partials`.
 __device__ __forceinline__ void cube_finish(const CubeWalk& a, dd total, bool abs_sum, double m1, double factor, dd* red) {
   constexpr int kWarps = kCubeThreads / 32;
-  static_assert(2 * kWarps <= 32, "red holds the warps' totals and their m1");
-  const int lane = threadIdx.x & 31;
+  double* sums = reinterpret_cast<double*>(a.partials + gridDim.x);
   if (abs_sum) {
 #pragma unroll
     for (int d = 16; d >= 1; d >>= 1) m1 += __shfl_down_sync(0xffffffffu, m1, d);
-    if (lane == 0) red[kWarps + (threadIdx.x >> 5)].hi = m1;
+    if ((threadIdx.x & 31) == 0) {
+      sums[blockIdx.x * kWarps + (threadIdx.x >> 5)] = m1;
+      __threadfence();
+    }
   }
-  const dd bt = block_reduce_dd(total, red);  // red is written before its barrier
-  if (abs_sum && threadIdx.x == 0) {
-    double s = 0.0;
-    for (int w = 0; w < kWarps; w++) s += red[kWarps + w].hi;
-    a.partials[gridDim.x + blockIdx.x].hi = s;
-  }
+  const dd bt = block_reduce_dd(total, red);
   const bool last = grid_finish_dd(bt, a.partials, a.ticket, a.out, factor, red);
   if (!abs_sum || !last || threadIdx.x >= 32) return;
   double s = 0.0;
-  for (unsigned b = lane; b < gridDim.x; b += 32) s += __ldcg(&a.partials[gridDim.x + b].hi);
+  for (unsigned w = threadIdx.x; w < gridDim.x * kWarps; w += 32) s += __ldcg(sums + w);
 #pragma unroll
   for (int d = 16; d >= 1; d >>= 1) s += __shfl_down_sync(0xffffffffu, s, d);
-  if (lane == 0) *a.sums = s;
+  if (threadIdx.x == 0) *a.sums = s;
 }
 
 // FP64 walk; kAbs: *sums = sum |term| as well (16 of some 250 operations).

@@ -11,6 +11,9 @@ struct dd;
 
 // Threads per CTA, one CTA per SM (ryser_cube.cuh).
 constexpr int kCubeThreads = 256;
+// Partial sums per block, in double-double words: its total and its warps' sums
+// of |term|.
+constexpr int kCubePartials = 1 + kCubeThreads / 64;
 // Rows whose product the certified integer walk keeps in FP64 exactly.
 constexpr int kCubeExactRows = 8;
 
@@ -20,7 +23,7 @@ struct CubeWalk {
   int m;                     // log2 of the range alignment, in outer Gray indices
   uint64_t block0, nblocks;  // aligned blocks of 2^m outer indices of this launch
   uint64_t seg;              // cubes between two recomputations of b
-  dd* partials;  // two per block of the grid
+  dd* partials;  // kCubePartials per block of the grid
   unsigned* ticket;
   double* out;
   double* sums;  // sum |term| (walks that sum it)
