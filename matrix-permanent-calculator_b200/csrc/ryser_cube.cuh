@@ -564,10 +564,11 @@ __global__ void __launch_bounds__(kCubeThreads, 1) ryser_cube_sdd_kernel(const _
 // FP64 products (kDd false), or double-double products and sum with a
 // certified error (ryser_dense_intc.cuh), where products of up to
 // kCubeExactRows rows are kept in FP64 exactly (checked by the host).
-// FP64 products, order-40 shape of 140 values: 182 cycles per warp and cube,
-// 0.66 instructions issued per cycle and scheduler, FP64 pipe 46%, conversions
-// 30% (n = 40, density 1/2: 375 in the three-level row layout before).
-// Constants of both signs instead of mirrored ones: 200 (the compiler loads
+// FP64 products, order-40 shape of 140 values: 186 cycles per warp and cube,
+// 0.64 instructions issued per cycle and scheduler, FP64 pipe 46%, conversions
+// 30% (n = 40, density 1/2: 375 in the three-level row layout before).  In a
+// program of this walk alone, one sum a cube, 182:
+// constants of both signs instead of mirrored ones 200 (the compiler loads
 // them to registers early); left-over rows added to the bit pattern of 2^52 + b
 // instead of converted: 187; 12 warps of 168 registers: 185 and spills in the
 // larger shapes.  Certified: 364 cycles, of which the double-double arrays and
