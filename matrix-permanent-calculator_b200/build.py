@@ -24,9 +24,7 @@ LIB = PKG / "libperman_b200.so"
 CLI = PKG / "bin" / "perman"
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-# --compress-mode=size: the library holds some two thousand kernel instances,
-# 380 MB of device code that compresses tenfold
-NVCC_FLAGS = ["-O3", "--compress-mode=size", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-Wall",
+NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-Wall",
               "--expt-relaxed-constexpr", f"-I{INCLUDE}"]
 HOST_CXX = os.environ.get("PERM_HOST_CXX", "/usr/bin/g++")
 
@@ -74,7 +72,10 @@ def _compile(src: Path, force: bool) -> Path:
     obj = BUILD / (src.name + ".o")
     if not force and not _stale(obj, _deps(src)):
         return obj
-    cmd = [nvcc(), *ARCH, *NVCC_FLAGS, f"-ccbin={HOST_CXX}", "-c", str(src), "-o", str(obj)]
+    # the column cubes' 528 instances compress tenfold and load in 5 ms; row
+    # kernels' modules, larger, would take 25 ms instead of 20 (once a process)
+    small = ["--compress-mode=size"] if src.name.startswith("ryser_cube") else []
+    cmd = [nvcc(), *ARCH, *NVCC_FLAGS, *small, f"-ccbin={HOST_CXX}", "-c", str(src), "-o", str(obj)]
     if src.suffix == ".cpp":
         cmd = [nvcc(), "-x", "cu", *cmd[1:]]
     res = subprocess.run(cmd, capture_output=True, text=True)
