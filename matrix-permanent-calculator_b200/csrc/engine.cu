@@ -400,10 +400,10 @@ __global__ void __launch_bounds__(256) ryser_abs_sample_kernel(const double* col
     is_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
   }
   __syncthreads();
-  if (!is_last || threadIdx.x >= 32) return;
+  if (!is_last) return;
   __threadfence();
   local = local2 = 0.0;
-  for (unsigned b = threadIdx.x; b < gridDim.x; b += 32) {
+  for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x) {
     local += __ldcg(&partials[b].hi);
     local2 += __ldcg(&partials[b].lo);
   }
@@ -411,7 +411,16 @@ __global__ void __launch_bounds__(256) ryser_abs_sample_kernel(const double* col
     local += __shfl_down_sync(0xffffffffu, local, d);
     local2 += __shfl_down_sync(0xffffffffu, local2, d);
   }
+  if ((threadIdx.x & 31) == 0) {
+    red[threadIdx.x >> 5] = local;
+    red2[threadIdx.x >> 5] = local2;
+  }
+  __syncthreads();
   if (threadIdx.x == 0) {
+    for (int w = 1; w < (int)(blockDim.x >> 5); w++) {
+      local += red[w];
+      local2 += red2[w];
+    }
     out[0] = local;
     out[1] = local2;
     *ticket = 0u;
@@ -501,6 +510,11 @@ using namespace perm;
 struct DenseOperand;
 struct perm_matrix;
 
+// Result words of a call, and of the column cubes' sums of |term| after them
+// (kCubeWarps a block, at most kCubeBlocks blocks an SM).
+constexpr int kOutWords = 16;
+constexpr int kCubeBlocks = 2048 / kCubeThreads;
+
 // Smallest order of the column-cube walks: the shards of shard_bounds are
 // whole cubes of 16 terms from here on, and below it the search for four
 // columns (some 30 us on the host) costs what the walk gains.
@@ -531,8 +545,8 @@ struct perm_ctx {
   // scratch, allocated once
   dd* partials = nullptr;  // kMaxBlocks dd
   unsigned* ticket = nullptr;
-  // One block of 16 words, read back by one copy: [0..7] results, [8] d_err,
-  // [9..10] d_counters, [12..14] d_est.
+  // One block, read back by one copy: [0..7] results, [8] d_err, [9..10]
+  // d_counters, [12..14] d_est, from kOutWords on the column cubes' sums of |term|.
   double* d_out = nullptr;
   int* d_err = nullptr;
   unsigned long long* d_counters = nullptr;  // [0] queue head, [1] visited
@@ -723,13 +737,14 @@ static int ctx_init(perm_ctx* ctx, int device) {
   CU(ctx, cudaEventCreate(&ctx->ev1));
   CU(ctx, cudaMalloc(&ctx->partials, sizeof(dd) * kMaxBlocks * 2));
   CU(ctx, cudaMalloc(&ctx->ticket, sizeof(unsigned) * 4));
-  CU(ctx, cudaMalloc(&ctx->d_out, sizeof(double) * 16));
+  const size_t out_words = kOutWords + (size_t)ctx->num_sms * kCubeBlocks * kCubeWarps;
+  CU(ctx, cudaMalloc(&ctx->d_out, sizeof(double) * out_words));
   ctx->d_err = reinterpret_cast<int*>(ctx->d_out + 8);
   ctx->d_counters = reinterpret_cast<unsigned long long*>(ctx->d_out + 9);
   ctx->d_est = ctx->d_out + 12;
   CU(ctx, cudaMemset(ctx->ticket, 0, sizeof(unsigned) * 4));
-  CU(ctx, cudaMemset(ctx->d_out, 0, sizeof(double) * 16));
-  CU(ctx, cudaMallocHost(&ctx->h_out, sizeof(double) * 16));
+  CU(ctx, cudaMemset(ctx->d_out, 0, sizeof(double) * out_words));
+  CU(ctx, cudaMallocHost(&ctx->h_out, sizeof(double) * out_words));
   return PERM_OK;
 }
 
@@ -751,10 +766,12 @@ extern "C" int perm_ctx_create(int device, perm_ctx** out) {
 }
 
 // Reads back the result block (results, error flag, counters, moments) after
-// the stream drains; `meanwhile` runs on the host before the wait.
+// the stream drains, with `sums` words of the column cubes' sums; `meanwhile`
+// runs on the host before the wait.
 template <class Meanwhile>
-static int finish_and_read(perm_ctx* ctx, Meanwhile meanwhile) {
-  CU(ctx, cudaMemcpyAsync(ctx->h_out, ctx->d_out, sizeof(double) * 16, cudaMemcpyDeviceToHost, ctx->stream));
+static int finish_and_read(perm_ctx* ctx, int sums, Meanwhile meanwhile) {
+  CU(ctx, cudaMemcpyAsync(ctx->h_out, ctx->d_out, sizeof(double) * (kOutWords + sums), cudaMemcpyDeviceToHost,
+                          ctx->stream));
   meanwhile();
   CU(ctx, cudaStreamSynchronize(ctx->stream));
   CU(ctx, cudaGetLastError());
@@ -770,7 +787,7 @@ static int finish_and_read(perm_ctx* ctx, Meanwhile meanwhile) {
 }
 
 static int finish_and_read(perm_ctx* ctx) {
-  return finish_and_read(ctx, [] {});
+  return finish_and_read(ctx, 0, [] {});
 }
 
 // ---------------------------------------------------------------------------
@@ -2017,7 +2034,7 @@ static int dense_plan(perm_ctx* ctx, const DenseOperand& op, int shard, int nsha
   }
   int grid = std::min(kMaxBlocks, ctx->num_sms * occ_slot);
   if (op.shape >= 0) {
-    grid = std::min(grid, kMaxBlocks / kCubePartials);
+    grid = std::min(grid, ctx->num_sms * kCubeBlocks);
     p->m = 4 + cube_align((last - first) >> 4, (uint64_t)grid * operand_threads(op), nshards == 1 ? n - 5 : ms - 4);
     p->block0 = first >> p->m;
     p->nblocks = (last - first) >> p->m;
@@ -2052,7 +2069,7 @@ static int dense_launch(perm_ctx* ctx, const DenseOperand& op, const void* d_ima
     args.partials = ctx->partials;
     args.ticket = ctx->ticket;
     args.out = ctx->d_out;
-    args.sums = ctx->d_est;
+    args.sums = ctx->d_out + kOutWords;
     args.err = ctx->d_err;
     if (ctx->inject_timeouts > 0 && (kind == kCubeF64 || kind == kCubeF64Abs)) {
       args.inject = 16u;
@@ -2164,8 +2181,14 @@ static int dense_collect(perm_ctx* ctx, const DenseOperand& op, const DensePlan&
                          Meanwhile meanwhile) {
   const bool sums = op.variant == PERM_KERNEL_DENSE_SPLIT || op.variant == PERM_KERNEL_DENSE_INT_DD ||
                     op.variant == PERM_KERNEL_DENSE_SDD || op.abs_sum;
-  int rc = finish_and_read(ctx, meanwhile);
+  const int cube_sums = sums && op.shape >= 0 ? p.grid * kCubeWarps : 0;
+  int rc = finish_and_read(ctx, cube_sums, meanwhile);
   if (rc != PERM_OK) return rc;
+  if (cube_sums) {
+    double m1 = 0.0;
+    for (int w = 0; w < cube_sums; w++) m1 += ctx->h_out[kOutWords + w];
+    ctx->h_out[12] = m1;
+  }
   if (op.variant == PERM_KERNEL_DENSE_SPLIT) {
     ctx->split_m1 = ctx->h_out[12] * 2.0;  // |factor| = 2
     ctx->split_m2 = ctx->h_out[13] * 4.0;
@@ -3288,6 +3311,24 @@ struct BatchCube {
   uint64_t offset = 0;  // of its image in d_cubes, bytes
 };
 
+// A batch's sums of |term| of its column cubes: one block per cube adds its
+// warps' sums in a fixed order.
+struct CubeSum {
+  uint64_t first;  // in the sums of all cubes
+  int count;
+  int index;  // of the matrix
+};
+__global__ void __launch_bounds__(128) cube_sums_kernel(const CubeSum* cubes, const double* sums, double* results) {
+  __shared__ double red[4];
+  const CubeSum c = cubes[blockIdx.x];
+  double s = 0.0;
+  for (int w = threadIdx.x; w < c.count; w += 128) s += sums[c.first + w];
+  for (int d = 16; d >= 1; d >>= 1) s += __shfl_down_sync(0xffffffffu, s, d);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) results[3 * (size_t)c.index + 2] = ((red[0] + red[1]) + red[2]) + red[3];
+}
+
 struct perm_batch {
   int count = 0;
   uint64_t total_tiles = 0;
@@ -3305,6 +3346,8 @@ struct perm_batch {
   unsigned char* d_cubes = nullptr;  // column images of the column-cube walks
   dd* d_cube_partials = nullptr;     // per branch of the graph: partials, tickets
   unsigned* d_cube_tickets = nullptr;
+  double* d_cube_sums = nullptr;  // of all cubes' warps
+  CubeSum* d_cube_sum = nullptr;  // where each cube's are
   std::vector<double> roundings;  // per matrix: roundings per term
   std::vector<double> abs_scale;  // per matrix: factor of its sum |term|
   std::vector<std::pair<int, int>> exp2;  // matrices whose three results are multiplied by 2^second
@@ -3331,6 +3374,8 @@ static void batch_free(perm_batch* b) {
   cudaFree(b->d_cubes);
   cudaFree(b->d_cube_partials);
   cudaFree(b->d_cube_tickets);
+  cudaFree(b->d_cube_sums);
+  cudaFree(b->d_cube_sum);
   if (b->h_results) cudaFreeHost(b->h_results);
   delete b;
 }
@@ -3559,6 +3604,11 @@ static int batch_create_locked(perm_ctx* ctx, int count, const int* orders, cons
   BT(cudaMalloc(&b->d_tile_abs, sizeof(double) * std::max<uint64_t>(tiles, 1)));
   BT(cudaMalloc(&b->d_mat_done, sizeof(unsigned) * count));
   BT(cudaMalloc(&b->d_next, sizeof(unsigned long long)));
+  std::vector<CubeSum> cube_sum;
+  auto cube_grid = [&](const BatchCube& c) {
+    const uint64_t cubes_n = 1ull << (c.op.n - 5);
+    return (int)std::min<uint64_t>((uint64_t)ctx->num_sms, std::max<uint64_t>(1, cubes_n / (64 * kCubeThreads)));
+  };
   const size_t result_bytes = sizeof(double) * (3 * (size_t)count + 1);
   BT(cudaMalloc(&b->d_results, result_bytes));
   BT(cudaMemset(b->d_results, 0, result_bytes));
@@ -3571,6 +3621,19 @@ static int batch_create_locked(perm_ctx* ctx, int count, const int* orders, cons
     BT(cudaMalloc(&b->d_cube_partials, sizeof(dd) * kMaxBlocks * kBatchBranches));
     BT(cudaMalloc(&b->d_cube_tickets, sizeof(unsigned) * kBatchBranches));
     BT(cudaMemset(b->d_cube_tickets, 0, sizeof(unsigned) * kBatchBranches));
+    cube_sum.reserve(cube.size());
+    uint64_t warps = 0;
+    for (const BatchCube& c : cube) {
+      cube_sum.push_back({warps, cube_grid(c) * kCubeWarps, c.index});
+      warps += cube_sum.back().count;
+    }
+    BT(cudaMalloc(&b->d_cube_sums, sizeof(double) * warps));
+    BT(cudaMalloc(&b->d_cube_sum, sizeof(CubeSum) * cube_sum.size()));
+    BT(cudaMemcpy(b->d_cube_sum, cube_sum.data(), sizeof(CubeSum) * cube_sum.size(), cudaMemcpyHostToDevice));
+    if (int rc2 = allow_smem(ctx, (const void*)cube_sums_kernel, 0)) {  // loads it before the capture
+      batch_free(b);
+      return rc2;
+    }
     for (const BatchCube& c : cube)
       if (int rc2 = allow_smem(ctx, cube_kernel(c.op.shape, cube_kind(c.op) + 1), operand_smem(c.op))) {
         batch_free(b);
@@ -3637,15 +3700,14 @@ static int batch_create_locked(perm_ctx* ctx, int count, const int* orders, cons
     const BatchCube& c = cube[i];
     const int branch = (int)(i % branches);
     const uint64_t cubes_n = 1ull << (c.op.n - 5);
-    const int sms = std::min(ctx->num_sms, kMaxBlocks / kCubePartials);
-    const int grid = (int)std::min<uint64_t>((uint64_t)sms, std::max<uint64_t>(1, cubes_n / (64 * kCubeThreads)));
+    const int grid = cube_grid(c);
     const int m = cube_align(cubes_n, (uint64_t)grid * kCubeThreads, c.op.n - 5);
     CubeLaunch u;
     cube_args(c.op, b->d_cubes + c.offset, m, 0, cubes_n >> m, &u);
     u.walk.partials = b->d_cube_partials + (size_t)branch * kMaxBlocks;
     u.walk.ticket = b->d_cube_tickets + branch;
     u.walk.out = b->d_results + 3 * c.index;
-    u.walk.sums = b->d_results + 3 * c.index + 2;
+    u.walk.sums = b->d_cube_sums + cube_sum[i].first;
     u.walk.err = reinterpret_cast<int*>(b->d_results + 3 * (size_t)count);
     if (ctx->inject_timeouts > 0 && cube_kind(c.op) == kCubeF64) {
       u.walk.inject = 16u;
@@ -3661,6 +3723,8 @@ static int batch_create_locked(perm_ctx* ctx, int count, const int* orders, cons
     cudaEventRecord(br.join[i], br.stream[i]);
     cudaStreamWaitEvent(ctx->stream, br.join[i], 0);
   }
+  if (branches)
+    cube_sums_kernel<<<(unsigned)cube.size(), 128, 0, ctx->stream>>>(b->d_cube_sum, b->d_cube_sums, b->d_results);
   cudaMemcpyAsync(b->h_results, b->d_results, result_bytes, cudaMemcpyDeviceToHost, ctx->stream);
   BT(cudaStreamEndCapture(ctx->stream, &b->graph));
   BT(cudaGraphInstantiate(&b->exec, b->graph, 0));

@@ -103,10 +103,8 @@ __device__ __forceinline__ dd block_reduce_dd(dd v, dd* red) {
 // finishes last (atomic ticket) sums all partials in block order -- the
 // result is therefore independent of block scheduling -- writes it to *out
 // multiplied by `factor` (a power of two, exact), and re-arms the ticket.
-// `partials` holds gridDim.x entries, `ticket` starts (and ends) at 0.  True in
-// the block that finished last, to which all that the others wrote before the
-// call is visible.
-__device__ __forceinline__ bool grid_finish_dd(dd block_total, dd* partials, unsigned* ticket,
+// `partials` holds gridDim.x entries, `ticket` starts (and ends) at 0.
+__device__ __forceinline__ void grid_finish_dd(dd block_total, dd* partials, unsigned* ticket,
                                                double* out, double factor, dd* red) {
   __shared__ bool is_last;
   if (threadIdx.x == 0) {
@@ -116,7 +114,7 @@ __device__ __forceinline__ bool grid_finish_dd(dd block_total, dd* partials, uns
     is_last = (prev == gridDim.x - 1);
   }
   __syncthreads();
-  if (!is_last) return false;
+  if (!is_last) return;
   __threadfence();
   // Ordered sum by warp 0: each lane sums a strided slice in index order,
   // then the 32 lane sums are combined in a fixed tree.
@@ -138,7 +136,6 @@ __device__ __forceinline__ bool grid_finish_dd(dd block_total, dd* partials, uns
     }
   }
   (void)red;
-  return true;
 }
 
 // ---------------------------------------------------------------------------

@@ -423,31 +423,22 @@ __device__ __forceinline__ void cube_walk(const CubeWalk& a, Start start, Flip f
   }
 }
 
-// The thread totals' sum to *out and, with abs_sum, that of m1 to *sums; both in
-// a fixed order, so that a walk's error estimate is the same every time.  The
-// warps' m1 stand behind the blocks' totals in `partials`.
+// The thread totals' sum to *out and, with abs_sum, every warp's sum of m1 to
+// `sums`, which are added in their order afterwards (by the host, or by
+// cube_sums_kernel in a batch), so that a walk's error estimate is the same every
+// time.  Adding them here, by the block that finishes last, changed the register
+// allocation of the certified walks: up to 4% slower by shape.
 __device__ __forceinline__ void cube_finish(const CubeWalk& a, dd total, bool abs_sum, double m1, double factor, dd* red) {
-  constexpr int kWarps = kCubeThreads / 32;
-  double* sums = reinterpret_cast<double*>(a.partials + gridDim.x);
   if (abs_sum) {
 #pragma unroll
     for (int d = 16; d >= 1; d >>= 1) m1 += __shfl_down_sync(0xffffffffu, m1, d);
-    if ((threadIdx.x & 31) == 0) {
-      sums[blockIdx.x * kWarps + (threadIdx.x >> 5)] = m1;
-      __threadfence();
-    }
+    if ((threadIdx.x & 31) == 0) a.sums[blockIdx.x * kCubeWarps + (threadIdx.x >> 5)] = m1;
   }
   const dd bt = block_reduce_dd(total, red);
-  const bool last = grid_finish_dd(bt, a.partials, a.ticket, a.out, factor, red);
-  if (!abs_sum || !last || threadIdx.x >= 32) return;
-  double s = 0.0;
-  for (unsigned w = threadIdx.x; w < gridDim.x * kWarps; w += 32) s += __ldcg(sums + w);
-#pragma unroll
-  for (int d = 16; d >= 1; d >>= 1) s += __shfl_down_sync(0xffffffffu, s, d);
-  if (threadIdx.x == 0) *a.sums = s;
+  grid_finish_dd(bt, a.partials, a.ticket, a.out, factor, red);
 }
 
-// FP64 walk; kAbs: *sums = sum |term| as well (16 of some 250 operations).
+// FP64 walk; kAbs: its sum |term| as well (16 of some 250 operations).
 template <int kShape, bool kAbs>
 __global__ void __launch_bounds__(kCubeThreads, 1) ryser_cube_kernel(const __grid_constant__ CubeArgs a) {
   constexpr int N = cube_rows(kCubeShapes[kShape]);

@@ -11,9 +11,7 @@ struct dd;
 
 // Threads per CTA, one CTA per SM (ryser_cube.cuh).
 constexpr int kCubeThreads = 256;
-// Partial sums per block, in double-double words: its total and its warps' sums
-// of |term|.
-constexpr int kCubePartials = 1 + kCubeThreads / 64;
+constexpr int kCubeWarps = kCubeThreads / 32;
 // Rows whose product the certified integer walk keeps in FP64 exactly.
 constexpr int kCubeExactRows = 8;
 
@@ -23,10 +21,10 @@ struct CubeWalk {
   int m;                     // log2 of the range alignment, in outer Gray indices
   uint64_t block0, nblocks;  // aligned blocks of 2^m outer indices of this launch
   uint64_t seg;              // cubes between two recomputations of b
-  dd* partials;  // kCubePartials per block of the grid
+  dd* partials;
   unsigned* ticket;
   double* out;
-  double* sums;  // sum |term| (walks that sum it)
+  double* sums;  // kCubeWarps per block: sum |term| (walks that sum it)
   int* err;
   uint32_t inject;  // failure injection (tests): staging expects this many extra bytes
 };
