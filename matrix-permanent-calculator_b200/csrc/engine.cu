@@ -510,8 +510,8 @@ using namespace perm;
 struct DenseOperand;
 struct perm_matrix;
 
-// Result words of a call, and of the column cubes' sums of |term| after them
-// (kCubeWarps a block, at most kCubeBlocks blocks an SM).
+// Result words of a call; the column cubes' partials are behind them (kCubeWords a
+// block, at most kCubeBlocks blocks an SM).
 constexpr int kOutWords = 16;
 constexpr int kCubeBlocks = 2048 / kCubeThreads;
 
@@ -546,7 +546,7 @@ struct perm_ctx {
   dd* partials = nullptr;  // kMaxBlocks dd
   unsigned* ticket = nullptr;
   // One block, read back by one copy: [0..7] results, [8] d_err, [9..10]
-  // d_counters, [12..14] d_est, from kOutWords on the column cubes' sums of |term|.
+  // d_counters, [12..14] d_est, from kOutWords on the column cubes' partials.
   double* d_out = nullptr;
   int* d_err = nullptr;
   unsigned long long* d_counters = nullptr;  // [0] queue head, [1] visited
@@ -737,7 +737,7 @@ static int ctx_init(perm_ctx* ctx, int device) {
   CU(ctx, cudaEventCreate(&ctx->ev1));
   CU(ctx, cudaMalloc(&ctx->partials, sizeof(dd) * kMaxBlocks * 2));
   CU(ctx, cudaMalloc(&ctx->ticket, sizeof(unsigned) * 4));
-  const size_t out_words = kOutWords + (size_t)ctx->num_sms * kCubeBlocks * kCubeWarps;
+  const size_t out_words = kOutWords + (size_t)ctx->num_sms * kCubeBlocks * kCubeWords;
   CU(ctx, cudaMalloc(&ctx->d_out, sizeof(double) * out_words));
   ctx->d_err = reinterpret_cast<int*>(ctx->d_out + 8);
   ctx->d_counters = reinterpret_cast<unsigned long long*>(ctx->d_out + 9);
@@ -766,11 +766,11 @@ extern "C" int perm_ctx_create(int device, perm_ctx** out) {
 }
 
 // Reads back the result block (results, error flag, counters, moments) after
-// the stream drains, with `sums` words of the column cubes' sums; `meanwhile`
+// the stream drains, with `partials` words of a column-cube walk's; `meanwhile`
 // runs on the host before the wait.
 template <class Meanwhile>
-static int finish_and_read(perm_ctx* ctx, int sums, Meanwhile meanwhile) {
-  CU(ctx, cudaMemcpyAsync(ctx->h_out, ctx->d_out, sizeof(double) * (kOutWords + sums), cudaMemcpyDeviceToHost,
+static int finish_and_read(perm_ctx* ctx, int partials, Meanwhile meanwhile) {
+  CU(ctx, cudaMemcpyAsync(ctx->h_out, ctx->d_out, sizeof(double) * (kOutWords + partials), cudaMemcpyDeviceToHost,
                           ctx->stream));
   meanwhile();
   CU(ctx, cudaStreamSynchronize(ctx->stream));
@@ -2066,10 +2066,9 @@ static int dense_launch(perm_ctx* ctx, const DenseOperand& op, const void* d_ima
     CubeLaunch u;
     cube_args(op, d_image, p.m - 4, p.block0, p.nblocks, &u);
     CubeWalk& args = u.walk;
-    args.partials = ctx->partials;
+    args.partials = reinterpret_cast<dd*>(ctx->d_out + kOutWords);
     args.ticket = ctx->ticket;
     args.out = ctx->d_out;
-    args.sums = ctx->d_out + kOutWords;
     args.err = ctx->d_err;
     if (ctx->inject_timeouts > 0 && (kind == kCubeF64 || kind == kCubeF64Abs)) {
       args.inject = 16u;
@@ -2181,12 +2180,13 @@ static int dense_collect(perm_ctx* ctx, const DenseOperand& op, const DensePlan&
                          Meanwhile meanwhile) {
   const bool sums = op.variant == PERM_KERNEL_DENSE_SPLIT || op.variant == PERM_KERNEL_DENSE_INT_DD ||
                     op.variant == PERM_KERNEL_DENSE_SDD || op.abs_sum;
-  const int cube_sums = sums && op.shape >= 0 ? p.grid * kCubeWarps : 0;
-  int rc = finish_and_read(ctx, cube_sums, meanwhile);
+  const bool cube_sums = sums && op.shape >= 0;
+  int rc = finish_and_read(ctx, cube_sums ? p.grid * kCubeWords : 0, meanwhile);
   if (rc != PERM_OK) return rc;
   if (cube_sums) {
+    const double* warps = ctx->h_out + kOutWords + 2 * p.grid;
     double m1 = 0.0;
-    for (int w = 0; w < cube_sums; w++) m1 += ctx->h_out[kOutWords + w];
+    for (int w = 0; w < p.grid * kCubeWarps; w++) m1 += warps[w];
     ctx->h_out[12] = m1;
   }
   if (op.variant == PERM_KERNEL_DENSE_SPLIT) {
@@ -3314,15 +3314,16 @@ struct BatchCube {
 // A batch's sums of |term| of its column cubes: one block per cube adds its
 // warps' sums in a fixed order.
 struct CubeSum {
-  uint64_t first;  // in the sums of all cubes
+  uint64_t first;  // of its words in the partials of all cubes
   int count;
   int index;  // of the matrix
 };
-__global__ void __launch_bounds__(128) cube_sums_kernel(const CubeSum* cubes, const double* sums, double* results) {
+__global__ void __launch_bounds__(128) cube_sums_kernel(const CubeSum* cubes, const double* partials, double* results) {
   __shared__ double red[4];
   const CubeSum c = cubes[blockIdx.x];
   double s = 0.0;
-  for (int w = threadIdx.x; w < c.count; w += 128) s += sums[c.first + w];
+  const double* warps = partials + c.first + 2 * (c.count / kCubeWarps);
+  for (int w = threadIdx.x; w < c.count; w += 128) s += warps[w];
   for (int d = 16; d >= 1; d >>= 1) s += __shfl_down_sync(0xffffffffu, s, d);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
   __syncthreads();
@@ -3344,10 +3345,9 @@ struct perm_batch {
   double* d_results = nullptr;
   double* h_results = nullptr;  // pinned: (hi, lo, sum |term|) per matrix, then the error flag
   unsigned char* d_cubes = nullptr;  // column images of the column-cube walks
-  dd* d_cube_partials = nullptr;     // per branch of the graph: partials, tickets
-  unsigned* d_cube_tickets = nullptr;
-  double* d_cube_sums = nullptr;  // of all cubes' warps
-  CubeSum* d_cube_sum = nullptr;  // where each cube's are
+  double* d_cube_partials = nullptr;  // of all cubes
+  unsigned* d_cube_tickets = nullptr;  // per branch of the graph
+  CubeSum* d_cube_sum = nullptr;      // where each cube's are
   std::vector<double> roundings;  // per matrix: roundings per term
   std::vector<double> abs_scale;  // per matrix: factor of its sum |term|
   std::vector<std::pair<int, int>> exp2;  // matrices whose three results are multiplied by 2^second
@@ -3374,7 +3374,6 @@ static void batch_free(perm_batch* b) {
   cudaFree(b->d_cubes);
   cudaFree(b->d_cube_partials);
   cudaFree(b->d_cube_tickets);
-  cudaFree(b->d_cube_sums);
   cudaFree(b->d_cube_sum);
   if (b->h_results) cudaFreeHost(b->h_results);
   delete b;
@@ -3618,16 +3617,16 @@ static int batch_create_locked(perm_ctx* ctx, int count, const int* orders, cons
     for (const BatchCube& c : cube) memcpy(images.data() + c.offset, c.op.image.data(), c.op.image.size());
     BT(cudaMalloc(&b->d_cubes, cube_bytes));
     BT(cudaMemcpy(b->d_cubes, images.data(), cube_bytes, cudaMemcpyHostToDevice));
-    BT(cudaMalloc(&b->d_cube_partials, sizeof(dd) * kMaxBlocks * kBatchBranches));
     BT(cudaMalloc(&b->d_cube_tickets, sizeof(unsigned) * kBatchBranches));
     BT(cudaMemset(b->d_cube_tickets, 0, sizeof(unsigned) * kBatchBranches));
     cube_sum.reserve(cube.size());
-    uint64_t warps = 0;
+    uint64_t words = 0;
     for (const BatchCube& c : cube) {
-      cube_sum.push_back({warps, cube_grid(c) * kCubeWarps, c.index});
-      warps += cube_sum.back().count;
+      const int grid = cube_grid(c);
+      cube_sum.push_back({words, grid * kCubeWarps, c.index});
+      words += (uint64_t)grid * kCubeWords;
     }
-    BT(cudaMalloc(&b->d_cube_sums, sizeof(double) * warps));
+    BT(cudaMalloc(&b->d_cube_partials, sizeof(double) * words));
     BT(cudaMalloc(&b->d_cube_sum, sizeof(CubeSum) * cube_sum.size()));
     BT(cudaMemcpy(b->d_cube_sum, cube_sum.data(), sizeof(CubeSum) * cube_sum.size(), cudaMemcpyHostToDevice));
     if (int rc2 = allow_smem(ctx, (const void*)cube_sums_kernel, 0)) {  // loads it before the capture
@@ -3704,10 +3703,9 @@ static int batch_create_locked(perm_ctx* ctx, int count, const int* orders, cons
     const int m = cube_align(cubes_n, (uint64_t)grid * kCubeThreads, c.op.n - 5);
     CubeLaunch u;
     cube_args(c.op, b->d_cubes + c.offset, m, 0, cubes_n >> m, &u);
-    u.walk.partials = b->d_cube_partials + (size_t)branch * kMaxBlocks;
+    u.walk.partials = reinterpret_cast<dd*>(b->d_cube_partials + cube_sum[i].first);
     u.walk.ticket = b->d_cube_tickets + branch;
     u.walk.out = b->d_results + 3 * c.index;
-    u.walk.sums = b->d_cube_sums + cube_sum[i].first;
     u.walk.err = reinterpret_cast<int*>(b->d_results + 3 * (size_t)count);
     if (ctx->inject_timeouts > 0 && cube_kind(c.op) == kCubeF64) {
       u.walk.inject = 16u;
@@ -3724,7 +3722,7 @@ static int batch_create_locked(perm_ctx* ctx, int count, const int* orders, cons
     cudaStreamWaitEvent(ctx->stream, br.join[i], 0);
   }
   if (branches)
-    cube_sums_kernel<<<(unsigned)cube.size(), 128, 0, ctx->stream>>>(b->d_cube_sum, b->d_cube_sums, b->d_results);
+    cube_sums_kernel<<<(unsigned)cube.size(), 128, 0, ctx->stream>>>(b->d_cube_sum, b->d_cube_partials, b->d_results);
   cudaMemcpyAsync(b->h_results, b->d_results, result_bytes, cudaMemcpyDeviceToHost, ctx->stream);
   BT(cudaStreamEndCapture(ctx->stream, &b->graph));
   BT(cudaGraphInstantiate(&b->exec, b->graph, 0));

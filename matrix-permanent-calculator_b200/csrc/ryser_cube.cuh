@@ -424,15 +424,19 @@ __device__ __forceinline__ void cube_walk(const CubeWalk& a, Start start, Flip f
 }
 
 // The thread totals' sum to *out and, with abs_sum, every warp's sum of m1 to
-// `sums`, which are added in their order afterwards (by the host, or by
+// the words behind the blocks' totals, which are added in their order afterwards (by the host, or by
 // cube_sums_kernel in a batch), so that a walk's error estimate is the same every
 // time.  Adding them here, by the block that finishes last, changed the register
 // allocation of the certified walks: up to 4% slower by shape.
 __device__ __forceinline__ void cube_finish(const CubeWalk& a, dd total, bool abs_sum, double m1, double factor, dd* red) {
+  double* sums = reinterpret_cast<double*>(a.partials + gridDim.x);
   if (abs_sum) {
 #pragma unroll
     for (int d = 16; d >= 1; d >>= 1) m1 += __shfl_down_sync(0xffffffffu, m1, d);
-    if ((threadIdx.x & 31) == 0) a.sums[blockIdx.x * kCubeWarps + (threadIdx.x >> 5)] = m1;
+    if ((threadIdx.x & 31) == 0) {
+      sums[blockIdx.x * kCubeWarps + (threadIdx.x >> 5)] = m1;
+      __threadfence();
+    }
   }
   const dd bt = block_reduce_dd(total, red);
   grid_finish_dd(bt, a.partials, a.ticket, a.out, factor, red);

@@ -12,6 +12,8 @@ struct dd;
 // Threads per CTA, one CTA per SM (ryser_cube.cuh).
 constexpr int kCubeThreads = 256;
 constexpr int kCubeWarps = kCubeThreads / 32;
+// Words a block leaves in `partials`: its total, and its warps' sums of |term|.
+constexpr int kCubeWords = 2 + kCubeWarps;
 // Rows whose product the certified integer walk keeps in FP64 exactly.
 constexpr int kCubeExactRows = 8;
 
@@ -21,10 +23,9 @@ struct CubeWalk {
   int m;                     // log2 of the range alignment, in outer Gray indices
   uint64_t block0, nblocks;  // aligned blocks of 2^m outer indices of this launch
   uint64_t seg;              // cubes between two recomputations of b
-  dd* partials;
+  dd* partials;  // the blocks' totals, then kCubeWarps doubles a block: sum |term| (walks that sum it)
   unsigned* ticket;
   double* out;
-  double* sums;  // kCubeWarps per block: sum |term| (walks that sum it)
   int* err;
   uint32_t inject;  // failure injection (tests): staging expects this many extra bytes
 };
