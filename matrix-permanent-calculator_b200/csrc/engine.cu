@@ -304,8 +304,8 @@ static const void* dense_kernel(int n) {
 // magnitudes depend strongly on |S| (|S| = 0 is the all-minus subset, often
 // the largest term), so a plain uniform sample of Gray indices either misses
 // the heavy classes or, hitting one, overstates the sums by 2^(n-1)/samples.
-// Each thread builds x(S) from scratch in FP64; out[0] and out[1] receive
-// the weighted sums of |prod x_j| and of its square.
+// Each thread builds x(S) from scratch in FP64; block b leaves its weighted sums
+// of |prod x_j| and of its square in out[2 b] and out[2 b + 1].
 __device__ __forceinline__ uint64_t splitmix64(uint64_t& state) {
   uint64_t z = (state += 0x9E3779B97F4A7C15ull);
   z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
@@ -314,8 +314,7 @@ __device__ __forceinline__ uint64_t splitmix64(uint64_t& state) {
 }
 
 __global__ void __launch_bounds__(256) ryser_abs_sample_kernel(const double* colA, int n, int np, int per_class,
-                                                                uint64_t seed, dd* partials, unsigned* ticket,
-                                                                double* out) {
+                                                                uint64_t seed, double* out) {
   __shared__ double sA[64 * 64];
   __shared__ double x0[64];
   __shared__ double red[8], red2[8];
@@ -386,44 +385,14 @@ __global__ void __launch_bounds__(256) ryser_abs_sample_kernel(const double* col
     red2[threadIdx.x >> 5] = local2;
   }
   __syncthreads();
-  // block sums in block order by the block that finishes last: the same every
-  // time, and the ticket ends at 0
-  __shared__ bool is_last;
   if (threadIdx.x == 0) {
     double t = 0.0, t2 = 0.0;
     for (int w = 0; w < (int)(blockDim.x >> 5); w++) {
       t += red[w];
       t2 += red2[w];
     }
-    partials[blockIdx.x] = {t, t2};
-    __threadfence();
-    is_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
-  }
-  __syncthreads();
-  if (!is_last) return;
-  __threadfence();
-  local = local2 = 0.0;
-  for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x) {
-    local += __ldcg(&partials[b].hi);
-    local2 += __ldcg(&partials[b].lo);
-  }
-  for (int d = 16; d >= 1; d >>= 1) {
-    local += __shfl_down_sync(0xffffffffu, local, d);
-    local2 += __shfl_down_sync(0xffffffffu, local2, d);
-  }
-  if ((threadIdx.x & 31) == 0) {
-    red[threadIdx.x >> 5] = local;
-    red2[threadIdx.x >> 5] = local2;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int w = 1; w < (int)(blockDim.x >> 5); w++) {
-      local += red[w];
-      local2 += red2[w];
-    }
-    out[0] = local;
-    out[1] = local2;
-    *ticket = 0u;
+    out[2 * blockIdx.x] = t;
+    out[2 * blockIdx.x + 1] = t2;
   }
 }
 
@@ -510,10 +479,13 @@ using namespace perm;
 struct DenseOperand;
 struct perm_matrix;
 
-// Result words of a call; the column cubes' partials are behind them (kCubeWords a
-// block, at most kCubeBlocks blocks an SM).
+// Result words of a call; behind them are the column cubes' partials (kCubeWords a
+// block, at most kCubeBlocks blocks an SM), or the moment sample's (2 a block).
 constexpr int kOutWords = 16;
 constexpr int kCubeBlocks = 2048 / kCubeThreads;
+constexpr int kSamplesPerClass = 8192;  // term-moment sample: threads per subset-size class
+// Blocks of the sample of an order-n matrix: classes |S| = 0 .. n-1.
+constexpr int moment_blocks(int n) { return n * kSamplesPerClass / 256; }
 
 // Smallest order of the column-cube walks: the shards of shard_bounds are
 // whole cubes of 16 terms from here on, and below it the search for four
@@ -546,7 +518,8 @@ struct perm_ctx {
   dd* partials = nullptr;  // kMaxBlocks dd
   unsigned* ticket = nullptr;
   // One block, read back by one copy: [0..7] results, [8] d_err, [9..10]
-  // d_counters, [12..14] d_est, from kOutWords on the column cubes' partials.
+  // d_counters, [12..14] d_est, from kOutWords on the partial sums of column cubes
+  // or of the term-moment sample.
   double* d_out = nullptr;
   int* d_err = nullptr;
   unsigned long long* d_counters = nullptr;  // [0] queue head, [1] visited
@@ -737,7 +710,8 @@ static int ctx_init(perm_ctx* ctx, int device) {
   CU(ctx, cudaEventCreate(&ctx->ev1));
   CU(ctx, cudaMalloc(&ctx->partials, sizeof(dd) * kMaxBlocks * 2));
   CU(ctx, cudaMalloc(&ctx->ticket, sizeof(unsigned) * 4));
-  const size_t out_words = kOutWords + (size_t)ctx->num_sms * kCubeBlocks * kCubeWords;
+  const size_t out_words = kOutWords + std::max((size_t)ctx->num_sms * kCubeBlocks * kCubeWords,
+                                                (size_t)2 * moment_blocks(PERM_MAX_EXACT_N));
   CU(ctx, cudaMalloc(&ctx->d_out, sizeof(double) * out_words));
   ctx->d_err = reinterpret_cast<int*>(ctx->d_out + 8);
   ctx->d_counters = reinterpret_cast<unsigned long long*>(ctx->d_out + 9);
@@ -766,8 +740,8 @@ extern "C" int perm_ctx_create(int device, perm_ctx** out) {
 }
 
 // Reads back the result block (results, error flag, counters, moments) after
-// the stream drains, with `partials` words of a column-cube walk's; `meanwhile`
-// runs on the host before the wait.
+// the stream drains, with `partials` words of partial sums; `meanwhile` runs on
+// the host before the wait.
 template <class Meanwhile>
 static int finish_and_read(perm_ctx* ctx, int partials, Meanwhile meanwhile) {
   CU(ctx, cudaMemcpyAsync(ctx->h_out, ctx->d_out, sizeof(double) * (kOutWords + partials), cudaMemcpyDeviceToHost,
@@ -2175,14 +2149,29 @@ static int dense_launch(perm_ctx* ctx, const DenseOperand& op, const void* d_ima
   return PERM_OK;
 }
 
+// The moments from the sample's block sums that were read back, in block order:
+// the same every time.
+static void add_moments(perm_ctx* ctx, int n) {
+  double s1 = 0.0, s2 = 0.0;
+  for (int b = 0; b < moment_blocks(n); b++) {
+    s1 += ctx->h_out[kOutWords + 2 * b];
+    s2 += ctx->h_out[kOutWords + 2 * b + 1];
+  }
+  ctx->h_out[12] = s1;
+  ctx->h_out[13] = s2;
+}
+
+// `sampled`: the moment sample was queued behind the walk (row layouts of FP64
+// columns).
 template <class Meanwhile>
 static int dense_collect(perm_ctx* ctx, const DenseOperand& op, const DensePlan& p, perm_result* out,
-                         Meanwhile meanwhile) {
+                         bool sampled, Meanwhile meanwhile) {
   const bool sums = op.variant == PERM_KERNEL_DENSE_SPLIT || op.variant == PERM_KERNEL_DENSE_INT_DD ||
                     op.variant == PERM_KERNEL_DENSE_SDD || op.abs_sum;
   const bool cube_sums = sums && op.shape >= 0;
-  int rc = finish_and_read(ctx, cube_sums ? p.grid * kCubeWords : 0, meanwhile);
+  int rc = finish_and_read(ctx, cube_sums ? p.grid * kCubeWords : sampled ? 2 * moment_blocks(op.n) : 0, meanwhile);
   if (rc != PERM_OK) return rc;
+  if (sampled) add_moments(ctx, op.n);
   if (cube_sums) {
     const double* warps = ctx->h_out + kOutWords + 2 * p.grid;
     double m1 = 0.0;
@@ -2214,7 +2203,7 @@ static int dense_collect(perm_ctx* ctx, const DenseOperand& op, const DensePlan&
 }
 
 static int dense_collect(perm_ctx* ctx, const DenseOperand& op, const DensePlan& p, perm_result* out) {
-  return dense_collect(ctx, op, p, out, [] {});
+  return dense_collect(ctx, op, p, out, false, [] {});
 }
 
 static int check_dense_args(perm_ctx* ctx, const void* mat, int n, int dtype, const void* out) {
@@ -2257,8 +2246,6 @@ static int check_variant(perm_ctx* ctx, int variant) {
 //    for split-dd also the drift of the remainder row sums xl over K updates
 //    (64 n^2 K).  Like the double-double bound, of the (hi, lo) pair: value,
 //    its sum rounded once, adds at most u.
-constexpr int kSamplesPerClass = 8192;  // term-moment sample: threads per subset-size class
-
 struct ErrEstimate {
   double s1 = 0, s2 = 0, worst = 0, random = 0;
 };
@@ -2309,14 +2296,12 @@ static bool plain_columns(const DenseOperand& op) {
   return op.shape < 0 && (op.variant == PERM_KERNEL_DENSE || op.variant == PERM_KERNEL_DENSE_DD);
 }
 
-// Queues the term-moment sample of the column image d_col_fp64 (sums to d_est).
+// Queues the term-moment sample of the column image d_col_fp64.
 static int queue_moments(perm_ctx* ctx, const void* d_col_fp64, int n) {
   const int np = (n + 1) & ~1;
   const int per_class = kSamplesPerClass;
-  const uint64_t threads = (uint64_t)n * per_class;  // classes |S| = 0 .. n-1
-  ryser_abs_sample_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, ctx->stream>>>(
-      static_cast<const double*>(d_col_fp64), n, np, per_class, 0x243F6A8885A308D3ull, ctx->partials, ctx->ticket,
-      ctx->d_est);
+  ryser_abs_sample_kernel<<<moment_blocks(n), 256, 0, ctx->stream>>>(
+      static_cast<const double*>(d_col_fp64), n, np, per_class, 0x243F6A8885A308D3ull, ctx->d_out + kOutWords);
   CU(ctx, cudaGetLastError());
   return PERM_OK;
 }
@@ -2331,8 +2316,10 @@ static int estimate_error(perm_ctx* ctx, const void* d_col_fp64, int n, const De
   *e = ErrEstimate();
   if (n < 2) return PERM_OK;
   if (int rc = queue_moments(ctx, d_col_fp64, n)) return rc;
-  CU(ctx, cudaMemcpyAsync(ctx->h_out + 12, ctx->d_est, 2 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+  CU(ctx, cudaMemcpyAsync(ctx->h_out + kOutWords, ctx->d_out + kOutWords, 2 * moment_blocks(n) * sizeof(double),
+                          cudaMemcpyDeviceToHost, ctx->stream));
   CU(ctx, cudaStreamSynchronize(ctx->stream));
+  add_moments(ctx, n);
   estimate_from_moments(ctx, n, op, value, e);
   return PERM_OK;
 }
@@ -2582,18 +2569,16 @@ static int policy_predicts_sdd(perm_ctx* ctx, const void* mat, int n, int dtype,
   int rc;
   if ((rc = stage_operand(ctx, f))) return rc;
   const int np = (n + 1) & ~1;
-  const uint64_t threads = (uint64_t)n * kSamplesPerClass;
   CU(ctx, cudaMemsetAsync(ctx->d_est + 2, 0, 2 * sizeof(double), ctx->stream));
-  ryser_abs_sample_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, ctx->stream>>>(
-      reinterpret_cast<const double*>(ctx->d_stage), n, np, kSamplesPerClass, 0x243F6A8885A308D3ull, ctx->partials,
-      ctx->ticket, ctx->d_est);
-  CU(ctx, cudaGetLastError());
+  if ((rc = queue_moments(ctx, ctx->d_stage, n))) return rc;
   weighted_rasmussen_kernel<<<(kPredictTrials + 255) / 256, 256, 0, ctx->stream>>>(
       reinterpret_cast<const double*>(ctx->d_stage), n, np, kPredictTrials, 0x13198A2E03707344ull, log2_ub,
       ctx->d_est + 2);
   CU(ctx, cudaGetLastError());
-  CU(ctx, cudaMemcpyAsync(ctx->h_out + 12, ctx->d_est, 3 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+  CU(ctx, cudaMemcpyAsync(ctx->h_out, ctx->d_out, sizeof(double) * (kOutWords + 2 * moment_blocks(n)),
+                          cudaMemcpyDeviceToHost, ctx->stream));
   CU(ctx, cudaStreamSynchronize(ctx->stream));
+  add_moments(ctx, n);
   const double s1 = ctx->h_out[12] * 2.0;  // |factor| = 2
   const double mean_scaled = ctx->h_out[14] / kPredictTrials;
   if (!(mean_scaled > 0.0)) return PERM_OK;  // no trial found a permutation: leave it to the walk
@@ -2665,7 +2650,7 @@ static int exact_dense_call(perm_ctx* ctx, const void* mat, int n, int dtype, in
   const bool sampled = refine && n >= 2 && plain_columns(op);
   if (sampled && (rc = queue_moments(ctx, ctx->d_stage, n))) return rc;
   int matching = -1;
-  if ((rc = dense_collect(ctx, op, p, out, [&] {
+  if ((rc = dense_collect(ctx, op, p, out, sampled, [&] {
          if (policy) matching = has_perfect_matching(mat, n, dtype);
        })))
     return rc;

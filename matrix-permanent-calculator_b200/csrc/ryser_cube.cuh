@@ -424,10 +424,12 @@ __device__ __forceinline__ void cube_walk(const CubeWalk& a, Start start, Flip f
 }
 
 // The thread totals' sum to *out and, with abs_sum, every warp's sum of m1 to
-// the words behind the blocks' totals, which are added in their order afterwards (by the host, or by
-// cube_sums_kernel in a batch), so that a walk's error estimate is the same every
-// time.  Adding them here, by the block that finishes last, changed the register
-// allocation of the certified walks: up to 4% slower by shape.
+// the words behind the blocks' totals, which are added in their order afterwards
+// (by the host, or by cube_sums_kernel in a batch), so that a walk's error estimate
+// is the same every time.  The form matters to the register allocation of the
+// certified walks: added here by the block that finishes last, or stored without
+// the fence (the kernel's end makes the stores visible too), they were up to 4 or 5%
+// slower by shape; so they are within 0.7% of atomic additions in any order.
 __device__ __forceinline__ void cube_finish(const CubeWalk& a, dd total, bool abs_sum, double m1, double factor, dd* red) {
   double* sums = reinterpret_cast<double*>(a.partials + gridDim.x);
   if (abs_sum) {
